@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import os
+import re
 import time
 import subprocess
 import sys
@@ -13,19 +14,22 @@ LIB = PKG / 'libkvm_b200.so'
 CLI = PKG / 'kvm_exec'
 NVCC = os.environ.get('NVCC', '/usr/local/cuda/bin/nvcc')
 CXX = os.environ.get('CXX', 'g++')
-UNITS = ('kvm_exec', 'kvm_static')
-FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-O3', '-std=c++17', '-lineinfo', '-Xcompiler', '-fPIC',
+UNITS = ('kvm_exec', 'kvm_static', 'kvm_unit_flat', 'kvm_unit_rows', 'kvm_unit_mm', 'kvm_unit_attn', 'kvm_unit_decode')
+# relocatable device code: the op families (kvm_unit_*) are linked into both executor kernels; 96 registers is what those kernels' block sizes leave a thread
+FLAGS = ['-gencode', 'arch=compute_100a,code=sm_100a', '-rdc=true', '-maxrregcount=96', '-O3', '-std=c++17', '-lineinfo', '-Xcompiler', '-fPIC',
          '--expt-relaxed-constexpr', '--extended-lambda', '-Xcudafe', '--diag_suppress=177']
 
 
-# files that only one of the two translation units reads (everything else under csrc/ and include/ feeds both)
-ONLY = {'kvm_exec': {'kvm_exec.cu', 'kvm_sched.cuh', 'kvm_host.inl', 'kvm_gemm_host.inl', 'kvm_static_host.inl', 'kvm_json.hpp'},
-        'kvm_static': {'kvm_static.cu', 'kvm_static.cuh'}}
-
-
-def sources(unit=None):
-    skip = {'kvm_cli.cpp'} | (set().union(*(v for k, v in ONLY.items() if k != unit)) if unit else set())
-    return [p for p in sorted(CSRC.glob('*')) if p.name not in skip] + [PKG.parent / 'include' / 'kvm_b200.h', PKG.parent / 'include' / 'kvm_ops.def']
+def sources(unit):
+    """The files a translation unit is made of: its own source and everything it includes."""
+    seen, todo = set(), [CSRC / f'{unit}.cu']
+    while todo:
+        p = todo.pop()
+        if p in seen:
+            continue
+        seen.add(p)
+        todo += [(p.parent / m).resolve() for m in re.findall(r'^ *#include "([^"]+)"', p.read_text(), re.M)]
+    return seen
 
 
 def unit_stale(unit) -> bool:
@@ -40,7 +44,7 @@ def stale() -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Two translation units (the ready-queue kernel + host code, the static-schedule kernel), compiled side by side, then linked."""
+    """The translation units (two executor kernels, the op families), compiled side by side, then linked."""
     if not force and not stale():
         return LIB
     objs, procs = [], []

@@ -149,13 +149,8 @@ __device__ __forceinline__ bool kvm_vec_ok(const KvmBuf& b) { return ((uintptr_t
 #define KVM_M_BF16 4
 #define KVM_M_FLT (KVM_M_F32 | KVM_M_BF16)
 
-// Op bodies are inlined into the dispatcher.  For a per-op report of registers and spills from the compiler (-Xptxas -v), build once
-// with -DKVM_OPS_NOINLINE: every op then is a function of its own (measured 3% slower on a training step, so not the default).
-#ifdef KVM_OPS_NOINLINE
+// An op body: a function of its own, so that it is compiled with registers of its own (see kvm_dispatch.cuh).
 #define KVM_OP_FN static __device__ __noinline__
-#else
-#define KVM_OP_FN static __device__
-#endif
 
 // Fetch table entry `idx` (an argument word). Optional buffers: idx == -1 gives p == nullptr and returns true.
 __device__ __forceinline__ bool kvm_buf(const KvmCtx& c, int idx, int mask, KvmBuf& out, bool optional = false) {

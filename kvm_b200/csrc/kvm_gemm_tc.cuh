@@ -144,7 +144,7 @@ __device__ __forceinline__ void kvm_tc_store32(const KvmMmArgs& g, const float (
     if (g.pre.p) kvm_st8(g.pre, (size_t)m * g.pre.ld + n + j0, v);
     if (g.flags & 8) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = kvm_gelu(v[j]);
+      for (int j = 0; j < 8; ++j) v[j] = g.out.dtype == KVM_BF16 ? kvm_gelu_s(v[j]) : kvm_gelu(v[j]);
     }
     if (g.res.p) { kvm_ld8(g.res, (size_t)m * g.res.ld + n + j0, t);
 #pragma unroll
@@ -201,7 +201,7 @@ static __device__ void kvm_tc_epilogue_staged(const KvmCtx& c, const KvmMmArgs& 
         if (g.pre.p) kvm_st8(g.pre, (size_t)m * g.pre.ld + n, v);
         if (g.flags & 8) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = kvm_gelu(v[j]);
+          for (int j = 0; j < 8; ++j) v[j] = g.out.dtype == KVM_BF16 ? kvm_gelu_s(v[j]) : kvm_gelu(v[j]);
         }
         if (g.res.p) { kvm_ld8(g.res, (size_t)m * g.res.ld + n, t);
 #pragma unroll
@@ -224,7 +224,7 @@ static __device__ void kvm_tc_epilogue_staged(const KvmCtx& c, const KvmMmArgs& 
 // Barriers: the attention set (full 0..2, empty 3..5, accumulator 6) with their completed-phase counts in ctl[KVM_CTL_ACNT + i].
 #define KVM_TCP_STAGES 3
 #define KVM_TCP_STAGE_BYTES (2 * KVM_TC_A_BYTES + KVM_TC_B_BYTES)
-static __device__ void kvm_mm_tc_pair(const KvmCtx& c, const KvmMmArgs& g, const int4& aux) {
+static __device__ __noinline__ void kvm_mm_tc_pair(const KvmCtx& c, const KvmMmArgs& g, const int4& aux) {
   int* ctl = c.ctl;
   int* cnt = ctl + KVM_CTL_ACNT;
   auto bar = [&](int i) { return kvm_bar_addr(ctl, KVM_CTL_ABAR + i); };
@@ -310,14 +310,13 @@ static __device__ void kvm_mm_tc_pair(const KvmCtx& c, const KvmMmArgs& g, const
   }
 }
 
-static __device__ void kvm_tce_epilogue(const KvmCtx& c, const KvmMmArgs& g);
 __device__ __forceinline__ void kvm_mbar_arrive_local(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 // aux.x = 1: tensor-core path planned by the host (aux.y / aux.z = tensor-map indices of A / B); else SIMT fallback.
+// (A tile whose mainloop the engine warps run does not come here: kvm_tce_tile.)
 KVM_OP_FN void kvm_op_matmul_mma_bf16(const KvmCtx& c, const int32_t* a, const int4& aux) {
   KvmMmArgs g;
   if (!kvm_mm_args(c, a, 2, g)) return;
   if (aux.x != 1 || (c.cfg_flags & KVM_CFG_NO_TENSOR_CORES)) { kvm_mm_simt(c, g); return; }
-  if (c.engine) { kvm_tce_epilogue(c, g); return; }      // the engine warps run this tile's mainloop (ready-queue kernel)
   if (c.pair >= 0) { g.m0 &= ~255; kvm_mm_tc_pair(c, g, aux); return; }       // this task and its partner: rows m0.. and m0+128..
   int* ctl = c.ctl;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -481,7 +480,7 @@ __device__ __forceinline__ bool kvm_tce_mma(int* ctl, uint32_t ring0, uint32_t t
 // The compute group's share of a tile whose mainloop the engine runs: wait for the accumulator, drain it 64 columns at a time
 // through the staging area (TMEM -> shared memory by (lane quarter, 16 columns) per warp; then thread = (row, 8 columns): every
 // global access a whole row segment), hand the accumulator back.
-static __device__ void kvm_tce_epilogue(const KvmCtx& c, const KvmMmArgs& g) {
+static __device__ __forceinline__ void kvm_tce_epilogue(const KvmCtx& c, const KvmMmArgs& g) {
   int* ctl = c.ctl;
   const uint32_t acc = c.gemm_seq & 1u, use = c.gemm_seq >> 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = warp & 3, cgi = warp >> 2;
@@ -523,7 +522,7 @@ static __device__ void kvm_tce_epilogue(const KvmCtx& c, const KvmMmArgs& g) {
             if (g.pre.p) kvm_st8(g.pre, (size_t)m * g.pre.ld + n, v);
             if (g.flags & 8) {
 #pragma unroll
-              for (int j = 0; j < 8; ++j) v[j] = kvm_gelu(v[j]);
+              for (int j = 0; j < 8; ++j) v[j] = g.out.dtype == KVM_BF16 ? kvm_gelu_s(v[j]) : kvm_gelu(v[j]);
             }
             if (g.res.p) { kvm_ld8(g.res, (size_t)m * g.res.ld + n, t);
 #pragma unroll
@@ -552,4 +551,11 @@ static __device__ void kvm_tce_epilogue(const KvmCtx& c, const KvmMmArgs& g) {
     kvm_sync();
     if (threadIdx.x == 0 && ok) kvm_mbar_arrive_local(kvm_bar_addr(ctl, KVM_TCE_BAR_ACC_EMPTY + acc));
   }
+}
+
+// The compute group's body of such a tile, inlined into the ready-queue kernel (the most frequent task of a bf16 step: a call would
+// save and restore some fifty registers per thread).
+__device__ __forceinline__ void kvm_tce_tile(const KvmCtx& c, const int32_t* a) {
+  KvmMmArgs g;
+  if (kvm_mm_args(c, a, 2, g)) kvm_tce_epilogue(c, g);
 }

@@ -1,0 +1,553 @@
+// Typed bodies of the memory-bound ops that make up most of the tasks of a training program, inlined into the executor kernels (a
+// call would save and restore some fifty registers per thread through local memory, which the little L1 beside 227 KB of shared
+// memory cannot hold: 2-4 us per task).  Each takes the common storage types and alignments and returns false for anything else,
+// argument errors included: the op's general body (kvm_ops_rows.cuh, kvm_ops_flat.cuh, kvm_ops_attn.cuh) then does the task or
+// reports the error.  Storage types are template arguments, so that the loads of a batch are issued back to back.
+// One SM's share of HBM is 44 KB/us at a loaded latency of 1.5 us: the loops below keep 48-64 KB per SM in flight.
+#pragma once
+#include "kvm_attn_tc.cuh"
+#include "kvm_decode_stream.cuh"
+#include "kvm_dev.cuh"
+#include "kvm_ops_flat.cuh"
+#include "kvm_ops_rows.cuh"
+
+__device__ __forceinline__ bool kvm_hot_buf(const KvmCtx& c, int idx, int dtype, KvmBuf& out) {
+  if (idx < 0 || idx >= c.nbufs) return false;
+  out = c.bufs[idx];
+  return out.p != nullptr && out.dtype == dtype && ((uintptr_t)out.p & 15) == 0;
+}
+__device__ __forceinline__ bool kvm_hot_float(const KvmCtx& c, int idx, KvmBuf& out) {
+  if (idx < 0 || idx >= c.nbufs) return false;
+  out = c.bufs[idx];
+  return out.p != nullptr && out.dtype != KVM_I32 && ((uintptr_t)out.p & 15) == 0;
+}
+__device__ __forceinline__ bool kvm_hot_mat(const KvmBuf& b, int rows, int cols) { return rows <= b.rows && cols <= b.cols && (b.ld & 3) == 0; }
+__device__ __forceinline__ bool kvm_hot_flat(const KvmBuf& b, long long n) { return b.ld == b.cols && n <= (long long)b.rows * b.cols; }
+__device__ __forceinline__ float4 kvm_bf16x4(uint2 u) { return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u)); }
+__device__ __forceinline__ uint2 kvm_to_bf16x4(float4 v) {
+  uint2 u;
+  ((__nv_bfloat162*)&u)[0] = __floats2bfloat162_rn(v.x, v.y);
+  ((__nv_bfloat162*)&u)[1] = __floats2bfloat162_rn(v.z, v.w);
+  return u;
+}
+__device__ __forceinline__ void kvm_st4(const KvmBuf& b, size_t i, float4 v) {
+  if (b.dtype == KVM_BF16) *(uint2*)((__nv_bfloat16*)b.p + i) = kvm_to_bf16x4(v);
+  else *(float4*)((float*)b.p + i) = v;
+}
+
+// ---- layernorm forward, float32 rows -------------------------------------------------------------------------------------------
+// A warp per row, NV float4 per lane; gamma and beta wait in shared memory, the next row is in flight while this one is reduced.
+template <int NV>
+__device__ __forceinline__ void kvm_hot_ln_fwd_t(const KvmBuf& x, const KvmBuf& out, float* mean, float* rstd, const float* gs, int r0, int r1, int d, float eps) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float* xp = (const float*)x.p;
+  constexpr bool AHEAD = NV <= 6;                     // 1024-wide rows leave no registers for a second one
+  float4 nx[NV];
+  auto load = [&](int r) {
+#pragma unroll
+    for (int t = 0; t < NV; ++t) { const int k = lane * 4 + t * 128; nx[t] = (r < r1 && k < d) ? *(const float4*)(xp + (size_t)r * x.ld + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+  };
+  if (AHEAD) load(r0 + warp);
+#pragma unroll 1
+  for (int r = r0 + warp; r < r1; r += KVM_NWARPS) {
+    float4 v[NV];
+    float s = 0.0f, q = 0.0f;
+    if (!AHEAD) load(r);
+#pragma unroll
+    for (int t = 0; t < NV; ++t) { v[t] = nx[t]; s += (v[t].x + v[t].y) + (v[t].z + v[t].w); }
+    if (AHEAD) load(r + KVM_NWARPS);
+    const float mu = kvm_warp_sum(s) / d;
+#pragma unroll
+    for (int t = 0; t < NV; ++t) if (lane * 4 + t * 128 < d) {
+      v[t].x -= mu; v[t].y -= mu; v[t].z -= mu; v[t].w -= mu;
+      q += (v[t].x * v[t].x + v[t].y * v[t].y) + (v[t].z * v[t].z + v[t].w * v[t].w);
+    }
+    const float rs = 1.0f / sqrtf(kvm_warp_sum(q) / d + eps);
+#pragma unroll
+    for (int t = 0; t < NV; ++t) {
+      const int k = lane * 4 + t * 128;
+      if (k < d) {
+        const float4 g = *(const float4*)(gs + k), b = *(const float4*)(gs + 1024 + k);
+        kvm_st4(out, (size_t)r * out.ld + k, make_float4(v[t].x * rs * g.x + b.x, v[t].y * rs * g.y + b.y, v[t].z * rs * g.z + b.z, v[t].w * rs * g.w + b.w));
+      }
+    }
+    if (lane == 0) { rstd[r] = rs; mean[r] = mu; }
+  }
+}
+__device__ __forceinline__ bool kvm_hot_ln_fwd(const KvmCtx& c, const int32_t* a) {
+  KvmBuf x, g, be, out, mean, rstd;
+  const int r0 = a[6], r1 = a[7], d = a[8];
+  const float eps = kvm_bits_f32(a[9]);
+  if (!kvm_hot_buf(c, a[0], KVM_F32, x) || !kvm_hot_buf(c, a[1], KVM_F32, g) || !kvm_hot_buf(c, a[2], KVM_F32, be) || !kvm_hot_float(c, a[3], out) || !kvm_hot_buf(c, a[4], KVM_F32, mean) ||
+      !kvm_hot_buf(c, a[5], KVM_F32, rstd)) return false;
+  if (r0 < 0 || r1 < r0 || d <= 0 || d > 1024 || (d & 3) || !kvm_hot_mat(x, r1, d) || !kvm_hot_mat(out, r1, d) || !kvm_hot_flat(g, d) || !kvm_hot_flat(be, d) || !kvm_hot_flat(mean, r1) ||
+      !kvm_hot_flat(rstd, r1)) return false;
+  float* gs = (float*)c.smem;                     // gamma, beta
+  kvm_sync();
+  if (threadIdx.x * 4 < d) { *(float4*)(gs + threadIdx.x * 4) = *(const float4*)((const float*)g.p + threadIdx.x * 4); *(float4*)(gs + 1024 + threadIdx.x * 4) = *(const float4*)((const float*)be.p + threadIdx.x * 4); }
+  kvm_sync();
+  float* mp = (float*)mean.p; float* rp = (float*)rstd.p;
+  if (d <= 256) kvm_hot_ln_fwd_t<2>(x, out, mp, rp, gs, r0, r1, d, eps);
+  else if (d <= 768) kvm_hot_ln_fwd_t<6>(x, out, mp, rp, gs, r0, r1, d, eps);
+  else kvm_hot_ln_fwd_t<8>(x, out, mp, rp, gs, r0, r1, d, eps);
+  return true;
+}
+
+// ---- layernorm backward (dx), float32 x / dx, dy float32 or bf16 ------------------------------------------------------------------------
+template <int NV, bool YB>
+__device__ __forceinline__ void kvm_hot_ln_bwd_t(const KvmBuf& x, const KvmBuf& dy, const KvmBuf& dx, const float* mean, const float* rstd, const float* gs, int r0, int r1, int d, int acc) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+  for (int r = r0 + warp; r < r1; r += KVM_NWARPS) {
+    float4 xv[NV], yf[YB ? 1 : NV];
+    uint2 yb[YB ? NV : 1];
+    const float* xp = (const float*)x.p + (size_t)r * x.ld;
+    float* op = (float*)dx.p + (size_t)r * dx.ld;
+#pragma unroll
+    for (int t = 0; t < NV; ++t) { const int k = lane * 4 + t * 128; xv[t] = k < d ? *(const float4*)(xp + k) : zero; }
+#pragma unroll
+    for (int t = 0; t < NV; ++t) {
+      const int k = lane * 4 + t * 128;
+      if (YB) yb[t] = k < d ? *(const uint2*)((const __nv_bfloat16*)dy.p + (size_t)r * dy.ld + k) : make_uint2(0u, 0u);
+      else yf[t] = k < d ? *(const float4*)((const float*)dy.p + (size_t)r * dy.ld + k) : zero;
+    }
+    const float mu = mean[r], rs = rstd[r];
+    auto grad = [&](int t) {                       // dy * gamma of this lane's piece t
+      const int k = lane * 4 + t * 128;
+      const float4 y = YB ? kvm_bf16x4(yb[YB ? t : 0]) : yf[YB ? 0 : t];
+      if (k >= d) return zero;
+      const float4 g = *(const float4*)(gs + k);
+      return make_float4(y.x * g.x, y.y * g.y, y.z * g.z, y.w * g.w);
+    };
+    float s1 = 0.0f, s2 = 0.0f;
+#pragma unroll
+    for (int t = 0; t < NV; ++t) {
+      const float4 g = grad(t);
+      xv[t] = make_float4((xv[t].x - mu) * rs, (xv[t].y - mu) * rs, (xv[t].z - mu) * rs, (xv[t].w - mu) * rs);
+      s1 += (g.x + g.y) + (g.z + g.w);
+      s2 += (g.x * xv[t].x + g.y * xv[t].y) + (g.z * xv[t].z + g.w * xv[t].w);
+    }
+    s1 = kvm_warp_sum(s1) / d;
+    s2 = kvm_warp_sum(s2) / d;
+#pragma unroll
+    for (int t = 0; t < NV; ++t) {
+      const int k = lane * 4 + t * 128;
+      if (k < d) {
+        const float4 g = grad(t);
+        const float4 o = acc ? *(const float4*)(op + k) : zero;
+        float4 v = make_float4(rs * (g.x - s1 - xv[t].x * s2), rs * (g.y - s1 - xv[t].y * s2), rs * (g.z - s1 - xv[t].z * s2), rs * (g.w - s1 - xv[t].w * s2));
+        if (acc) v = make_float4(__fadd_rn(o.x, v.x), __fadd_rn(o.y, v.y), __fadd_rn(o.z, v.z), __fadd_rn(o.w, v.w));
+        *(float4*)(op + k) = v;
+      }
+    }
+  }
+}
+__device__ __forceinline__ bool kvm_hot_ln_bwd(const KvmCtx& c, const int32_t* a) {
+  KvmBuf x, dy, g, mean, rstd, dx;
+  const int r0 = a[6], r1 = a[7], d = a[8], acc = a[9];
+  if (!kvm_hot_buf(c, a[0], KVM_F32, x) || !kvm_hot_float(c, a[1], dy) || !kvm_hot_buf(c, a[2], KVM_F32, g) || !kvm_hot_buf(c, a[3], KVM_F32, mean) || !kvm_hot_buf(c, a[4], KVM_F32, rstd) ||
+      !kvm_hot_buf(c, a[5], KVM_F32, dx)) return false;
+  if (r0 < 0 || r1 < r0 || d <= 0 || d > 1024 || (d & 3) || !kvm_hot_mat(x, r1, d) || !kvm_hot_mat(dy, r1, d) || !kvm_hot_mat(dx, r1, d) || !kvm_hot_flat(g, d) || !kvm_hot_flat(mean, r1) ||
+      !kvm_hot_flat(rstd, r1)) return false;
+  float* gs = (float*)c.smem;
+  kvm_sync();
+  if (threadIdx.x * 4 < d) *(float4*)(gs + threadIdx.x * 4) = *(const float4*)((const float*)g.p + threadIdx.x * 4);
+  kvm_sync();
+  const float* mp = (const float*)mean.p; const float* rp = (const float*)rstd.p;
+  const bool yb = dy.dtype == KVM_BF16;
+  if (d <= 256) { if (yb) kvm_hot_ln_bwd_t<2, true>(x, dy, dx, mp, rp, gs, r0, r1, d, acc); else kvm_hot_ln_bwd_t<2, false>(x, dy, dx, mp, rp, gs, r0, r1, d, acc); }
+  else if (!yb) return false;                      // wide float32 rows: the general body
+  else if (d <= 768) kvm_hot_ln_bwd_t<6, true>(x, dy, dx, mp, rp, gs, r0, r1, d, acc);
+  else kvm_hot_ln_bwd_t<8, true>(x, dy, dx, mp, rp, gs, r0, r1, d, acc);
+  return true;
+}
+
+// ---- column sums (and the parameter gradients of a norm) -------------------------------------------------------------------------------
+// 64 columns at a time: a thread owns 4 neighbouring columns of every 32nd row, four rows' loads in flight (float32 rows: 16 bytes
+// per thread and row instead of the 4 of one column per thread, which left the loop at 10 KB/us).  Row groups are added in a fixed
+// order through shared memory.
+template <int MODE, bool XB, bool YB>
+__device__ __forceinline__ void kvm_hot_colreduce_t(float* red, const KvmBuf& x, const KvmBuf& dy, const float* mean, const float* rstd, float* o1, float* o2, int R, int c0, int c1, int acc) {
+  const int cq = threadIdx.x & 15, rg = threadIdx.x >> 4;
+  constexpr int U = MODE == 0 ? 8 : 4;
+#pragma unroll 1
+  for (int cb = c0; cb < c1; cb += 64) {
+    const int col = cb + cq * 4;
+    float4 s1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), s2 = s1;
+    if (col < c1) {
+      auto ldx = [&](int r) { return XB ? kvm_bf16x4(*(const uint2*)((const __nv_bfloat16*)x.p + (size_t)r * x.ld + col)) : *(const float4*)((const float*)x.p + (size_t)r * x.ld + col); };
+      auto ldy = [&](int r) { return YB ? kvm_bf16x4(*(const uint2*)((const __nv_bfloat16*)dy.p + (size_t)r * dy.ld + col)) : *(const float4*)((const float*)dy.p + (size_t)r * dy.ld + col); };
+      auto add = [&](float4 xv, float4 gv, float mu, float rs) {
+        if (MODE == 0) { s1.x += xv.x; s1.y += xv.y; s1.z += xv.z; s1.w += xv.w; }
+        else {
+          s1.x += gv.x * (xv.x - mu) * rs; s1.y += gv.y * (xv.y - mu) * rs; s1.z += gv.z * (xv.z - mu) * rs; s1.w += gv.w * (xv.w - mu) * rs;
+          s2.x += gv.x; s2.y += gv.y; s2.z += gv.z; s2.w += gv.w;
+        }
+      };
+      int r = rg;
+#pragma unroll 1
+      for (; r + (U - 1) * 32 < R; r += U * 32) {
+        float4 xv[U], gv[MODE == 1 ? U : 1];
+        float mu[MODE == 1 ? U : 1], rs[MODE == 1 ? U : 1];
+#pragma unroll
+        for (int u = 0; u < U; ++u) { xv[u] = ldx(r + u * 32); if (MODE == 1) { gv[u] = ldy(r + u * 32); mu[u] = mean ? mean[r + u * 32] : 0.0f; rs[u] = rstd[r + u * 32]; } }
+#pragma unroll
+        for (int u = 0; u < U; ++u) { if (MODE == 1) add(xv[u], gv[u], mu[u], rs[u]); else add(xv[u], xv[u], 0.0f, 0.0f); }
+      }
+#pragma unroll 1
+      for (; r < R; r += 32) { if (MODE == 1) add(ldx(r), ldy(r), mean ? mean[r] : 0.0f, rstd[r]); else { const float4 v = ldx(r); add(v, v, 0.0f, 0.0f); } }
+    }
+    kvm_sync();
+    *(float4*)(red + rg * 64 + cq * 4) = s1;
+    if (MODE == 1) *(float4*)(red + 2048 + rg * 64 + cq * 4) = s2;
+    kvm_sync();
+    if (threadIdx.x < (MODE == 1 ? 128 : 64)) {
+      const int k = threadIdx.x & 63, w = threadIdx.x >> 6, cc = cb + k;
+      float t = 0.0f;
+#pragma unroll
+      for (int g = 0; g < 32; ++g) t += red[w * 2048 + g * 64 + k];
+      float* o = w ? o2 : o1;
+      if (cc < c1 && o) o[cc] = acc ? __fadd_rn(o[cc], t) : t;
+    }
+  }
+}
+__device__ __forceinline__ bool kvm_hot_colsum(const KvmCtx& c, const int32_t* a) {
+  KvmBuf x, out;
+  const int R = a[2], c0 = a[3], c1 = a[4];
+  if (!kvm_hot_float(c, a[0], x) || !kvm_hot_buf(c, a[1], KVM_F32, out)) return false;
+  if (R < 0 || c0 < 0 || c1 < c0 || ((c0 | c1) & 3) || !kvm_hot_mat(x, R, c1) || !kvm_hot_flat(out, c1)) return false;
+  KvmBuf none{};
+  if (x.dtype == KVM_BF16) kvm_hot_colreduce_t<0, true, false>((float*)c.smem, x, none, nullptr, nullptr, (float*)out.p, nullptr, R, c0, c1, a[5]);
+  else kvm_hot_colreduce_t<0, false, false>((float*)c.smem, x, none, nullptr, nullptr, (float*)out.p, nullptr, R, c0, c1, a[5]);
+  return true;
+}
+__device__ __forceinline__ bool kvm_hot_norm_params(const KvmCtx& c, const int32_t* a) {
+  KvmBuf x, dy, mean, rstd, dg, db;
+  const int R = a[6], d = a[7], c0 = a[8], c1 = a[9];
+  if (!kvm_hot_buf(c, a[0], KVM_F32, x) || !kvm_hot_float(c, a[1], dy) || !kvm_hot_buf(c, a[2], KVM_F32, mean) || !kvm_hot_buf(c, a[3], KVM_F32, rstd) || !kvm_hot_buf(c, a[4], KVM_F32, dg) ||
+      !kvm_hot_buf(c, a[5], KVM_F32, db)) return false;
+  if (R < 0 || c0 < 0 || c1 < c0 || c1 > d || ((c0 | c1) & 3) || !kvm_hot_mat(x, R, d) || !kvm_hot_mat(dy, R, d) || !kvm_hot_flat(mean, R) || !kvm_hot_flat(rstd, R) || !kvm_hot_flat(dg, d) ||
+      !kvm_hot_flat(db, d)) return false;
+  if (dy.dtype == KVM_BF16) kvm_hot_colreduce_t<1, false, true>((float*)c.smem, x, dy, (const float*)mean.p, (const float*)rstd.p, (float*)dg.p, (float*)db.p, R, c0, c1, a[10]);
+  else kvm_hot_colreduce_t<1, false, false>((float*)c.smem, x, dy, (const float*)mean.p, (const float*)rstd.p, (float*)dg.p, (float*)db.p, R, c0, c1, a[10]);
+  return true;
+}
+
+// ---- attention delta: sum over a head's columns of o * dO -----------------------------------------------------------------------------
+// An item is 8 neighbouring columns (hd / 8 neighbouring lanes make a head), four items per thread in flight.
+template <bool B>
+__device__ __forceinline__ void kvm_hot_delta_t(const KvmBuf& o, const KvmBuf& dO, float* delta, int r0, int r1, int T, int H, int hd) {
+  constexpr int U = B ? 4 : 2, P = B ? 1 : 2;          // items in flight, 16-byte pieces of an item
+  const int cpr = H * hd / 8, lph = hd / 8, lane = threadIdx.x & 31;
+  const int dr = KVM_NT / cpr, dq = KVM_NT % cpr;      // KVM_NT items further on
+  int r = r0 + threadIdx.x / cpr, q = threadIdx.x % cpr;
+#pragma unroll 1
+  while (__any_sync(0xffffffffu, r < r1)) {
+    uint4 ov[U][P], dv[U][P];
+    int rr = r, qq = q;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (rr < r1) {
+        const uint4* op = (const uint4*)((const char*)o.p + ((size_t)rr * o.ld + qq * 8) * (B ? 2 : 4));
+        const uint4* dp = (const uint4*)((const char*)dO.p + ((size_t)rr * dO.ld + qq * 8) * (B ? 2 : 4));
+#pragma unroll
+        for (int i = 0; i < P; ++i) { ov[u][i] = op[i]; dv[u][i] = dp[i]; }
+      }
+      rr += dr; qq += dq;
+      if (qq >= cpr) { qq -= cpr; ++rr; }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float s = 0.0f;
+      if (r < r1) {
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          const uint32_t x[4] = {ov[u][i].x, ov[u][i].y, ov[u][i].z, ov[u][i].w}, y[4] = {dv[u][i].x, dv[u][i].y, dv[u][i].z, dv[u][i].w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (B) s += __uint_as_float(x[j] << 16) * __uint_as_float(y[j] << 16) + __uint_as_float(x[j] & 0xffff0000u) * __uint_as_float(y[j] & 0xffff0000u);
+            else s += __uint_as_float(x[j]) * __uint_as_float(y[j]);
+          }
+        }
+      }
+      for (int w = lph >> 1; w; w >>= 1) s += __shfl_xor_sync(0xffffffffu, s, w);      // KVM_NT and cpr are multiples of hd / 8: a head never straddles warps or steps
+      if (r < r1 && (lane % lph) == 0) delta[(size_t)((r / T) * H + q / lph) * T + r % T] = s;
+      r += dr; q += dq;
+      if (q >= cpr) { q -= cpr; ++r; }
+    }
+  }
+}
+__device__ __forceinline__ bool kvm_hot_delta(const KvmCtx& c, const int32_t* a) {
+  KvmBuf o, dO, delta;
+  const int r0 = a[3], r1 = a[4], T = a[5], H = a[6], hd = a[7];
+  if (!kvm_hot_float(c, a[0], o) || !kvm_hot_float(c, a[1], dO) || !kvm_hot_buf(c, a[2], KVM_F32, delta)) return false;
+  if (o.dtype != dO.dtype || !(hd == 32 || hd == 64 || hd == 128) || r0 < 0 || r1 < r0 || T <= 0 || H <= 0 || !kvm_hot_mat(o, r1, H * hd) || !kvm_hot_mat(dO, r1, H * hd) ||
+      ((o.ld | dO.ld) & 7) || !kvm_hot_flat(delta, (long long)((r1 + T - 1) / T) * H * T) || (long long)(r1 - r0) * H * hd >= (1LL << 30)) return false;
+  if (o.dtype == KVM_BF16) kvm_hot_delta_t<true>(o, dO, (float*)delta.p, r0, r1, T, H, hd);
+  else kvm_hot_delta_t<false>(o, dO, (float*)delta.p, r0, r1, T, H, hd);
+  return true;
+}
+
+// ---- cross entropy of long bf16 rows (forward and gradient in one op) -------------------------------------------------------------------
+// A row is fetched once, by a bulk copy into shared memory that runs while the row before it is worked on (two row buffers; with
+// room for one only, the next copy starts when the row is done), and read from there three times: maximum, sum, gradient.  Maximum
+// and sum take one barrier each.  Bound by HBM (read + write, 4 bytes per logit: 4.6 us for 50304 of them at an SM's share) with
+// the exponentials (two per logit, 16 a cycle: 3.2 us) beside it; the loop it replaces read the row twice from HBM, 19 us a row.
+__device__ __forceinline__ bool kvm_hot_ce_fused(const KvmCtx& c, const int32_t* a) {
+  KvmBuf lg, tg, rl, ls, dl;
+  const int r0 = a[5], r1 = a[6], V = a[7];
+  if (!kvm_hot_buf(c, a[0], KVM_BF16, lg) || !kvm_hot_buf(c, a[1], KVM_I32, tg) || !kvm_hot_buf(c, a[2], KVM_F32, rl) || !kvm_hot_buf(c, a[3], KVM_F32, ls) || !kvm_hot_buf(c, a[4], KVM_BF16, dl)) return false;
+  if (a[8] != -1 || a[9] <= 0 || r0 < 0 || r1 <= r0 || V <= 1024 || (V & 7) || ((lg.ld | dl.ld) & 7) || !kvm_hot_mat(lg, r1, V) || !kvm_hot_mat(dl, r1, V) || !kvm_hot_flat(tg, r1) ||
+      !kvm_hot_flat(rl, r1) || !kvm_hot_flat(ls, r1) || c.smem_bytes < 1024 + V * 2) return false;
+  const int* tp = (const int*)tg.p;
+  for (int r = r0; r < r1; ++r) if (tp[r] < 0 || tp[r] >= V) return false;      // ignored rows and bad tokens: the general body
+  const float f = __fmul_rn((float)(1.0 / (double)a[9]), kvm_bits_f32(a[10]));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, pitch = (V * 2 + 127) & ~127;
+  const bool two = c.smem_bytes >= 1024 + 2 * pitch;
+  float* red = (float*)c.smem;                         // [2][16] maxima, [2][16] sums of the warps
+  int* cnt = c.ctl + KVM_CTL_ACNT + 7;
+  const uint32_t bar = kvm_bar_addr(c.ctl, KVM_CTL_ABAR + 7), dst = kvm_smem_addr(c.smem + 1024);
+  const __nv_bfloat16* src = (const __nv_bfloat16*)lg.p;
+  const int phase0 = *cnt;
+  auto fetch = [&](int r) {                            // thread 0
+    kvm_mbar_expect_tx(bar, (uint32_t)V * 2);
+    kvm_bulk_g2s(dst + (two ? ((r - r0) & 1) * pitch : 0), src + (size_t)r * lg.ld, (uint32_t)V * 2, bar);
+  };
+  kvm_sync();                                          // the scratch is free, and everyone has read the phase count
+  if (tid == 0) { asm volatile("fence.proxy.async;" ::: "memory"); fetch(r0); }      // logits written by other tasks' plain stores
+  bool ok = true;
+#pragma unroll 1
+  for (int r = r0; r < r1; ++r) {
+    const unsigned char* row = c.smem + 1024 + (two ? ((r - r0) & 1) * pitch : 0);
+    const int t = tp[r];
+    if (!kvm_mbar_wait(bar, (phase0 + r - r0) & 1)) ok = false;
+    if (two && tid == 0 && r + 1 < r1) fetch(r + 1);   // the other buffer was last read before the barrier at the end of the previous row
+    __nv_bfloat162 mx = __halves2bfloat162(__ushort_as_bfloat16(0xff80), __ushort_as_bfloat16(0xff80));
+#pragma unroll 4
+    for (int k = tid * 8; k < V; k += KVM_NT * 8) {
+      const uint4 v = *(const uint4*)(row + k * 2);
+      const __nv_bfloat162* h = (const __nv_bfloat162*)&v;
+      mx = __hmax2(mx, __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
+    }
+    float m = kvm_warp_max(fmaxf(__bfloat162float(mx.x), __bfloat162float(mx.y)));
+    float* rr = red + ((r - r0) & 1) * 32;
+    if (lane == 0) rr[warp] = m;
+    kvm_sync();
+    m = rr[0];
+#pragma unroll
+    for (int w = 1; w < KVM_NWARPS; ++w) m = fmaxf(m, rr[w]);
+    const float m2 = m * KVM_LOG2E;
+    float s = 0.0f;
+#pragma unroll 2
+    for (int k = tid * 8; k < V; k += KVM_NT * 8) {
+      const uint4 v = *(const uint4*)(row + k * 2);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      float e[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) e[i] = kvm_ex2(fmaf(__uint_as_float(w[i] << 16), KVM_LOG2E, -m2)) + kvm_ex2(fmaf(__uint_as_float(w[i] & 0xffff0000u), KVM_LOG2E, -m2));
+      s += (e[0] + e[1]) + (e[2] + e[3]);
+    }
+    s = kvm_warp_sum(s);
+    if (lane == 0) rr[16 + warp] = s;
+    kvm_sync();
+    s = 0.0f;
+#pragma unroll
+    for (int w = 0; w < KVM_NWARPS; ++w) s += rr[16 + w];
+    const float lse = m + logf(s), l2 = lse * KVM_LOG2E;
+    if (tid == 0) { ((float*)ls.p)[r] = lse; ((float*)rl.p)[r] = lse - __bfloat162float(*(const __nv_bfloat16*)(row + t * 2)); }
+    __nv_bfloat16* out = (__nv_bfloat16*)dl.p + (size_t)r * dl.ld;
+#pragma unroll 2
+    for (int k = tid * 8; k < V; k += KVM_NT * 8) {
+      const uint4 v = *(const uint4*)(row + k * 2);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      uint4 o;
+      uint32_t* ow = (uint32_t*)&o;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float p = kvm_ex2(fmaf(__uint_as_float(w[i] << 16), KVM_LOG2E, -l2)), q = kvm_ex2(fmaf(__uint_as_float(w[i] & 0xffff0000u), KVM_LOG2E, -l2));
+        if (k + 2 * i == t) p -= 1.0f;
+        if (k + 2 * i + 1 == t) q -= 1.0f;
+        const __nv_bfloat162 h = __floats2bfloat162_rn(p * f, q * f);
+        ow[i] = *(const uint32_t*)&h;
+      }
+      *(uint4*)(out + k) = o;
+    }
+    kvm_sync();                                        // everyone is done with the row
+    if (!two && tid == 0 && r + 1 < r1) fetch(r + 1);
+  }
+  if (!ok) kvm_att_fail(c, 127);
+  if (tid == 0) *cnt = phase0 + (r1 - r0);
+  return true;
+}
+
+// ---- flat ranges --------------------------------------------------------------------------------------------------------------------------
+// NI inputs of a flat range come through shared memory: bulk copies of SE elements per input, four stages deep (96-128 KB in flight,
+// none of it in registers), every thread works on its part of the stage that has landed and stores its results from registers.
+// With the same bytes in flight in registers the loops spilled, and the spills' traffic cost more than the loads.
+// body(stage, i, n): stage = the inputs' parts of the stage (shared memory), elements [i, i + n) of the range.
+#define KVM_STREAM_DEPTH 4
+#define KVM_STREAM_BAR 8                               // barriers KVM_CTL_ABAR + 8 .. + 11 and their completed-phase counts
+template <int NI, int SE, class Body>
+__device__ __forceinline__ void kvm_stream(const KvmCtx& c, const char* const (&in)[NI], const int (&eb)[NI], int e0, int e1, Body body) {
+  int off[NI], bytes = 0;
+#pragma unroll
+  for (int n = 0; n < NI; ++n) { off[n] = bytes; bytes += SE * eb[n]; }
+  const int ns = (e1 - e0 + SE - 1) / SE;
+  int* cnt = c.ctl + KVM_CTL_ACNT + KVM_STREAM_BAR;
+  auto bar = [&](int s) { return kvm_bar_addr(c.ctl, KVM_CTL_ABAR + KVM_STREAM_BAR + (s & (KVM_STREAM_DEPTH - 1))); };
+  auto issue = [&](int s) {                            // thread 0
+    const int i = e0 + s * SE, n = min(SE, e1 - i);
+    uint32_t tx = 0;
+#pragma unroll
+    for (int k = 0; k < NI; ++k) tx += (uint32_t)(n * eb[k]);
+    kvm_mbar_expect_tx(bar(s), tx);
+    const uint32_t dst = kvm_smem_addr(c.smem + 1024) + (uint32_t)((s & (KVM_STREAM_DEPTH - 1)) * bytes);
+#pragma unroll
+    for (int k = 0; k < NI; ++k) kvm_bulk_g2s(dst + off[k], in[k] + (size_t)i * eb[k], (uint32_t)(n * eb[k]), bar(s));
+  };
+  uint32_t ph[KVM_STREAM_DEPTH];
+#pragma unroll
+  for (int s = 0; s < KVM_STREAM_DEPTH; ++s) ph[s] = (uint32_t)cnt[s];
+  kvm_sync();                                          // the scratch is free, the counts have been read
+  if (threadIdx.x == 0) {
+    asm volatile("fence.proxy.async;" ::: "memory");   // inputs written by other tasks' plain stores
+    for (int s = 0; s < min(ns, KVM_STREAM_DEPTH); ++s) issue(s);
+  }
+  uint32_t par = 0;
+#pragma unroll
+  for (int s = 0; s < KVM_STREAM_DEPTH; ++s) par |= (ph[s] & 1u) << s;
+  bool ok = true;
+#pragma unroll 1
+  for (int s = 0; s < ns; ++s) {
+    const int d = s & (KVM_STREAM_DEPTH - 1);
+    if (!kvm_mbar_wait(bar(s), (par >> d) & 1u)) ok = false;
+    par ^= 1u << d;
+    const char* st = (const char*)c.smem + 1024 + d * bytes;
+    const char* part[NI];
+#pragma unroll
+    for (int n = 0; n < NI; ++n) part[n] = st + off[n];
+    const int i = e0 + s * SE;
+    body(part, i, min(SE, e1 - i));
+    kvm_sync();                                        // the stage has been read
+    if (threadIdx.x == 0 && s + KVM_STREAM_DEPTH < ns) issue(s + KVM_STREAM_DEPTH);
+  }
+  if (!ok) kvm_att_fail(c, 2000);
+  if (threadIdx.x < KVM_STREAM_DEPTH) cnt[threadIdx.x] += (ns - (int)threadIdx.x + KVM_STREAM_DEPTH - 1) / KVM_STREAM_DEPTH;
+}
+__device__ __forceinline__ bool kvm_hot_range(int e0, int e1, int align) { return e0 >= 0 && e1 > e0 && ((e0 | e1) & (align - 1)) == 0; }
+
+// Elementwise map over inputs of one storage type: 8 KB of each input per stage, 16 bytes per thread.
+template <int NI, bool B, class F>
+__device__ __forceinline__ void kvm_hot_map_t(const KvmCtx& c, const char* const (&in)[NI], void* out, int e0, int e1, F f) {
+  constexpr int E = B ? 8 : 4;
+  int eb[NI];
+#pragma unroll
+  for (int n = 0; n < NI; ++n) eb[n] = B ? 2 : 4;
+  kvm_stream<NI, KVM_NT * E>(c, in, eb, e0, e1, [&](const char* const (&part)[NI], int i, int n) {
+    const int k = (int)threadIdx.x * E;
+    if (k >= n) return;
+    uint4 x[NI], w;
+#pragma unroll
+    for (int m = 0; m < NI; ++m) x[m] = *(const uint4*)(part[m] + k * (B ? 2 : 4));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float lo[NI], hi[NI];
+#pragma unroll
+      for (int m = 0; m < NI; ++m) {
+        const uint32_t u = j == 0 ? x[m].x : j == 1 ? x[m].y : j == 2 ? x[m].z : x[m].w;
+        lo[m] = B ? __uint_as_float(u << 16) : __uint_as_float(u);
+        hi[m] = __uint_as_float(u & 0xffff0000u);
+      }
+      if (B) ((__nv_bfloat162*)&w)[j] = __floats2bfloat162_rn(f(lo), f(hi));
+      else ((uint32_t*)&w)[j] = __float_as_uint(f(lo));
+    }
+    *(uint4*)((char*)out + (size_t)(i + k) * (B ? 2 : 4)) = w;
+  });
+}
+// Two inputs and an output of one storage type (or one input: `second` < 0).
+template <int NI, bool B, class F>
+__device__ __forceinline__ bool kvm_hot_map(const KvmCtx& c, int i0, int i1, int o, int e0, int e1, F f) {
+  KvmBuf x, y, z;
+  const int dt = B ? KVM_BF16 : KVM_F32;
+  if (!kvm_hot_range(e0, e1, B ? 8 : 4) || !kvm_hot_buf(c, i0, dt, x) || (NI == 2 && !kvm_hot_buf(c, i1, dt, y)) || !kvm_hot_buf(c, o, dt, z) || !kvm_hot_flat(x, e1) ||
+      (NI == 2 && !kvm_hot_flat(y, e1)) || !kvm_hot_flat(z, e1)) return false;
+  const char* in[NI];
+  in[0] = (const char*)x.p;
+  if (NI == 2) in[NI - 1] = (const char*)y.p;
+  kvm_hot_map_t<NI, B>(c, in, z.p, e0, e1, f);
+  return true;
+}
+// f32 -> bf16
+__device__ __forceinline__ bool kvm_hot_round_bf16(const KvmCtx& c, const int32_t* a) {
+  KvmBuf x, o;
+  const int e0 = a[2], e1 = a[3];
+  if (!kvm_hot_buf(c, a[0], KVM_F32, x) || !kvm_hot_buf(c, a[1], KVM_BF16, o) || !kvm_hot_range(e0, e1, 4) || !kvm_hot_flat(x, e1) || !kvm_hot_flat(o, e1)) return false;
+  const char* const in[1] = {(const char*)x.p};
+  const int eb[1] = {4};
+  kvm_stream<1, 4 * KVM_NT * 4>(c, in, eb, e0, e1, [&](const char* const (&part)[1], int i, int n) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) { const int k = (u * KVM_NT + (int)threadIdx.x) * 4; if (k < n) *(uint2*)((__nv_bfloat16*)o.p + i + k) = kvm_to_bf16x4(*(const float4*)(part[0] + k * 4)); }
+  });
+  return true;
+}
+// AdamW, float32 state
+__device__ __forceinline__ bool kvm_hot_adamw(const KvmCtx& c, const int32_t* a) {
+  KvmBuf p, g, m, v, gs, st;
+  const int e0 = a[6], e1 = a[7];
+  if (!kvm_hot_buf(c, a[0], KVM_F32, p) || !kvm_hot_buf(c, a[1], KVM_F32, g) || !kvm_hot_buf(c, a[2], KVM_F32, m) || !kvm_hot_buf(c, a[3], KVM_F32, v) || a[4] < 0 || a[4] >= c.nbufs ||
+      a[5] < 0 || a[5] >= c.nbufs) return false;
+  gs = c.bufs[a[4]]; st = c.bufs[a[5]];
+  if (!gs.p || gs.dtype != KVM_F32 || !st.p || st.dtype != KVM_I32 || !kvm_hot_range(e0, e1, 4) || !kvm_hot_flat(p, e1) || !kvm_hot_flat(g, e1) || !kvm_hot_flat(m, e1) || !kvm_hot_flat(v, e1)) return false;
+  const int t = ((const int*)st.p)[0];
+  if (t < 1) return false;
+  const KvmAdamK k = kvm_adamw_consts(c, t, kvm_bits_f32(a[8]), kvm_bits_f32(a[9]), kvm_bits_f32(a[10]), kvm_bits_f32(a[11]), kvm_bits_f32(a[12]), ((const float*)gs.p)[0]);
+  const char* const in[4] = {(const char*)p.p, (const char*)g.p, (const char*)m.p, (const char*)v.p};
+  const int eb[4] = {4, 4, 4, 4};
+  float* pp = (float*)p.p; float* mp = (float*)m.p; float* vp = (float*)v.p;
+  kvm_stream<4, KVM_NT * 4>(c, in, eb, e0, e1, [&](const char* const (&part)[4], int i, int n) {
+    const int q = (int)threadIdx.x * 4;
+    if (q >= n) return;
+    float4 P = *(const float4*)(part[0] + q * 4), M = *(const float4*)(part[2] + q * 4), W = *(const float4*)(part[3] + q * 4);
+    const float4 G = *(const float4*)(part[1] + q * 4);
+    kvm_adamw_step(k, G.x, P.x, M.x, W.x); kvm_adamw_step(k, G.y, P.y, M.y, W.y); kvm_adamw_step(k, G.z, P.z, M.z, W.z); kvm_adamw_step(k, G.w, P.w, M.w, W.w);
+    *(float4*)(pp + i + q) = P; *(float4*)(mp + i + q) = M; *(float4*)(vp + i + q) = W;
+  });
+  return true;
+}
+__device__ __forceinline__ bool kvm_hot_gradnorm(const KvmCtx& c, const int32_t* a) {
+  KvmBuf g, part;
+  const int slot = a[2], e0 = a[3], e1 = a[4];
+  if (!kvm_hot_buf(c, a[0], KVM_F32, g) || !kvm_hot_buf(c, a[1], KVM_F32, part) || slot < 0 || !kvm_hot_range(e0, e1, 4) || !kvm_hot_flat(g, e1) || !kvm_hot_flat(part, slot + 1)) return false;
+  double s = 0.0;
+  const char* const in[1] = {(const char*)g.p};
+  const int eb[1] = {4};
+  kvm_stream<1, 4 * KVM_NT * 4>(c, in, eb, e0, e1, [&](const char* const (&st)[1], int, int n) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = (u * KVM_NT + (int)threadIdx.x) * 4;
+      if (k < n) { const float4 v = *(const float4*)(st[0] + k * 4); s += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w); }
+    }
+  });
+  s = kvm_block_sum(s, (double*)c.smem);
+  if (threadIdx.x == 0) ((float*)part.p)[slot] = (float)s;
+  return true;
+}
+
+// The typed form of op `op`, if there is one for these buffers.  BIG: programs with long rows (the ready-queue kernel).
+template <bool BIG>
+__device__ __forceinline__ bool kvm_hot(const KvmCtx& c, int op, const int32_t* a) {
+  switch (op) {
+    case 35: return kvm_hot_ln_fwd(c, a);
+    case 37: return kvm_hot_ln_bwd(c, a);
+    case 39: return kvm_hot_norm_params(c, a);
+    case 41: return !a[5] && kvm_hot_map<2, true>(c, a[0], a[1], a[2], a[3], a[4], [](const float (&v)[2]) { return __fmul_rn(v[1], kvm_gelu_grad_s(v[0])); });
+    case 46: return kvm_hot_delta(c, a);
+    case 54: return kvm_hot_adamw(c, a);
+    case 55: return kvm_hot_gradnorm(c, a);
+    case 61: return kvm_hot_colsum(c, a);
+    case 113: return kvm_hot_round_bf16(c, a);
+    case 127: return BIG && kvm_hot_ce_fused(c, a);
+    default: return false;
+  }
+}

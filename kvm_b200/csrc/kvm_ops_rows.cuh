@@ -14,6 +14,40 @@ KVM_OP_FN void kvm_op_embedding_fwd(const KvmCtx& c, const int32_t* a) {
   if (r0 < 0 || r1 < r0 || T <= 0 || d <= 0 || !kvm_flat_ok(c, ids, r1) || !kvm_mat_ok(c, out, r1, d) || !kvm_mat_ok(c, wte, 0, d) ||
       !kvm_mat_ok(c, wpe, T, d)) { c.fail(KVM_OPE_RANGE, r0, r1); return; }
   const int* id = (const int*)ids.p;
+  if (wte.dtype == KVM_F32 && out.dtype == KVM_F32 && (!wpe.p || (wpe.dtype == KVM_F32 && (wpe.ld & 3) == 0 && kvm_vec_ok(wpe))) && ((d | wte.ld | out.ld) & 3) == 0 && kvm_vec_ok(wte) &&
+      kvm_vec_ok(out)) {
+    // float32 tables: four 16-byte pieces per thread and table in flight (the scalar loop below has one element in flight, and each
+    // waits for its token id: 300 us for 256 rows of 768 values, 20 us here for the same rows)
+    const int cpr = d / 4, items = (r1 - r0) * cpr;
+    for (int i0 = 0; i0 < items; i0 += 4 * KVM_NT) {
+      int tok[4];
+      float4 x[4], y[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) { const int it = i0 + u * KVM_NT + threadIdx.x; tok[u] = it < items ? id[r0 + it / cpr] : -1; }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int it = i0 + u * KVM_NT + threadIdx.x;
+        x[u] = y[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (it < items) {
+          const int r = r0 + it / cpr, col = (it % cpr) * 4;
+          if (tok[u] < 0 || tok[u] >= wte.rows) c.fail_any(KVM_OPE_TOKEN, tok[u], r);
+          else {
+            x[u] = *(const float4*)((const float*)wte.p + (size_t)tok[u] * wte.ld + col);
+            if (wpe.p) y[u] = *(const float4*)((const float*)wpe.p + (size_t)(r % T) * wpe.ld + col);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int it = i0 + u * KVM_NT + threadIdx.x;
+        if (it < items) {
+          if (wpe.p) { x[u].x = __fadd_rn(x[u].x, y[u].x); x[u].y = __fadd_rn(x[u].y, y[u].y); x[u].z = __fadd_rn(x[u].z, y[u].z); x[u].w = __fadd_rn(x[u].w, y[u].w); }
+          *(float4*)((float*)out.p + (size_t)(r0 + it / cpr) * out.ld + (it % cpr) * 4) = x[u];
+        }
+      }
+    }
+    return;
+  }
   long long n = (long long)(r1 - r0) * d;
   for (long long e = threadIdx.x; e < n; e += KVM_NT) {
     int r = r0 + (int)(e / d), col = (int)(e % d), tok = id[r];
@@ -28,8 +62,10 @@ KVM_OP_FN void kvm_op_embedding_fwd(const KvmCtx& c, const int32_t* a) {
 }
 
 // One task owns keys [v0,v1): rows with a key in range are compacted in ascending order into shared memory (block-wide
-// ordered scan), then added row by row, each thread owning columns, so every element sums its rows in ascending order
-// with one float32 add each (runtime/ref_gpt.py:55-66).
+// ordered scan) together with their key; a warp then adds the rows of its keys (key mod 16) one after the other, its lanes over the
+// columns, so every element sums its rows in ascending order with one float32 add each (runtime/ref_gpt.py:55-66) while sixteen
+// keys go on side by side.  (The whole block on one row at a time was a serial chain of read-modify-writes over all hits of the
+// task: 183 us for 512 rows of 128 columns.)
 KVM_OP_FN void kvm_op_embedding_bwd(const KvmCtx& c, const int32_t* a) {
   KvmBuf ids, dout, dt;
   if (!kvm_buf(c, a[0], KVM_M_I32, ids, true) || !kvm_buf(c, a[1], KVM_M_FLT, dout) || !kvm_buf(c, a[2], KVM_M_F32, dt)) return;
@@ -37,49 +73,88 @@ KVM_OP_FN void kvm_op_embedding_bwd(const KvmCtx& c, const int32_t* a) {
   if (N < 0 || v0 < 0 || v1 < v0 || d <= 0 || (!ids.p && mod <= 0) || !kvm_mat_ok(c, dout, N, d) || !kvm_mat_ok(c, dt, v1, d) ||
       !kvm_flat_ok(c, ids, N)) { c.fail(KVM_OPE_RANGE, v0, v1); return; }
   float* tab = (float*)dt.p;
+  const bool vec = dout.dtype == KVM_F32 && ((d | dout.ld | dt.ld) & 3) == 0 && kvm_vec_ok(dout) && kvm_vec_ok(dt);
+  const int cpr = vec ? d / 4 : d;
   if (!ids.p) {
-    // positional table: key k collects rows k, k+mod, k+2*mod, ... in that (ascending) order; thread = (key, column)
-    for (long long e = threadIdx.x; e < (long long)(v1 - v0) * d; e += KVM_NT) {
-      const int key = v0 + (int)(e / d), col = (int)(e % d);
+    // positional table: key k collects rows k, k+mod, k+2*mod, ... in that (ascending) order; thread = (key, column or four columns),
+    // eight rows' loads in flight
+    for (long long e = threadIdx.x; e < (long long)(v1 - v0) * cpr; e += KVM_NT) {
+      const int key = v0 + (int)(e / cpr), col = (int)(e % cpr) * (vec ? 4 : 1);
       const size_t o = (size_t)key * dt.ld + col;
+      if (vec) {
+        float4 sum = acc ? *(const float4*)(tab + o) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (key < mod)
+          for (int r = key; r < N; r += 8 * mod) {
+            float4 x[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) if (r + (long long)u * mod < N) x[u] = *(const float4*)((const float*)dout.p + (size_t)(r + u * mod) * dout.ld + col);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) if (r + (long long)u * mod < N) {
+              sum.x = __fadd_rn(sum.x, x[u].x); sum.y = __fadd_rn(sum.y, x[u].y); sum.z = __fadd_rn(sum.z, x[u].z); sum.w = __fadd_rn(sum.w, x[u].w);
+            }
+          }
+        *(float4*)(tab + o) = sum;
+        continue;
+      }
       float sum = acc ? tab[o] : 0.0f;
       if (key < mod) for (int r = key; r < N; r += mod) sum = __fadd_rn(sum, kvm_ld(dout, (size_t)r * dout.ld + col));
       tab[o] = sum;
     }
     return;
   }
-  if (!acc)
-    for (long long e = threadIdx.x; e < (long long)(v1 - v0) * d; e += KVM_NT) tab[(size_t)(v0 + e / d) * dt.ld + e % d] = 0.0f;
-  int* list = (int*)c.smem;                       // [cap] rows, then KVM_NWARPS+1 counters
-  const int cap = (c.smem_bytes - 256) / 4;
-  int* wcnt = list + cap;
+  if (!acc) {
+    for (long long e = threadIdx.x; e < (long long)(v1 - v0) * cpr; e += KVM_NT) {
+      float* o = tab + (size_t)(v0 + e / cpr) * dt.ld + (e % cpr) * (vec ? 4 : 1);
+      if (vec) *(float4*)o = make_float4(0.0f, 0.0f, 0.0f, 0.0f); else *o = 0.0f;
+    }
+  }
+  int2* list = (int2*)c.smem;                     // [cap] (row, key), then KVM_NWARPS counters
+  const int cap = (c.smem_bytes - 256) / 8;
+  int* wcnt = (int*)(list + cap);
   const int* id = (const int*)ids.p;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   kvm_sync();
   for (int base = 0; base < N;) {
     // fill the list with up to cap matching rows starting at `base`
     int filled = 0, next = base;
-    while (next < N && filled + KVM_NT <= cap) {
-      int r = next + threadIdx.x;
-      int key = r < N ? (id ? id[r] : r % mod) : -1;
-      bool hit = r < N && key >= v0 && key < v1;
-      unsigned m = __ballot_sync(0xffffffffu, hit);
-      if (lane == 0) wcnt[warp] = __popc(m);
+    while (next < N && filled + 4 * KVM_NT <= cap) {
+      // four rows per thread and pass (a thread's rows are neighbours, so ascending order is thread order)
+      const int r = next + threadIdx.x * 4;
+      int key[4], n = 0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) key[u] = r + u < N ? id[r + u] : -1;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) { if (key[u] < v0 || key[u] >= v1) key[u] = -1; n += key[u] >= 0; }
+      int incl = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += t; }
+      if (lane == 31) wcnt[warp] = incl;
       kvm_sync();
-      int off = filled;
-      for (int w = 0; w < warp; ++w) off += wcnt[w];
-      if (hit) list[off + __popc(m & ((1u << lane) - 1))] = r;
-      int tot = 0;
-      for (int w = 0; w < KVM_NWARPS; ++w) tot += wcnt[w];
+      int off = filled + incl - n, tot = 0;
+      for (int w = 0; w < KVM_NWARPS; ++w) { if (w < warp) off += wcnt[w]; tot += wcnt[w]; }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) if (key[u] >= 0) list[off++] = make_int2(r + u, key[u]);
       kvm_sync();
-      filled += tot; next += KVM_NT;
+      filled += tot; next += 4 * KVM_NT;
     }
-    kvm_sync();
-    for (int i = 0; i < filled; ++i) {
-      int r = list[i], key = id ? id[r] : r % mod;
-      for (int col = threadIdx.x; col < d; col += KVM_NT) {
-        size_t o = (size_t)key * dt.ld + col;
-        tab[o] = __fadd_rn(tab[o], kvm_ld(dout, (size_t)r * dout.ld + col));
+    for (int i0 = 0; i0 < filled; i0 += 32) {
+      const int2 e = i0 + lane < filled ? list[i0 + lane] : make_int2(0, -1);
+      unsigned mine = __ballot_sync(0xffffffffu, e.y >= 0 && (e.y & (KVM_NWARPS - 1)) == warp);
+      while (mine) {
+        const int src = __ffs(mine) - 1;
+        mine &= mine - 1;
+        const int r = __shfl_sync(0xffffffffu, e.x, src), key = __shfl_sync(0xffffffffu, e.y, src);
+        float* o = tab + (size_t)key * dt.ld;
+        if (vec) {
+          for (int k = lane * 4; k < d; k += 512) {        // four pieces of the row in flight
+            float4 x[4], y[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) if (k + u * 128 < d) { x[u] = *(const float4*)((const float*)dout.p + (size_t)r * dout.ld + k + u * 128); y[u] = *(const float4*)(o + k + u * 128); }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) if (k + u * 128 < d)
+              *(float4*)(o + k + u * 128) = make_float4(__fadd_rn(y[u].x, x[u].x), __fadd_rn(y[u].y, x[u].y), __fadd_rn(y[u].z, x[u].z), __fadd_rn(y[u].w, x[u].w));
+          }
+        } else for (int k = lane; k < d; k += 32) o[k] = __fadd_rn(o[k], kvm_ld(dout, (size_t)r * dout.ld + k));
       }
     }
     kvm_sync();
@@ -105,6 +180,18 @@ KVM_OP_FN void kvm_op_gather_rows(const KvmCtx& c, const int32_t* a) {
   int r0 = a[3], r1 = a[4], d = a[5];
   if (r0 < 0 || r1 < r0 || d <= 0 || !kvm_flat_ok(c, idx, r1) || !kvm_mat_ok(c, dst, r1, d) || !kvm_mat_ok(c, src, 0, d)) {
     c.fail(KVM_OPE_RANGE, r0, r1); return; }
+  if (src.dtype == KVM_BF16 && dst.dtype == KVM_F32 && ((d | src.ld | dst.ld) & 7) == 0 && kvm_vec_ok(src) && kvm_vec_ok(dst)) {      // a decode step's embedding rows: 8 values per access
+    const int cpr = d / 8;
+#pragma unroll 2
+    for (int it = threadIdx.x; it < (r1 - r0) * cpr; it += KVM_NT) {
+      const int r = r0 + it / cpr, col = (it % cpr) * 8, i = ((const int*)idx.p)[r];
+      float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (i < 0 || i >= src.rows) c.fail_any(KVM_OPE_TOKEN, i, r);
+      else kvm_ld8t<true>(src.p, (size_t)i * src.ld + col, v);
+      kvm_st8t<false>(dst.p, (size_t)r * dst.ld + col, v);
+    }
+    return;
+  }
   for (long long e = threadIdx.x; e < (long long)(r1 - r0) * d; e += KVM_NT) {
     int r = r0 + (int)(e / d), col = (int)(e % d), i = ((const int*)idx.p)[r];
     float v = 0.0f;
@@ -379,9 +466,55 @@ KVM_OP_FN void kvm_op_rope_bwd(const KvmCtx& c, const int32_t* a) { kvm_rope(c, 
 
 // ---- cross entropy: the block walks rows; per row one pass for (max, sum) and one for the gradient -------------------------------------
 // MODE bit 0: forward (rowloss, lse); bit 1: backward (dlogits).
+// Short rows (V <= 1024): a warp per row, RP rows of a warp side by side, the row in NV registers per lane over both passes (a block per
+// row spends its time in two block reductions: 408 us for 256 rows of 10 classes).
+template <int MODE, bool LB, int NV, int RP>
+static __device__ void kvm_ce_short_t(const KvmCtx& c, const KvmBuf& lg, const KvmBuf& tg, const KvmBuf& rl, const KvmBuf& ls, const KvmBuf& dl, int r0, int r1, int V, int ignore, float f) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int rb = r0 + warp * RP; rb < r1; rb += KVM_NWARPS * RP) {
+    int t[RP];
+    float v[RP][NV], lse[RP];
+#pragma unroll
+    for (int i = 0; i < RP; ++i) {
+      const int r = min(rb + i, r1 - 1);
+      t[i] = ((const int*)tg.p)[r];
+#pragma unroll
+      for (int j = 0; j < NV; ++j) { const int k = lane + 32 * j; v[i][j] = k < V ? kvm_ldt<LB>(lg.p, (size_t)r * lg.ld + k) : -INFINITY; }
+      if (!(MODE & 1)) lse[i] = ((const float*)ls.p)[r];
+    }
+#pragma unroll
+    for (int i = 0; i < RP; ++i) {
+      const int r = rb + i;
+      if (MODE & 1) {
+        float m = v[i][0], s = 0.0f;
+#pragma unroll
+        for (int j = 1; j < NV; ++j) m = fmaxf(m, v[i][j]);
+        m = kvm_warp_max(m);
+#pragma unroll
+        for (int j = 0; j < NV; ++j) s += __expf(v[i][j] - m);
+        s = kvm_warp_sum(s);
+        lse[i] = t[i] == ignore ? 0.0f : m + logf(s);
+      }
+      if (r >= r1) continue;
+      if (t[i] != ignore && (t[i] < 0 || t[i] >= V)) { if (lane == 0) c.fail_any(KVM_OPE_TOKEN, t[i], r); continue; }
+      if ((MODE & 1) && lane == 0) { ((float*)ls.p)[r] = lse[i]; ((float*)rl.p)[r] = t[i] == ignore ? 0.0f : lse[i] - kvm_ldt<LB>(lg.p, (size_t)r * lg.ld + t[i]); }
+      if (MODE & 2) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+          const int k = lane + 32 * j;
+          if (k < V) kvm_st(dl, (size_t)r * dl.ld + k, t[i] == ignore ? 0.0f : (__expf(v[i][j] - lse[i]) - (k == t[i] ? 1.0f : 0.0f)) * f);
+        }
+      }
+    }
+  }
+}
 template <int MODE, bool LB, bool DB>      // storage types of the logits and of their gradient as template arguments: no type test inside the loops
 static __device__ void kvm_ce_t(const KvmCtx& c, const KvmBuf& lg, const KvmBuf& tg, const KvmBuf& rl, const KvmBuf& ls, const KvmBuf& dl, int r0, int r1, int V,
                          int ignore, float f) {
+  // a short row in registers while a task has rows for most of the warps, or the row is so short that a block cannot use its threads on it
+  if (V <= 32) { kvm_ce_short_t<MODE, LB, 1, 8>(c, lg, tg, rl, ls, dl, r0, r1, V, ignore, f); return; }
+  if (V <= 256) { kvm_ce_short_t<MODE, LB, 8, 2>(c, lg, tg, rl, ls, dl, r0, r1, V, ignore, f); return; }
+  if (V <= 1024) { kvm_ce_short_t<MODE, LB, 32, 1>(c, lg, tg, rl, ls, dl, r0, r1, V, ignore, f); return; }
   float* red = (float*)c.smem;
   const bool vec = (V & 7) == 0 && (lg.ld & 7) == 0 && kvm_vec_ok(lg) && (!(MODE & 2) || ((dl.ld & 7) == 0 && kvm_vec_ok(dl)));
   for (int r = r0; r < r1; ++r) {
@@ -479,6 +612,26 @@ KVM_OP_FN void kvm_op_softmax_ce_reduce(const KvmCtx& c, const int32_t* a) {
 // ---- optimiser ---------------------------------------------------------------------------------------------------------------------
 // AdamW in the reference's strict float32 step order (runtime/ref_gpt.py:457-471): every operation below is one rounded
 // float32 operation with no fused multiply-add, so p, m, v come out bit-identical to the CPU model.
+struct KvmAdamK { float lr, b1, b2, eps, bc1, bc2, omb1, omb2, lrwd, gsc; };
+// Constants of one task; the two double-precision powers run on two warps side by side.  Whole compute group.
+__device__ __forceinline__ KvmAdamK kvm_adamw_consts(const KvmCtx& c, int t, float lr, float b1, float b2, float eps, float wd, float gsc) {
+  float* sh = (float*)c.smem;
+  kvm_sync();
+  if (threadIdx.x == 0) sh[0] = (float)(1.0 - (double)(float)pow((double)b1, (double)t));
+  if (threadIdx.x == 32) sh[1] = (float)(1.0 - (double)(float)pow((double)b2, (double)t));
+  kvm_sync();
+  KvmAdamK k;
+  k.lr = lr; k.b1 = b1; k.b2 = b2; k.eps = eps; k.bc1 = sh[0]; k.bc2 = sh[1]; k.omb1 = (float)(1.0 - (double)b1); k.omb2 = (float)(1.0 - (double)b2); k.lrwd = __fmul_rn(lr, wd); k.gsc = gsc;
+  return k;
+}
+__device__ __forceinline__ void kvm_adamw_step(const KvmAdamK& k, float g, float& p, float& m, float& v) {
+  const float gi = __fmul_rn(g, k.gsc);
+  m = __fadd_rn(__fmul_rn(k.b1, m), __fmul_rn(k.omb1, gi));
+  v = __fadd_rn(__fmul_rn(k.b2, v), __fmul_rn(__fmul_rn(k.omb2, gi), gi));
+  const float decay = __fmul_rn(k.lrwd, p);
+  const float step = __fdiv_rn(__fmul_rn(k.lr, __fdiv_rn(m, k.bc1)), __fadd_rn(__fsqrt_rn(__fdiv_rn(v, k.bc2)), k.eps));
+  p = __fsub_rn(__fsub_rn(p, decay), step);
+}
 static __device__ void kvm_adamw(const KvmCtx& c, const int32_t* a, bool lr_buf) {
   KvmBuf p, g, m, v, gs, st, lrb;
   if (!kvm_buf(c, a[0], KVM_M_F32, p) || !kvm_buf(c, a[1], KVM_M_FLT, g) || !kvm_buf(c, a[2], KVM_M_F32, m) || !kvm_buf(c, a[3], KVM_M_F32, v) ||
@@ -489,35 +642,18 @@ static __device__ void kvm_adamw(const KvmCtx& c, const int32_t* a, bool lr_buf)
   const int t = ((const int*)st.p)[0];
   if (t < 1) { c.fail(KVM_OPE_RANGE, t); return; }
   const float lr = lr_buf ? ((const float*)lrb.p)[0] : kvm_bits_f32(a[8]);
-  const float b1 = kvm_bits_f32(a[9]), b2 = kvm_bits_f32(a[10]), eps = kvm_bits_f32(a[11]), wd = kvm_bits_f32(a[12]);
-  float* sh = (float*)c.smem;
-  kvm_sync();
-  if (threadIdx.x == 0) {
-    sh[0] = (float)(1.0 - (double)(float)pow((double)b1, (double)t));
-    sh[1] = (float)(1.0 - (double)(float)pow((double)b2, (double)t));
-  }
-  kvm_sync();
-  const float bc1 = sh[0], bc2 = sh[1], gsc = gs.p ? ((const float*)gs.p)[0] : 1.0f;
-  const float omb1 = (float)(1.0 - (double)b1), omb2 = (float)(1.0 - (double)b2), lrwd = __fmul_rn(lr, wd);
+  const KvmAdamK k = kvm_adamw_consts(c, t, lr, kvm_bits_f32(a[9]), kvm_bits_f32(a[10]), kvm_bits_f32(a[11]), kvm_bits_f32(a[12]), gs.p ? ((const float*)gs.p)[0] : 1.0f);
   float* pp = (float*)p.p; float* mp = (float*)m.p; float* vp = (float*)v.p;
-  auto upd = [&](float pi, float gi0, float mi0, float vi0, float& po, float& mo, float& vo) {
-    float gi = __fmul_rn(gi0, gsc);
-    mo = __fadd_rn(__fmul_rn(b1, mi0), __fmul_rn(omb1, gi));
-    vo = __fadd_rn(__fmul_rn(b2, vi0), __fmul_rn(__fmul_rn(omb2, gi), gi));
-    float decay = __fmul_rn(lrwd, pi);
-    float step = __fdiv_rn(__fmul_rn(lr, __fdiv_rn(mo, bc1)), __fadd_rn(__fsqrt_rn(__fdiv_rn(vo, bc2)), eps));
-    po = __fsub_rn(__fsub_rn(pi, decay), step);
-  };
   const bool vec = (e0 & 7) == 0 && kvm_vec_ok(p) && kvm_vec_ok(g) && kvm_vec_ok(m) && kvm_vec_ok(v);
   long long body = vec ? ((e1 - e0) & ~7LL) : 0;
   for (long long i = e0 + (long long)threadIdx.x * 8; i + 8 <= e0 + body; i += (long long)KVM_NT * 8) {
     float P[8], G[8], M[8], Vv[8];
     kvm_ld8(p, i, P); kvm_ld8(g, i, G); kvm_ld8(m, i, M); kvm_ld8(v, i, Vv);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) upd(P[j], G[j], M[j], Vv[j], P[j], M[j], Vv[j]);
+    for (int j = 0; j < 8; ++j) kvm_adamw_step(k, G[j], P[j], M[j], Vv[j]);
     kvm_st8(p, i, P); kvm_st8(m, i, M); kvm_st8(v, i, Vv);
   }
-  for (long long i = e0 + body + threadIdx.x; i < e1; i += KVM_NT) upd(pp[i], kvm_ld(g, i), mp[i], vp[i], pp[i], mp[i], vp[i]);
+  for (long long i = e0 + body + threadIdx.x; i < e1; i += KVM_NT) kvm_adamw_step(k, kvm_ld(g, i), pp[i], mp[i], vp[i]);
 }
 KVM_OP_FN void kvm_op_adamw(const KvmCtx& c, const int32_t* a) { kvm_adamw(c, a, false); }
 KVM_OP_FN void kvm_op_adamw_lr(const KvmCtx& c, const int32_t* a) { kvm_adamw(c, a, true); }
@@ -578,8 +714,27 @@ static __device__ void kvm_argmax_rows(const KvmCtx& c, const KvmBuf& lg, const 
   float* rv = (float*)c.smem;
   int* ri = (int*)(rv + KVM_NWARPS);
   for (int r = r0; r < r1; ++r) {
-    float bv = -INFINITY; int bi = 0x7fffffff;
-    for (int k = threadIdx.x; k < V; k += KVM_NT) {
+    float bv = -INFINITY; int bi = 0x7fffffff, k0 = 0;
+    if (lg.dtype == KVM_F32 && (lg.ld & 3) == 0 && kvm_vec_ok(lg)) {
+      // four 16-byte pieces per thread in flight; each thread meets its columns in ascending order (a scalar column per thread and trip
+      // took 92 us for 151,936 logits, one load in flight)
+      const float* row = (const float*)lg.p + (size_t)r * lg.ld;
+      for (; k0 + 16 * KVM_NT <= V; k0 += 16 * KVM_NT) {
+        float4 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = *(const float4*)(row + k0 + (u * KVM_NT + threadIdx.x) * 4);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int k = k0 + (u * KVM_NT + threadIdx.x) * 4;
+          if (x[u].x > bv) { bv = x[u].x; bi = k; }
+          if (x[u].y > bv) { bv = x[u].y; bi = k + 1; }
+          if (x[u].z > bv) { bv = x[u].z; bi = k + 2; }
+          if (x[u].w > bv) { bv = x[u].w; bi = k + 3; }
+        }
+      }
+    }
+#pragma unroll 4
+    for (int k = k0 + threadIdx.x; k < V; k += KVM_NT) {
       float v = kvm_ld(lg, (size_t)r * lg.ld + k);
       if (v > bv || (v == bv && k < bi)) { bv = v; bi = k; }
     }

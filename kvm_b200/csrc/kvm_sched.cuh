@@ -14,6 +14,9 @@
 // dependency counters are armed by a tiny kernel, so no admitter CTA is needed.
 // Every wait has a time limit after which the kernel records KVM_ERR_TIMEOUT and all workers leave.
 #pragma once
+#include "kvm_attn_tc.cuh"
+#include "kvm_dispatch.cuh"
+#include "kvm_hot.cuh"
 #include "kvm_state.cuh"
 
 #define KVM_NSLOT 2               // tasks a worker holds at most: one running and one staged behind it (more slots let a worker hoard ready tasks while others idle)
@@ -221,7 +224,7 @@ __global__ void __launch_bounds__(KVM_EXEC_THREADS, 1) kvm_exec_kernel(KvmDevSta
   extern __shared__ __align__(1024) unsigned char kvm_smem[];
   KvmSlot* slots = (KvmSlot*)kvm_smem;                 // the slot ring
   int* ctl = (int*)(kvm_smem + KVM_NSLOT * sizeof(KvmSlot));   // ctl[0] = TMEM base, ctl[1..] scratch
-  static_assert(KVM_NSLOT * sizeof(KvmSlot) + 96 * sizeof(int) + 288 <= KVM_EXEC_SMEM_HDR, "header too small");      // slots | control words | ... | rope cache (288)
+  static_assert(KVM_NSLOT * sizeof(KvmSlot) + 96 * sizeof(int) <= KVM_EXEC_CTX_OFF && KVM_EXEC_CTX_OFF + sizeof(KvmCtx) + 288 <= KVM_EXEC_SMEM_HDR, "header too small");      // slots | control words | ... | rope cache (288)
   const int tid = threadIdx.x;
   const bool is_sched = tid >= KVM_NT && tid < KVM_NT + 32;
   const int engine_role = tid == KVM_NT + 32 ? 1 : tid == KVM_NT + 64 ? 2 : 0;      // one thread each: TMA producer, MMA issuer
@@ -418,15 +421,18 @@ __global__ void __launch_bounds__(KVM_EXEC_THREADS, 1) kvm_exec_kernel(KvmDevSta
       }
     }
   } else {
-    KvmCtx c;
-    c.nbufs = S.nbufs; c.err = S.err; c.cfg_flags = S.cfg_flags; c.ctl = ctl; c.tmaps = S.tmaps;
-    c.bufs = buf_cache ? (const KvmBuf*)(kvm_smem + KVM_EXEC_SMEM_HDR) : S.bufs;
-    const int used = used_hdr;
-    c.smem = kvm_smem + used; c.smem_bytes = (int)dyn - used;
-    c.engine = engine_on ? 1 : 0; c.gemm_seq = 0;
-    c.rope_cache = (float*)(kvm_smem + KVM_EXEC_SMEM_HDR - 288);
-    c.yield_word = ctl + KVM_CTL_YIELD; c.q_head = S.head; c.q_tail = S.tail;
-    c.deadline = t_begin + S.timeout_ns - S.timeout_ns / 8;      // a task's own wait gives up (and names itself) before the launch's stall limit does
+    // The context lives in shared memory: in registers its fields would be live across every op body, in local memory every look at
+    // it would be a trip to L2 (there is next to no L1 beside the shared memory).
+    KvmCtx& c = *(KvmCtx*)(kvm_smem + KVM_EXEC_CTX_OFF);
+    if (tid == 0) {
+      c.nbufs = S.nbufs; c.err = S.err; c.cfg_flags = S.cfg_flags; c.ctl = ctl; c.tmaps = S.tmaps;
+      c.bufs = buf_cache ? (const KvmBuf*)(kvm_smem + KVM_EXEC_SMEM_HDR) : S.bufs;
+      c.smem = kvm_smem + used_hdr; c.smem_bytes = (int)dyn - used_hdr;
+      c.engine = engine_on ? 1 : 0; c.gemm_seq = 0;
+      c.rope_cache = (float*)(kvm_smem + KVM_EXEC_SMEM_HDR - 288);
+      c.yield_word = ctl + KVM_CTL_YIELD; c.q_head = S.head; c.q_tail = S.tail;
+      c.deadline = t_begin + S.timeout_ns - S.timeout_ns / 8;      // a task's own wait gives up (and names itself) before the launch's stall limit does
+    }
     unsigned tiles = 0;
     int cur = 0;
     while (true) {
@@ -441,33 +447,31 @@ __global__ void __launch_bounds__(KVM_EXEC_THREADS, 1) kvm_exec_kernel(KvmDevSta
         while (kvm_ld_volatile_shared(&sl.state) != 1) {
           if ((++polls & 1023u) == 0 && kvm_globaltimer() - t_begin > 2 * S.timeout_ns) { full = false; break; }   // the scheduler always answers first
         }
-        sl.go = !full ? 0 : (*(volatile int*)&S.err->code == 0 ? 1 : 2);      // 0 leave, 1 run the op, 2 finish the task without running it
+        const int task = full ? sl.task : -1;
+        sl.go = task < 0 ? 0 : (*(volatile int*)&S.err->code == 0 ? 1 : 2);      // 0 leave, 1 run the op, 2 finish the task without running it
+        if (task >= 0) {
+          c.task = task; c.pair = sl.pair; c.gemm_seq = tiles;
+          c.yield_count = S.claim + task;         // the claim word of a task that is not a stacked GEMM tile is free: it counts the task's yields
+          const int wv = sl.desc[8];
+          if (wv >= 0 && wv < S.nvars && kvm_ld_acquire(&S.versions[wv]) < sl.desc[9] + S.ver_off[wv]) kvm_dev_fail(S, KVM_ERR_WAIT_VIOLATION, task, wv);
+          if (S.trace) {
+            S.t_start[task] = kvm_globaltimer(); S.t_smid[task] = (int)kvm_smid();
+            if (c.pair >= 0) { S.t_start[c.pair] = S.t_start[task]; S.t_smid[c.pair] = S.t_smid[task]; }
+          }
+        }
       }
       kvm_sync();
       const int go = kvm_ld_volatile_shared(&sl.go);
       if (go == 0) break;
-      const int task = sl.task;
-      if (task < 0) break;
-      c.task = task; c.pair = sl.pair;
-      if (tid == 0) {
-        const int wv = sl.desc[8];
-        if (wv >= 0 && wv < S.nvars && kvm_ld_acquire(&S.versions[wv]) < sl.desc[9] + S.ver_off[wv]) kvm_dev_fail(S, KVM_ERR_WAIT_VIOLATION, task, wv);
-        if (S.trace) {
-          S.t_start[task] = kvm_globaltimer(); S.t_smid[task] = (int)kvm_smid();
-          if (c.pair >= 0) { S.t_start[c.pair] = S.t_start[task]; S.t_smid[c.pair] = S.t_smid[task]; }
-        }
-      }
       const int op = sl.desc[0];
       const bool tile = sl.kind == 1;
-      c.gemm_seq = tiles;
-      c.yield_count = S.claim + task;           // the claim word of a task that is not a stacked GEMM tile is free: it counts the task's yields
-      if (op != 0 && go == 1) kvm_dispatch(c, op, sl.args, sl.aux);
-      if (tile) ++tiles;
+      if (tile) { if (go == 1) kvm_tce_tile(c, sl.args); ++tiles; }
+      else if (op != 0 && go == 1 && !kvm_hot<true>(c, op, sl.args)) kvm_dispatch(c, op, sl.args, sl.aux);
       // this task's generic-proxy writes (global results, shared scratch) ordered before any later TMA access to them
       asm volatile("fence.proxy.async;" ::: "memory");
       kvm_sync();                       // every thread's writes happen before thread 0's fence below (barrier, then a cumulative gpu-scope fence)
       if (tid == 0) {
-        if (S.trace) { S.t_end[task] = kvm_globaltimer(); if (c.pair >= 0) S.t_end[c.pair] = S.t_end[task]; }
+        if (S.trace) { S.t_end[c.task] = kvm_globaltimer(); if (c.pair >= 0) S.t_end[c.pair] = S.t_end[c.task]; }
         __threadfence();
         const int y = ctl[KVM_CTL_YIELD];
         ctl[KVM_CTL_YIELD] = 0;

@@ -61,8 +61,7 @@ __device__ __forceinline__ void kvm_dev_fail(const KvmDevState& S, int code, int
 #define KVM_NCLASS 4
 __device__ __forceinline__ int kvm_class_of(int priority) { return priority < 0 ? 0 : (priority >> 3) >= KVM_NCLASS ? KVM_NCLASS - 1 : (priority >> 3); }
 
-static __device__ void kvm_dispatch(const KvmCtx& c, int op, const int32_t* args, const int4& aux);
-
 #define KVM_EXEC_SMEM_HDR 2048     // slots + control words at the start of dynamic shared memory
+#define KVM_EXEC_CTX_OFF 1024       // the compute group's KvmCtx in that header
 #define KVM_BUFCACHE_BYTES 32768    // shared-memory copy of the buffer table (up to 1024 buffers), after the header
 

@@ -16,7 +16,9 @@
 //
 // Every wait is bounded (time limit); on expiry KVM_ERR_TIMEOUT is recorded, every CTA leaves, copies in flight are awaited.
 #pragma once
+#include "kvm_attn_tc.cuh"
 #include "kvm_dispatch.cuh"
+#include "kvm_ops_decode.cuh"
 #include "kvm_static_api.h"
 
 #define KVM_ST_SLOTS 4                 // record ring depth (tasks fetched ahead)
@@ -38,7 +40,9 @@ struct KvmStSlot {
   int j0, j1, newrow;         // attention: key range of the split, index of the appended key inside it (-1 none)
   KvmBuf lb[7];               // streamed tasks: the buffer-table entries of the task's buffer arguments (argument j -> lb[j]), looked up once by the front warp
 };
-static_assert(sizeof(KvmStSlot) * KVM_ST_SLOTS + 128 * 4 + 64 + 288 + 128 <= KVM_ST_HDR, "static header too small");      // slots | control words | ... | rope cache (288) | ring barriers (128)
+#define KVM_ST_CTX_BYTES 192            // the compute group's KvmCtx, in front of the rope cache
+static_assert(sizeof(KvmCtx) <= KVM_ST_CTX_BYTES, "context grew");
+static_assert(sizeof(KvmStSlot) * KVM_ST_SLOTS + 128 * 4 + KVM_ST_CTX_BYTES + 288 + 128 <= KVM_ST_HDR, "static header too small");      // slots | control words | ... | rope cache (288) | ring barriers (128)
 
 __device__ __forceinline__ bool kvm_mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -91,7 +95,7 @@ __device__ __forceinline__ bool kvm_ring_wait_warp(const KvmRing& ring, unsigned
 // Stage use `cit + ci` holds rows n0 + ci*R .. of the weight matrix in full (R*K*2 bytes).  All sixteen warps consume: warp = (row r of the
 // stage, part of K); the activation row v = bf16(prologue(x)) is staged once as bf16.  Partial sums are added in part order.
 // Semantics as kvm_op_gemv_bf16 (runtime/ref_extra.py:398-415).  Always consumes its nchunks stage uses, also after an error.
-KVM_OP_FN void kvm_gemv_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing& ring, unsigned cit, int R, int NC, unsigned long long deadline,
+static __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing& ring, unsigned cit, int R, int NC, unsigned long long deadline,
                                      unsigned long long t_task, int* stamp) {
   KvmBuf x, x2, gm, w, out, res;
   const int n0 = a[6], n1 = a[7], K = a[8], pro = a[9];
@@ -795,15 +799,17 @@ __global__ void __launch_bounds__(KVM_NT + 32, 1) kvm_static_kernel(KvmStaticSta
     }
     sctl[2] = (int)pit;
   } else {
-    KvmCtx c;
-    c.nbufs = S.nbufs; c.err = S.err; c.cfg_flags = S.cfg_flags; c.ctl = ctl; c.tmaps = S.tmaps; c.pair = -1; c.engine = 0; c.gemm_seq = 0;
-    c.rope_cache = (float*)(kvm_smem + KVM_ST_HDR - 128 - 288);
-    c.yield_word = nullptr; c.yield_count = nullptr; c.q_head = c.q_tail = nullptr;      // program order: a waiting task waits in place
-    c.deadline = deadline - S.timeout_ns / 8;      // a task's own wait gives up (and names itself) before the launch's stall limit does
-    c.bufs = buf_cache ? (const KvmBuf*)(kvm_smem + KVM_ST_HDR) : S.bufs;
-    const int used = KVM_ST_HDR + (buf_cache ? cache_bytes : 0);
-    c.smem = kvm_smem + used;
-    c.smem_bytes = (int)dyn - used - (use_ring ? ring_bytes : 0);
+    KvmCtx& c = *(KvmCtx*)(kvm_smem + KVM_ST_HDR - 128 - 288 - KVM_ST_CTX_BYTES);      // in shared memory (see kvm_sched.cuh)
+    if (tid == 0) {
+      c.nbufs = S.nbufs; c.err = S.err; c.cfg_flags = S.cfg_flags; c.ctl = ctl; c.tmaps = S.tmaps; c.pair = -1; c.engine = 0; c.gemm_seq = 0;
+      c.rope_cache = (float*)(kvm_smem + KVM_ST_HDR - 128 - 288);
+      c.yield_word = nullptr; c.yield_count = nullptr; c.q_head = c.q_tail = nullptr;      // program order: a waiting task waits in place
+      c.deadline = deadline - S.timeout_ns / 8;      // a task's own wait gives up (and names itself) before the launch's stall limit does
+      c.bufs = buf_cache ? (const KvmBuf*)(kvm_smem + KVM_ST_HDR) : S.bufs;
+      const int used = KVM_ST_HDR + (buf_cache ? cache_bytes : 0);
+      c.smem = kvm_smem + used;
+      c.smem_bytes = (int)dyn - used - (use_ring ? ring_bytes : 0);
+    }
     unsigned cit = 0;
     int finished = 0;
     for (int i = 0; i < n; ++i) {
@@ -815,12 +821,12 @@ __global__ void __launch_bounds__(KVM_NT + 32, 1) kvm_static_kernel(KvmStaticSta
           if ((++polls & 1023u) == 0 && kvm_globaltimer() > deadline + S.timeout_ns) { st = 3; break; }      // the front warp always answers first
         }
         sl.go = st == 3 ? 0 : (*(volatile int*)&S.err->code == 0 ? 1 : 2);
+        c.task = sl.task;
       }
       kvm_sync();
       const int go = kvm_ld_volatile_shared(&sl.go);
       if (go == 0) break;
       const int task = sl.task;
-      c.task = task;
       unsigned long long t_task = 0;
       if (tid == 0 && S.trace) { t_task = kvm_globaltimer(); S.t_start[task] = t_task; sctl[3] = 0; }
       const int op = sl.desc[0], kind = sl.kind, nch = sl.nchunks;
