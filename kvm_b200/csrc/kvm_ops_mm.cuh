@@ -29,6 +29,29 @@ __device__ __forceinline__ float kvm_mm_epilogue(const KvmMmArgs& g, float acc, 
   return v;
 }
 
+// Four neighbouring columns of a row.  With float32 buffers on 16-byte boundaries everything the epilogue reads is loaded as vectors
+// before the first use; otherwise column by column.
+template <bool VEC>
+__device__ __forceinline__ void kvm_mm_epilogue4(const KvmMmArgs& g, const float (&acc)[4], int m, int n, int n_end) {
+  const bool simple = VEC && n + 4 <= n_end && !(g.flags & (4 | 512)) && g.out.dtype == KVM_F32 && (g.out.ld & 3) == 0 && kvm_vec_ok(g.out) && (!g.bias.p || kvm_vec_ok(g.bias)) &&
+                      (!g.res.p || (g.res.dtype == KVM_F32 && (g.res.ld & 3) == 0 && kvm_vec_ok(g.res))) &&
+                      (!g.pre.p || (g.pre.dtype == KVM_F32 && (g.pre.ld & 3) == 0 && kvm_vec_ok(g.pre)));
+  if (!simple) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) if (n + j < n_end) kvm_st(g.out, (size_t)m * g.out.ld + n + j, kvm_mm_epilogue(g, acc[j], m, n + j));
+    return;
+  }
+  float v[4] = {acc[0], acc[1], acc[2], acc[3]}, bi[4] = {0, 0, 0, 0}, re[4] = {0, 0, 0, 0};
+  if (g.bias.p) *(float4*)bi = *(const float4*)((const float*)g.bias.p + n);
+  if (g.res.p) *(float4*)re = *(const float4*)((const float*)g.res.p + (size_t)m * g.res.ld + n);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) { v[j] = __fmul_rn(v[j], g.alpha); if (g.bias.p) v[j] = __fadd_rn(v[j], bi[j]); }
+  if (g.pre.p) *(float4*)((float*)g.pre.p + (size_t)m * g.pre.ld + n) = make_float4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) { if (g.flags & 8) v[j] = kvm_gelu(v[j]); if (g.res.p) v[j] = __fadd_rn(v[j], re[j]); }
+  *(float4*)((float*)g.out.p + (size_t)m * g.out.ld + n) = make_float4(v[0], v[1], v[2], v[3]);
+}
+
 // Decode and check the 13 argument words shared by matmul_tile / matmul_tile_bf16 / matmul_mma_bf16.
 static __device__ bool kvm_mm_args(const KvmCtx& c, const int32_t* a, int kind /*0 f32 tile, 1 bf16 tile, 2 mma 128x256*/, KvmMmArgs& g) {
   const int opmask = kind == 0 ? KVM_M_F32 : KVM_M_FLT, omask = kind == 0 ? KVM_M_F32 : KVM_M_FLT;
@@ -51,54 +74,111 @@ static __device__ bool kvm_mm_args(const KvmCtx& c, const int32_t* a, int kind /
   return true;
 }
 
-// SIMT tile: 64x64 sub-tiles, K staged through shared memory 32 at a time; thread = (row, 8 columns).
-static __device__ void kvm_mm_simt(const KvmCtx& c, const KvmMmArgs& g) {
-  float (*As)[65] = (float (*)[65])c.smem;                  // [32][65]: As[k][m]
-  float (*Bs)[64] = (float (*)[64])(c.smem + 32 * 65 * 4);  // [32][64]: Bs[k][n]
-  const bool ta = g.flags & 1, tb = g.flags & 2;
+// ---- SIMT tile ----------------------------------------------------------------------------------------------------------------
+// 64x64 sub-tiles, K staged through shared memory 32 at a time.  The first eight warps multiply, a thread owns 4 rows x 4 columns:
+// per k two LDS.128 for 16 products.  The exact multiply-then-add (two roundings per step, no fused multiply-add) needs 64 issue
+// cycles per k and SM, the two loads 64 cycles of shared-memory bandwidth; the form before (one row x 8 columns per thread, all
+// sixteen warps) asked shared memory for 3 loads per 8 products.  The packed f32x2 instructions do not help: the compiler
+// contracts a packed multiply and add into a packed FMA.
+// All sixteen warps stage: chunk i+2 is in flight from global memory (registers) while chunk i is multiplied, chunk i+1 is in the
+// other shared buffer: one barrier per chunk.  Both arrays are stored [k][.] with their 16-byte units XOR-swizzled by (k / 4) & 7, so
+// that the transposing stores (k contiguous in global memory) spread over the banks as well as the loads do.
+// A warp whose rows or columns lie outside the tile (10-column logits) skips the arithmetic.
+#define KVM_SM_A_BYTES (32 * 64 * 4)
+#define KVM_SM_STAGE (2 * KVM_SM_A_BYTES)
+
+// Four consecutive elements along the contiguous axis of an operand: row `r` (outer index), columns c..c+3, zero outside [rows, cols).
+template <bool VEC>
+__device__ __forceinline__ void kvm_sm_fetch(const KvmBuf& b, bool round_ops, int r, int c, int rows, int cols, float (&v)[4]) {
+  if (r < rows && c + 4 <= cols && VEC) {
+    const float4 f = *(const float4*)((const float*)b.p + (size_t)r * b.ld + c);
+    v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = (r < rows && c + j < cols) ? (VEC ? ((const float*)b.p)[(size_t)r * b.ld + c + j] : kvm_ld(b, (size_t)r * b.ld + c + j)) : 0.0f;
+  }
+  if (!VEC && round_ops) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = kvm_bf16_round(v[j]);
+  }
+}
+template <bool VEC>
+static __device__ __noinline__ void kvm_mm_simt_t(const KvmCtx& c, const KvmMmArgs& g) {
+  const bool ta = g.flags & 1, tb = g.flags & 2, two = c.smem_bytes >= 2 * KVM_SM_STAGE;
   const int m_end = min(g.m0 + g.tm, g.M), n_end = min(g.n0 + g.tn, g.N);
-  const int row = threadIdx.x >> 3, cg = (threadIdx.x & 7) * 8;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rg = (warp & 1) * 8 + (lane & 7), cg = (warp >> 1) * 4 + (lane >> 3);      // warps 0..7: rows 4 rg .., columns 4 cg ..
+  // this thread's share of a chunk: A element (am, ak .. ak+3) or, transposed, (am .. am+3, ak); B likewise
+  const int am = ta ? (tid & 15) * 4 : tid >> 3, ak = ta ? tid >> 4 : (tid & 7) * 4;
+  const int bn = tb ? tid >> 3 : (tid & 15) * 4, bk = tb ? (tid & 7) * 4 : tid >> 4;
   for (int mb = g.m0; mb < m_end; mb += 64)
     for (int nb = g.n0; nb < n_end; nb += 64) {
-      float acc[8];
+      const bool active = warp < 8 && mb + (warp & 1) * 32 < m_end && nb + (warp >> 1) * 16 < n_end;
+      float acc[4][4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
-      for (int k0 = 0; k0 < g.K; k0 += 32) {
-        kvm_sync();
-        for (int e = threadIdx.x; e < 32 * 64; e += KVM_NT) {
-          int kk, mm;
-          if (ta) { kk = e >> 6; mm = e & 63; } else { mm = e >> 5; kk = e & 31; }
-          float v = 0.0f;
-          if (k0 + kk < g.K && mb + mm < m_end) {
-            v = ta ? kvm_ld(g.a, (size_t)(k0 + kk) * g.a.ld + mb + mm) : kvm_ld(g.a, (size_t)(mb + mm) * g.a.ld + k0 + kk);
-            if (g.round_ops) v = kvm_bf16_round(v);
-          }
-          As[kk][mm] = v;
-          int kb, nn;
-          if (tb) { nn = e >> 5; kb = e & 31; } else { kb = e >> 6; nn = e & 63; }
-          float w = 0.0f;
-          if (k0 + kb < g.K && nb + nn < n_end) {
-            w = tb ? kvm_ld(g.b, (size_t)(nb + nn) * g.b.ld + k0 + kb) : kvm_ld(g.b, (size_t)(k0 + kb) * g.b.ld + nb + nn);
-            if (g.round_ops) w = kvm_bf16_round(w);
-          }
-          Bs[kb][nn] = w;
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+      float xa[2][4], xb[2][4];
+      auto fetch = [&](int k0, float (&va)[4], float (&vb)[4]) {
+        if (ta) kvm_sm_fetch<VEC>(g.a, g.round_ops, k0 + ak, mb + am, g.K, m_end, va);
+        else kvm_sm_fetch<VEC>(g.a, g.round_ops, mb + am, k0 + ak, m_end, g.K, va);
+        if (tb) kvm_sm_fetch<VEC>(g.b, g.round_ops, nb + bn, k0 + bk, n_end, g.K, vb);
+        else kvm_sm_fetch<VEC>(g.b, g.round_ops, k0 + bk, nb + bn, g.K, n_end, vb);
+      };
+      auto put1 = [&](unsigned char* st, int o, int k, bool along_k, const float (&v)[4]) {      // element (o, k) of a [k][64] array, four along k or along o
+        const int q = (k >> 2) & 7;
+        if (along_k) {
+          const int at = (((o >> 2) ^ q) << 4) + (o & 3) * 4;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) *(float*)(st + (k + j) * 256 + at) = v[j];
+        } else *(float4*)(st + k * 256 + (((o >> 2) ^ q) << 4)) = make_float4(v[0], v[1], v[2], v[3]);
+      };
+      auto put = [&](unsigned char* st, const float (&va)[4], const float (&vb)[4]) { put1(st, am, ak, !ta, va); put1(st + KVM_SM_A_BYTES, bn, bk, tb, vb); };
+      const int nch = (g.K + 31) / 32;
+      fetch(0, xa[0], xb[0]);
+      if (nch > 1) fetch(32, xa[1], xb[1]);
+      kvm_sync();                                           // whatever used the scratch before is done with it
+      put(c.smem, xa[0], xb[0]);
+      for (int i = 0; i < nch; ++i) {
+        kvm_sync();                                         // chunk i is in its buffer
+        unsigned char* st = c.smem + (two ? (i & 1) * KVM_SM_STAGE : 0);
+        if (i + 2 < nch) fetch((i + 2) * 32, xa[0], xb[0]);
+        if (two && i + 1 < nch) put(c.smem + ((i + 1) & 1) * KVM_SM_STAGE, xa[1], xb[1]);
+        if (active) {
+          const int kmax = min(32, g.K - i * 32);
+          auto step = [&](int k, int q) {
+            const float4 x = *(const float4*)(st + k * 256 + ((rg ^ q) << 4)), y = *(const float4*)(st + KVM_SM_A_BYTES + k * 256 + ((cg ^ q) << 4));
+            const float xr[4] = {x.x, x.y, x.z, x.w}, yc[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) acc[r][j] = __fadd_rn(acc[r][j], __fmul_rn(xr[r], yc[j]));
+          };
+          if (kmax == 32) {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) step(k, (k >> 2) & 7);
+          } else
+            for (int k = 0; k < kmax; ++k) step(k, (k >> 2) & 7);
         }
-        kvm_sync();
-        const int kmax = min(32, g.K - k0);
-        for (int kk = 0; kk < kmax; ++kk) {
-          const float x = As[kk][row];
+        if (!two && i + 1 < nch) { kvm_sync(); put(c.smem, xa[1], xb[1]); }
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[j] = __fadd_rn(acc[j], __fmul_rn(x, Bs[kk][cg + j]));
+        for (int j = 0; j < 4; ++j) { xa[1][j] = xa[0][j]; xb[1][j] = xb[0][j]; }
+      }
+      if (active) {
+        const int n = nb + cg * 4;
+#pragma unroll
+        for (int rr = 0; rr < 4; ++rr) {
+          const int m = mb + rg * 4 + rr;
+          if (m < m_end) kvm_mm_epilogue4<VEC>(g, acc[rr], m, n, n_end);
         }
       }
-      const int m = mb + row;
-      if (m < m_end)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int n = nb + cg + j;
-          if (n < n_end) kvm_st(g.out, (size_t)m * g.out.ld + n, kvm_mm_epilogue(g, acc[j], m, n));
-        }
     }
+}
+static __device__ void kvm_mm_simt(const KvmCtx& c, const KvmMmArgs& g) {
+  // vector loads: float32 operands as they are (no rounding), rows and tile origin on 16-byte boundaries
+  const bool vec = !g.round_ops && g.a.dtype == KVM_F32 && g.b.dtype == KVM_F32 && ((g.a.ld | g.b.ld | g.m0 | g.n0) & 3) == 0 && kvm_vec_ok(g.a) && kvm_vec_ok(g.b);
+  if (vec) kvm_mm_simt_t<true>(c, g); else kvm_mm_simt_t<false>(c, g);
 }
 
 KVM_OP_FN void kvm_op_matmul_tile(const KvmCtx& c, const int32_t* a) {
