@@ -279,7 +279,8 @@ def build_decode_rows(c: DecodeConfig, exact_caches: bool = False) -> Graph:
         x = xn
     logits = g.buffer('logits', B, V)
     gemv('head', x, 'wb.head', logits, V, d, 1, gamma='w.lnf', prio=1)
-    g.task('argmax', {'logits': logits, 'out': tok, 'r0': 0, 'r1': B, 'V': V}, [logits], [tok], 1, 'argmax')
+    for u in range(B):       # a task per user: one after the other in a single task they would be the longest phase of the step
+        g.task('argmax', {'logits': logits, 'out': tok, 'r0': u, 'r1': u + 1, 'V': V}, [(logits, (u, u + 1))], [(tok, (u, u + 1))], 1, f'argmax.{u}')
     g.task('counter_inc', {'x': lens, 'i0': 0, 'i1': B, 'delta': 1}, [lens], [lens], 0, 'advance')
     return g
 
