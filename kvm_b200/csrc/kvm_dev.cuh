@@ -189,8 +189,10 @@ __device__ __forceinline__ float kvm_warp_max(float v) {
   for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
-// Named barrier over the KVM_NT compute threads only (barrier 1; barrier 0 = whole CTA including the scheduler warp).
-__device__ __forceinline__ void kvm_sync() { asm volatile("bar.sync 1, %0;" ::"n"(KVM_NT) : "memory"); }
+// Named barrier over the KVM_NT compute threads only (barrier 1; barrier 0 = whole CTA including the scheduler warp).  A warp arrives
+// once: bar.sync counts a warp's arrival per executed instruction, so lanes that a branch or a polling loop has left apart must meet
+// first, or a warp that arrives in two pieces completes the barrier in another warp's place.
+__device__ __forceinline__ void kvm_sync() { __syncwarp(); asm volatile("bar.sync 1, %0;" ::"n"(KVM_NT) : "memory"); }
 
 // Block-wide sum; `red` is a KVM_NWARPS-element shared scratch. All compute threads get the result.
 template <class T>

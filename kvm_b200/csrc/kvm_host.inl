@@ -739,7 +739,7 @@ extern "C" int kvm_trace_detail(KvmExec* h, int32_t* detail, int32_t n) {
 extern "C" int kvm_launch_info(KvmExec* h, int32_t* workers, int32_t* threads, int32_t* smem_bytes) {
   if (!h) return KVM_E_ARG;
   if (workers) *workers = h->workers;
-  if (threads) *threads = h->use_static ? KVM_NT + 32 : KVM_EXEC_THREADS;
+  if (threads) *threads = h->use_static ? KVM_ST_THREADS : KVM_EXEC_THREADS;
   if (smem_bytes) *smem_bytes = h->smem_bytes;
   return 0;
 }

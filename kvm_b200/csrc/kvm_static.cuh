@@ -28,6 +28,7 @@
 struct KvmStSlot {
   int task;
   int state;                  // 0 free, 1 fetched, 2 ready, 3 leave
+  int pos;                    // position in the worker's list of the record the slot holds
   int go;
   int kind;                   // 0 generic op, 1 streamed gemv (one activation row, SIMT consumer), 2 streamed split attention, 3 streamed gemv on tensor cores (rows)
   int nchunks;                // stage uses of this task
@@ -92,167 +93,218 @@ __device__ __forceinline__ bool kvm_ring_wait_warp(const KvmRing& ring, unsigned
 }
 
 // ---- streamed GEMV, consumer side --------------------------------------------------------------------------------------------
-// Stage use `cit + ci` holds rows n0 + ci*R .. of the weight matrix in full (R*K*2 bytes).  All sixteen warps consume: warp = (row r of the
-// stage, part of K); the activation row v = bf16(prologue(x)) is staged once as bf16.  Partial sums are added in part order.
-// Semantics as kvm_op_gemv_bf16 (runtime/ref_extra.py:398-415).  Always consumes its nchunks stage uses, also after an error.
-static __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing& ring, unsigned cit, int R, int NC, unsigned long long deadline,
-                                     unsigned long long t_task, int* stamp) {
-  KvmBuf x, x2, gm, w, out, res;
-  const int n0 = a[6], n1 = a[7], K = a[8], pro = a[9];
-  const float eps = kvm_bits_f32(a[10]);
-  bool ok = kvm_buf_local(c, lb, a, 0, KVM_M_FLT, x) && kvm_buf_local(c, lb, a, 1, KVM_M_FLT, x2, true) && kvm_buf_local(c, lb, a, 2, KVM_M_F32, gm, true) &&
-            kvm_buf_local(c, lb, a, 3, KVM_M_BF16, w) && kvm_buf_local(c, lb, a, 4, KVM_M_FLT, out) && kvm_buf_local(c, lb, a, 5, KVM_M_FLT, res, true);
-  const int rows = n1 - n0;
-  const int KP = KVM_ST_ARRIVALS / R;
-  const int fixed = ((K * 2 + 127) & ~127) + 256 + ((rows + 7) & ~7) * KP * 4;
-  if (ok && (pro < 0 || pro > 2 || (pro == 1 && !gm.p) || (pro == 2 && !x2.p) || fixed > c.smem_bytes)) { c.fail(KVM_OPE_SHAPE, K, pro); ok = false; }
-  if (ok) ok = kvm_mat_ok(c, x, 1, K) && kvm_mat_ok(c, x2, 1, K) && kvm_flat_ok(c, gm, K) && kvm_mat_ok(c, out, 1, n1) && kvm_mat_ok(c, res, 1, n1);
-  __nv_bfloat16* vs = (__nv_bfloat16*)c.smem;
-  float* red = (float*)(c.smem + ((K * 2 + 127) & ~127));
-  float* parts = red + 64;                                 // [rows][KP]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  kvm_sync();                                              // the previous task is done with the scratch
-  if (ok) {
-    // ---- prologue: v = bf16(pro(x)) (all 16 warps)
-    if (pro == 1 && K <= 16 * KVM_NT && x.dtype == KVM_F32 && kvm_vec_ok(x) && kvm_vec_ok(gm)) {
-      // float32 row of up to 8192 values: four 16-byte loads of x and of gamma per thread, all in flight together (no storage-type
-      // test between them: with one, every load waits for the one before it), the row stays in registers for the statistics
-      float4 xr[4], gr[4];
-      float q = 0.0f;
+// Stage use `cit + ci` holds rows n0 + ci*R .. of the weight matrix in full (R*K*2 bytes).  All sixteen warps consume: warp = (row group,
+// part of K), KP parts of 256 columns or more, 16 / KP row groups of up to eight rows a stage.  A thread owns J pieces of eight columns
+// of the activation row v = bf16(prologue(x)): it computes them itself and keeps them as float32 over the task, so the activations cost
+// no shared memory and the prologue has one barrier at most (the sum of squares).  The eight rows' sums leave a warp through one
+// transposing reduction (nine shuffles for eight rows).
+// What bounds it: a 64 KB stage is 1.5 us of an SM's share of HBM and about 700 issue cycles here; every value of the loop has to stay
+// in registers, since a spilled one costs an L2 round trip per stage (the stages leave 28 KB of L1 for 512 threads' local memory).
+// Partial sums are added in part order.  Semantics as kvm_op_gemv_bf16 (runtime/ref_extra.py:398-415).  Always consumes its nchunks
+// stage uses, also after an error.
+__device__ __forceinline__ float kvm_silu_fast(float x) { return __fdividef(x, 1.0f + __expf(-x)); }      // for values that are rounded to bf16 next
+__device__ __forceinline__ unsigned long long kvm_pack2(float lo, float hi) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ void kvm_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+__device__ __forceinline__ uint4 kvm_pack_bf16x8(const float (&v)[8]) {
+  uint4 pk;
+  __nv_bfloat162* hh = (__nv_bfloat162*)&pk;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int k = (tid + u * KVM_NT) * 4;
-        xr[u] = k < K ? *(const float4*)((const float*)x.p + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        gr[u] = k < K ? *(const float4*)((const float*)gm.p + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      }
+  for (int j = 0; j < 4; ++j) hh[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+  return pk;
+}
+// acc += eight bf16 weights * eight float32 activations
+__device__ __forceinline__ void kvm_gv_dot8(unsigned long long& acc, const uint4& w, const unsigned long long (&x)[4]) {
+  const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-      for (int u = 0; u < 4; ++u) q += xr[u].x * xr[u].x + xr[u].y * xr[u].y + xr[u].z * xr[u].z + xr[u].w * xr[u].w;
-      q = kvm_block_sum(q, red);
-      const float rs = 1.0f / sqrtf(q / K + eps);
+  for (int i = 0; i < 4; ++i) kvm_fma2(acc, kvm_pack2(__uint_as_float(u[i] << 16), __uint_as_float(u[i] & 0xffff0000u)), x[i]);
+}
+// v = bf16(pro(x)) to shared memory, any storage types and alignments.
+static __device__ __noinline__ void kvm_gemv_stage_x(const KvmBuf* lb, __nv_bfloat16* vs, float* red, int K, int pro, float eps) {
+  const KvmBuf x = lb[0], x2 = lb[1];
+  const int tid = threadIdx.x;
+  float rs = 1.0f;
+  if (pro == 1) {
+    float q = 0.0f;
+    for (int k = tid; k < K; k += KVM_NT) { const float t = kvm_ld(x, k); q += t * t; }
+    q = kvm_block_sum(q, red);
+    rs = 1.0f / sqrtf(q / K + eps);
+  }
+  for (int k = tid; k < K; k += KVM_NT) {
+    const float p = kvm_ld(x, k);
+    vs[k] = __float2bfloat16_rn(pro == 1 ? p * rs * ((const float*)lb[2].p)[k] : pro == 2 ? kvm_silu(p) * kvm_ld(x2, k) : p);
+  }
+}
+// Warps a row is split over (a power of two: what is left of the sixteen takes other rows) and rows a stage holds; the front warp and
+// the consumers compute the same.
+__device__ __forceinline__ int kvm_gv_parts(int K) { return K > 2048 ? 16 : K > 1024 ? 8 : K > 512 ? 4 : K > 256 ? 2 : 1; }
+__device__ __forceinline__ int kvm_gv_rows(int K) { return (KVM_NWARPS / kvm_gv_parts(K)) * min(8, KVM_ST_STAGE / (K * 2 * (KVM_NWARPS / kvm_gv_parts(K)))); }
+#define KVM_GV_RED 256                                     // scratch: reduction words | partial sums [KP][rows]
+
+// Sums over the warp's lanes of eight values per lane: lane 4 r + (0..3) ends with the total of value r.
+__device__ __forceinline__ float kvm_gv_reduce8(float (&s)[8], int lane) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int k = (tid + u * KVM_NT) * 4;
-        if (k < K) {
-          *(__nv_bfloat162*)(vs + k) = __floats2bfloat162_rn(xr[u].x * rs * gr[u].x, xr[u].y * rs * gr[u].y);
-          *(__nv_bfloat162*)(vs + k + 2) = __floats2bfloat162_rn(xr[u].z * rs * gr[u].z, xr[u].w * rs * gr[u].w);
+  for (int i = 0; i < 4; ++i) {                            // lanes with bit 4 keep values 4..7
+    const float keep = lane & 16 ? s[i + 4] : s[i], give = lane & 16 ? s[i] : s[i + 4];
+    s[i] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float keep = lane & 8 ? s[i + 2] : s[i], give = lane & 8 ? s[i] : s[i + 2];
+    s[i] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+  }
+  const float keep = lane & 4 ? s[1] : s[0], give = lane & 4 ? s[0] : s[1];
+  float t = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+  t += __shfl_xor_sync(0xffffffffu, t, 2);
+  return t + __shfl_xor_sync(0xffffffffu, t, 1);
+}
+
+// The checks of kvm_op_gemv_bf16 on the slot's table entries, one entry at a time.
+__device__ __forceinline__ bool kvm_gv_args_ok(const KvmCtx& c, const int32_t* a, const KvmBuf* lb) {
+  const int K = a[8], n1 = a[7], pro = a[9];
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < 6; ++j) {
+    KvmBuf b;
+    ok = ok && kvm_buf_local(c, lb, a, j, j == 3 ? KVM_M_BF16 : j == 2 ? KVM_M_F32 : KVM_M_FLT, b, j == 1 || j == 2 || j == 5);
+    if (ok && ((j == 1 && pro == 2 && !b.p) || (j == 2 && pro == 1 && !b.p) || pro < 0 || pro > 2)) { c.fail(KVM_OPE_SHAPE, K, pro); ok = false; }
+    if (ok && j != 3) ok = j == 2 ? kvm_flat_ok(c, b, K) : kvm_mat_ok(c, b, 1, j >= 4 ? n1 : K);
+  }
+  return ok;
+}
+
+template <int J>
+__device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing ring, unsigned cit, int R, int NC, int* stamp) {
+  const int K = a[8], rows = a[7] - a[6], KP = kvm_gv_parts(K);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = warp & (KP - 1), rg = warp / KP, m = R * KP / KVM_NWARPS;      // rows rg*m .. of a stage
+  const int k0 = (part * 32 + lane) * 8, kstep = KP * 256;
+  float* parts = (float*)(c.smem + KVM_GV_RED);            // [KP][rows]
+  bool ok;
+  constexpr bool PACK = J > 3;                             // activations kept as bf16 pairs
+  unsigned long long xs[PACK ? 1 : J][4];
+  uint4 xp[PACK ? J : 1];
+  float rv = 0.0f;                                         // this thread's residual value, on its way while the weights stream
+  {
+    const int pro = a[9];
+    auto put = [&](int j, const float (&t)[8]) {
+      if (PACK) xp[PACK ? j : 0] = kvm_pack_bf16x8(t);
+      else
+#pragma unroll
+        for (int i = 0; i < 4; ++i) xs[PACK ? 0 : j][i] = kvm_pack2(t[2 * i], t[2 * i + 1]);
+    };
+    ok = kvm_gv_args_ok(c, a, lb);
+    if (ok && a[5] >= 0 && tid < rows) rv = kvm_ld(lb[5], a[6] + tid);
+    const KvmBuf x = lb[0];
+    bool f32 = x.dtype == KVM_F32 && kvm_vec_ok(x);
+    const float* up = nullptr;                             // the prologue's second operand: gamma or the up projection
+    if (pro == 1) { up = (const float*)lb[2].p; f32 = f32 && kvm_vec_ok(lb[2]); }
+    else if (pro == 2) { up = (const float*)lb[1].p; f32 = f32 && lb[1].dtype == KVM_F32 && kvm_vec_ok(lb[1]); }
+    if (ok && f32) {
+      // float32 rows: all loads of a thread in flight together
+      float v[J][8], u[J][8];
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int k = k0 + j * kstep;
+#pragma unroll
+        for (int i = 0; i < 8; i += 4) {
+          const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          const float4 t = k < K ? *(const float4*)((const float*)x.p + k + i) : zero, g = k < K && pro ? *(const float4*)(up + k + i) : zero;
+          v[j][i] = t.x; v[j][i + 1] = t.y; v[j][i + 2] = t.z; v[j][i + 3] = t.w;
+          u[j][i] = g.x; u[j][i + 1] = g.y; u[j][i + 2] = g.z; u[j][i + 3] = g.w;
         }
       }
-    } else if (pro == 1 && K <= 16 * KVM_NT) {
-      float xr[16], gr[16], q = 0.0f;
+      float rs = 1.0f;
+      if (pro == 1) {
+        float q = 0.0f;
 #pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int k = tid + u * KVM_NT;
-        xr[u] = k < K ? kvm_ld(x, k) : 0.0f;
-        gr[u] = k < K ? ((const float*)gm.p)[k] : 0.0f;
+        for (int j = 0; j < J; ++j)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) q += v[j][i] * v[j][i];
+        q = kvm_warp_sum(q);
+        float* red = (float*)c.smem;
+        if (lane == 0) red[warp] = q;
+        kvm_sync();
+        q = 0.0f;
+        for (int i = 0; i < KP; ++i) q += red[rg * KP + i];
+        rs = 1.0f / sqrtf(q / K + kvm_bits_f32(a[10]));
       }
 #pragma unroll
-      for (int u = 0; u < 16; ++u) q += xr[u] * xr[u];
-      q = kvm_block_sum(q, red);
-      const float rs = 1.0f / sqrtf(q / K + eps);
+      for (int j = 0; j < J; ++j) {
+        float t[8];
 #pragma unroll
-      for (int u = 0; u < 16; ++u) { const int k = tid + u * KVM_NT; if (k < K) vs[k] = __float2bfloat16_rn(xr[u] * rs * gr[u]); }
-    } else if (pro == 1) {
-      float q = 0.0f;
-      for (int k = tid; k < K; k += KVM_NT) { const float t = kvm_ld(x, k); q += t * t; }
-      q = kvm_block_sum(q, red);
-      const float rs = 1.0f / sqrtf(q / K + eps);
-      for (int k = tid; k < K; k += KVM_NT) vs[k] = __float2bfloat16_rn(kvm_ld(x, k) * rs * ((const float*)gm.p)[k]);
-    } else if (x.dtype == KVM_F32 && kvm_vec_ok(x) && (pro != 2 || (x2.dtype == KVM_F32 && kvm_vec_ok(x2)))) {
-      // three 16-byte loads per input and thread in flight per round (a 12288-wide SwiGLU row is two rounds)
-      for (int k0 = 0; k0 < K; k0 += 12 * KVM_NT) {
-        float4 p[3], q[3];
-#pragma unroll
-        for (int u = 0; u < 3; ++u) {
-          const int k = k0 + (tid + u * KVM_NT) * 4;
-          p[u] = k < K ? *(const float4*)((const float*)x.p + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          q[u] = (pro == 2 && k < K) ? *(const float4*)((const float*)x2.p + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-#pragma unroll
-        for (int u = 0; u < 3; ++u) {
-          const int k = k0 + (tid + u * KVM_NT) * 4;
-          if (k < K) {
-            const float4 v = pro == 2 ? make_float4(kvm_silu(p[u].x) * q[u].x, kvm_silu(p[u].y) * q[u].y, kvm_silu(p[u].z) * q[u].z, kvm_silu(p[u].w) * q[u].w) : p[u];
-            *(__nv_bfloat162*)(vs + k) = __floats2bfloat162_rn(v.x, v.y);
-            *(__nv_bfloat162*)(vs + k + 2) = __floats2bfloat162_rn(v.z, v.w);
-          }
-        }
+        for (int i = 0; i < 8; ++i) t[i] = kvm_bf16_round(pro == 1 ? v[j][i] * rs * u[j][i] : pro == 2 ? kvm_silu_fast(v[j][i]) * u[j][i] : v[j][i]);
+        put(j, t);
       }
     } else {
-      for (int k0 = 0; k0 < K; k0 += 8 * KVM_NT) {
-        float p[8], q[8];
+      // anything else is staged through shared memory (behind the partial sums)
+      __nv_bfloat16* vs = (__nv_bfloat16*)(c.smem + ((KVM_GV_RED + rows * KP * 4 + 15) & ~15));
+      if (ok) kvm_gemv_stage_x(lb, vs, (float*)c.smem, K, pro, kvm_bits_f32(a[10]));
+      kvm_sync();
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int k = k0 + tid + u * KVM_NT;
-          p[u] = k < K ? kvm_ld(x, k) : 0.0f;
-          q[u] = (pro == 2 && k < K) ? kvm_ld(x2, k) : 0.0f;
-        }
+      for (int j = 0; j < J; ++j) {
+        float t[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int k = k0 + tid + u * KVM_NT;
-          if (k < K) vs[k] = __float2bfloat16_rn(pro == 2 ? kvm_silu(p[u]) * q[u] : p[u]);
-        }
+        for (int i = 0; i < 8; ++i) t[i] = ok && k0 + j * kstep < K ? __bfloat162float(vs[k0 + j * kstep + i]) : 0.0f;
+        put(j, t);
       }
     }
   }
-  kvm_sync();
+  if (stamp && tid == 0) stamp[0] = (int)kvm_globaltimer();
   bool waited = true;
-  unsigned long long t_pro = 0, t_wait = 0, t_first = 0;
-  if (stamp && tid == 0) t_pro = kvm_globaltimer();
-  {
-    const int r = warp / KP, part = warp % KP;
-    const int plen = (((K + KP - 1) / KP) + 255) & ~255, kb = part * plen, ke = min(K, kb + plen);
-    for (int ci = 0; ci < NC; ++ci) {
-      const unsigned it = cit + ci;
-      unsigned long long tw = 0;
-      if (stamp && tid == 0) tw = kvm_globaltimer();
-      if (waited && !kvm_ring_wait_warp(ring, it, deadline, c.err)) waited = false;
-      if (stamp && tid == 0) { const unsigned long long d = kvm_globaltimer() - tw; t_wait += d; if (ci == 0) t_first = d; }
-      if (!waited) break;                                  // warp-uniform
-      if (ok && r < R && ci * R + r < rows) {
-        const unsigned char* st = kvm_ring_stage(ring, it) + (size_t)r * K * 2;
-        float acc0 = 0.0f, acc1 = 0.0f, acc2 = 0.0f, acc3 = 0.0f;
-        int k = kb + lane * 8;
-        for (; k + 256 < ke; k += 512) {                   // two 16-byte pieces of the row and of the activations in flight per trip
-          const uint4 wa = *(const uint4*)(st + k * 2), wb = *(const uint4*)(st + (k + 256) * 2);
-          const uint4 xa = *(const uint4*)(vs + k), xb = *(const uint4*)(vs + k + 256);
-          acc0 = fmaf(kvm_bf16lo(xa.x), kvm_bf16lo(wa.x), acc0); acc1 = fmaf(kvm_bf16hi(xa.x), kvm_bf16hi(wa.x), acc1);
-          acc2 = fmaf(kvm_bf16lo(xb.x), kvm_bf16lo(wb.x), acc2); acc3 = fmaf(kvm_bf16hi(xb.x), kvm_bf16hi(wb.x), acc3);
-          acc0 = fmaf(kvm_bf16lo(xa.y), kvm_bf16lo(wa.y), acc0); acc1 = fmaf(kvm_bf16hi(xa.y), kvm_bf16hi(wa.y), acc1);
-          acc2 = fmaf(kvm_bf16lo(xb.y), kvm_bf16lo(wb.y), acc2); acc3 = fmaf(kvm_bf16hi(xb.y), kvm_bf16hi(wb.y), acc3);
-          acc0 = fmaf(kvm_bf16lo(xa.z), kvm_bf16lo(wa.z), acc0); acc1 = fmaf(kvm_bf16hi(xa.z), kvm_bf16hi(wa.z), acc1);
-          acc2 = fmaf(kvm_bf16lo(xb.z), kvm_bf16lo(wb.z), acc2); acc3 = fmaf(kvm_bf16hi(xb.z), kvm_bf16hi(wb.z), acc3);
-          acc0 = fmaf(kvm_bf16lo(xa.w), kvm_bf16lo(wa.w), acc0); acc1 = fmaf(kvm_bf16hi(xa.w), kvm_bf16hi(wa.w), acc1);
-          acc2 = fmaf(kvm_bf16lo(xb.w), kvm_bf16lo(wb.w), acc2); acc3 = fmaf(kvm_bf16hi(xb.w), kvm_bf16hi(wb.w), acc3);
+  constexpr int RB = J <= 1 ? 4 : 1;          // rows whose loads are in flight together
+#pragma unroll 1
+  for (int ci = 0; ci < NC; ++ci) {
+    if (!kvm_ring_wait_warp(ring, cit + ci, c.deadline, c.err)) { waited = false; break; }      // warp-uniform
+    const unsigned char* st = kvm_ring_stage(ring, cit + ci) + (size_t)(rg * m) * (K * 2);
+    const int left = min(m, rows - ci * R - rg * m);
+    float s[8];
+#pragma unroll
+    for (int h = 0; h < 8; h += RB) {
+#pragma unroll
+      for (int r = 0; r < RB; ++r) s[h + r] = 0.0f;
+      if (h < left) {
+        uint4 w[RB][J];
+#pragma unroll
+        for (int r = 0; r < RB; ++r)
+#pragma unroll
+          for (int j = 0; j < J; ++j) w[r][j] = h + r < left && k0 + j * kstep < K ? *(const uint4*)(st + ((h + r) * K + k0 + j * kstep) * 2) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int r = 0; r < RB; ++r) {
+          unsigned long long acc = 0ull;
+#pragma unroll
+          for (int j = 0; j < J; ++j) {
+            if (PACK) {
+              const uint32_t p[4] = {xp[PACK ? j : 0].x, xp[PACK ? j : 0].y, xp[PACK ? j : 0].z, xp[PACK ? j : 0].w};
+              unsigned long long xx[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) xx[i] = kvm_pack2(__uint_as_float(p[i] << 16), __uint_as_float(p[i] & 0xffff0000u));
+              kvm_gv_dot8(acc, w[r][j], xx);
+            } else kvm_gv_dot8(acc, w[r][j], xs[PACK ? 0 : j]);
+          }
+          const float2 f = *(float2*)&acc;
+          s[h + r] = f.x + f.y;
         }
-        for (; k < ke; k += 256) {
-          const uint4 wv = *(const uint4*)(st + k * 2);
-          const uint4 xv = *(const uint4*)(vs + k);
-          acc0 = fmaf(kvm_bf16lo(xv.x), kvm_bf16lo(wv.x), acc0); acc1 = fmaf(kvm_bf16hi(xv.x), kvm_bf16hi(wv.x), acc1);
-          acc0 = fmaf(kvm_bf16lo(xv.y), kvm_bf16lo(wv.y), acc0); acc1 = fmaf(kvm_bf16hi(xv.y), kvm_bf16hi(wv.y), acc1);
-          acc0 = fmaf(kvm_bf16lo(xv.z), kvm_bf16lo(wv.z), acc0); acc1 = fmaf(kvm_bf16hi(xv.z), kvm_bf16hi(wv.z), acc1);
-          acc0 = fmaf(kvm_bf16lo(xv.w), kvm_bf16lo(wv.w), acc0); acc1 = fmaf(kvm_bf16hi(xv.w), kvm_bf16hi(wv.w), acc1);
-        }
-        const float sum = kvm_warp_sum((acc0 + acc1) + (acc2 + acc3));
-        if (lane == 0) parts[(ci * R + r) * KP + part] = sum;
       }
-      __syncwarp();
-      if (lane == 0) kvm_mbar_arrive(kvm_ring_empty(ring, it));
     }
-  }
-  __syncwarp();
-  if (stamp && tid == 0) {      // trace detail, one byte each in units of 0.2 us: prologue | stage loop (waits included) | waits for stages
-    (void)t_first;
-    stamp[0] = (int)min(255ull, (t_pro - t_task) / 200) | ((int)min(255ull, (kvm_globaltimer() - t_pro) / 200) << 8) | ((int)min(255ull, t_wait / 200) << 16);
+    const float t = kvm_gv_reduce8(s, lane);
+    __syncwarp();                                          // (the shuffles have met already; this orders the lanes' reads before the release)
+    if (lane == 0) kvm_mbar_arrive(kvm_ring_empty(ring, cit + ci));
+    if ((lane & 3) == 0 && (lane >> 2) < left) parts[part * rows + ci * R + rg * m + (lane >> 2)] = t;
   }
   if (!waited && *(volatile int*)&c.err->code == 0) kvm_stream_timeout(c, 1134);
+  if (stamp && tid == 0) stamp[1] = (int)kvm_globaltimer();
   kvm_sync();
-  if (ok && *(volatile int*)&c.err->code == 0)
+  if (ok && waited) {
+    const KvmBuf out = lb[4];
     for (int i = tid; i < rows; i += KVM_NT) {
       float sum = 0.0f;
-      for (int p = 0; p < KP; ++p) sum += parts[i * KP + p];
-      kvm_st(out, n0 + i, res.p ? __fadd_rn(sum, kvm_ld(res, n0 + i)) : sum);
+      for (int p = 0; p < KP; ++p) sum += parts[p * rows + i];
+      if (a[5] >= 0) sum = __fadd_rn(sum, i == tid ? rv : kvm_ld(lb[5], a[6] + i));
+      kvm_st(out, a[6] + i, sum);
     }
+  }
 }
+// rows of up to 32 Ki columns (what a stage holds) whose activations do not fit the registers beside the loop's: a function of its own
+KVM_OP_FN void kvm_gemv_ring_wide(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing ring, unsigned cit, int R, int NC) { kvm_gemv_ring<8>(c, a, lb, ring, cit, R, NC, nullptr); }
 
 // ---- streamed GEMV on tensor cores (gemv_bf16 with one activation row, gemv_bf16_rows with up to eight), consumer side --------------
 // D[16 x 8] += A[16 x 16] B[16 x 8] (mma.sync m16n8k16, bf16 operands, float32 accumulate) with A = activations (rows = activation
@@ -311,13 +363,6 @@ __device__ __forceinline__ void kvm_mma_bf16_16816(float (&d)[4], uint32_t a0, u
 __device__ __forceinline__ void kvm_mma_pro8(int pro, float (&v)[8], const float (&v2)[8], float rs) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) v[j] = pro == 1 ? v[j] * rs * v2[j] : pro == 2 ? kvm_silu(v[j]) * v2[j] : v[j];
-}
-__device__ __forceinline__ uint4 kvm_pack_bf16x8(const float (&v)[8]) {
-  uint4 pk;
-  __nv_bfloat162* hh = (__nv_bfloat162*)&pk;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) hh[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-  return pk;
 }
 // Staging of the activations v = bf16(pro(x)) for the tensor-core consumer, functions of their own (registers of their own).
 struct KvmStageX {
@@ -393,7 +438,7 @@ KVM_OP_FN void kvm_stage_rows(const KvmStageX& s, int kb, int kn) {
   }
 }
 template <bool CHUNKED>      // the k-chunk layout (accumulators of eight row groups live over the task) or the whole-row layout, a function each
-KVM_OP_FN void kvm_gemv_mma_ring_t(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool has_rows, const KvmRing& ring, unsigned cit, unsigned long long deadline,
+KVM_OP_FN void kvm_gemv_mma_ring_t(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool has_rows, const KvmRing ring, unsigned cit, unsigned long long deadline,
                                    unsigned long long t_task, int* stamp) {
   KvmBuf x, x2, gm, w, out, res;
   const int n0 = a[6], n1 = a[7], K = a[8], pro = a[9], r0 = has_rows ? a[11] : 0, r1 = has_rows ? a[12] : 1;
@@ -498,7 +543,7 @@ KVM_OP_FN void kvm_gemv_mma_ring_t(const KvmCtx& c, const int32_t* a, const KvmB
     }
 }
 
-__device__ __forceinline__ void kvm_gemv_mma_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool has_rows, const KvmRing& ring, unsigned cit, int nkc,
+__device__ __forceinline__ void kvm_gemv_mma_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool has_rows, const KvmRing ring, unsigned cit, int nkc,
                                                   unsigned long long deadline, unsigned long long t_task, int* stamp) {
   if (nkc > 1) kvm_gemv_mma_ring_t<true>(c, a, lb, has_rows, ring, cit, deadline, t_task, stamp);
   else kvm_gemv_mma_ring_t<false>(c, a, lb, has_rows, ring, cit, deadline, t_task, stamp);
@@ -507,7 +552,7 @@ __device__ __forceinline__ void kvm_gemv_mma_ring(const KvmCtx& c, const int32_t
 // ---- streamed split attention, consumer side ----------------------------------------------------------------------------------
 // Stage use `cit` holds the split's keys, `cit + 1` its values (the appended row left out).  Semantics as kvm_op_attn_decode_part
 // (runtime/ref_extra.py:421-498); the front warp has validated the geometry before it issued the copies.
-KVM_OP_FN void kvm_attn_part_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool qkn, const KvmRing& ring, unsigned cit, int j0, int j1, int newrow,
+KVM_OP_FN void kvm_attn_part_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool qkn, const KvmRing ring, unsigned cit, int j0, int j1, int newrow,
                                           unsigned long long deadline, unsigned long long t_task, int* stamp) {
   KvmBuf q, kc, vc, lens, part, kn, vn, gam{};
   bool ok = kvm_buf_local(c, lb, a, 0, KVM_M_FLT, q) && kvm_buf_local(c, lb, a, 1, KVM_M_FLT, kc) && kvm_buf_local(c, lb, a, 2, KVM_M_FLT, vc) &&
@@ -582,16 +627,16 @@ static __device__ void kvm_static_geometry(const KvmDevState& S, KvmStSlot& sl, 
   const int32_t* a = sl.args;
   if (op == 134 || op == 301) {
     const int wi = a[3], n0 = a[6], n1 = a[7], K = a[8], r0 = op == 301 ? a[11] : 0, r1 = op == 301 ? a[12] : 1;
-    if (wi < 0 || wi >= S.nbufs || n0 < 0 || n1 <= n0 || K <= 0 || (K & 255) || r0 < 0 || r1 <= r0 || r1 - r0 > 8) return;
+    if (wi < 0 || wi >= S.nbufs || n0 < 0 || n1 <= n0 || K <= 0 || (K & 7) || r0 < 0 || r1 <= r0 || r1 - r0 > 8) return;
     const KvmBuf w = sl.lb[3];
     if (!w.p || w.dtype != KVM_BF16 || (w.ld & 7) || ((uintptr_t)w.p & 15) || n1 > w.rows || K > w.cols) return;
     // one activation row: the SIMT consumer over stages of whole rows (measured faster than mma.sync fragments at one row: the
     // legacy tensor path of this part issues an m16n8k16 every few hundred cycles per warp); several rows: the tensor-core consumer
     if (op == 134 && K * 2 <= KVM_ST_STAGE) {
-      int R = KVM_ST_STAGE / (K * 2);
-      if (R > KVM_ST_ARRIVALS) R = KVM_ST_ARRIVALS;
-      if (((K * 2 + 127) & ~127) + 256 + ((n1 - n0 + 7) & ~7) * (KVM_ST_ARRIVALS / R) * 4 <= scratch_bytes) { sl.kind = 1; sl.R = R; sl.nchunks = (n1 - n0 + R - 1) / R; return; }
+      const int RG = KVM_NWARPS / kvm_gv_parts(K), R = min(kvm_gv_rows(K), (n1 - n0 + RG - 1) / RG * RG);
+      if (KVM_GV_RED + (n1 - n0) * kvm_gv_parts(K) * 4 + 16 + K * 2 <= scratch_bytes) { sl.kind = 1; sl.R = R; sl.nchunks = (n1 - n0 + R - 1) / R; return; }
     }
+    if (K & 255) return;
     const KvmMmaLayout L = kvm_gemv_mma_layout(n1 - n0, K, r1 - r0, scratch_bytes);
     if (L.ok) { sl.kind = 3; sl.R = L.R; sl.j0 = L.KC; sl.j1 = L.ng; sl.newrow = L.nkc; sl.nchunks = L.nchunks; }      // j0 / j1 / newrow double as KC / row groups / k-chunks
   } else if (op == 135 || op == 300) {
@@ -644,20 +689,19 @@ static __device__ void kvm_static_issue(const KvmDevState& S, const KvmStSlot& s
   }
 }
 
-__global__ void __launch_bounds__(KVM_NT + 32, 1) kvm_static_kernel(KvmStaticState T) {
+__global__ void __launch_bounds__(KVM_ST_THREADS, 1) kvm_static_kernel(KvmStaticState T) {
   extern __shared__ __align__(1024) unsigned char kvm_smem[];
   const KvmDevState& S = T.D;
   KvmStSlot* slots = (KvmStSlot*)kvm_smem;
   int* ctl = (int*)(kvm_smem + KVM_ST_SLOTS * sizeof(KvmStSlot));          // as in the dynamic kernel: ctl[0] = TMEM base, tensor-core barriers from ctl[8]
-  int* sctl = ctl + 96;                                                     // static path's own words: [0] consumer stage-use count, [1] tasks finished
+  int* sctl = ctl + 96;                                                     // static path's own words: [0] consumer stage-use count, [1] tasks finished, [2] producer stage-use count, [3..5] trace, [6] leave
   const uint32_t sbar = kvm_smem_addr(kvm_smem + KVM_ST_HDR - 128);         // stream ring barriers: full[3] | empty[3]
   const int tid = threadIdx.x;
-  const bool is_front = tid >= KVM_NT;
   const int w = blockIdx.x;
   unsigned dyn;
   asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
-  if (tid < KVM_ST_SLOTS) { slots[tid].state = 0; slots[tid].task = -1; }
-  if (tid == 0) { sctl[0] = 0; sctl[1] = 0; ((int*)(kvm_smem + KVM_ST_HDR - 128 - 288))[0] = 0; ((int*)(kvm_smem + KVM_ST_HDR - 128 - 288))[1] = 0; }
+  if (tid < KVM_ST_SLOTS) { slots[tid].state = 0; slots[tid].task = -1; slots[tid].pos = -1; }
+  if (tid == 0) { sctl[0] = 0; sctl[1] = 0; sctl[6] = 0; ((int*)(kvm_smem + KVM_ST_HDR - 128 - 288))[0] = 0; ((int*)(kvm_smem + KVM_ST_HDR - 128 - 288))[1] = 0; }
   kvm_tc_init(ctl, kvm_smem);
   const unsigned ring_ns = T.ring == 2 ? 2u : 3u;
   const int ring_bytes = (int)ring_ns * KVM_ST_STAGE;
@@ -672,7 +716,7 @@ __global__ void __launch_bounds__(KVM_NT + 32, 1) kvm_static_kernel(KvmStaticSta
   if (buf_cache) {
     const uint4* src = (const uint4*)S.bufs;
     uint4* dst = (uint4*)(kvm_smem + KVM_ST_HDR);
-    for (int i = tid; i < S.nbufs * 2; i += KVM_NT + 32) dst[i] = src[i];
+    for (int i = tid; i < S.nbufs * 2; i += KVM_ST_THREADS) dst[i] = src[i];
   }
   __syncthreads();
   const unsigned long long t_begin = kvm_globaltimer();
@@ -684,41 +728,61 @@ __global__ void __launch_bounds__(KVM_NT + 32, 1) kvm_static_kernel(KvmStaticSta
   ring.base_addr = kvm_smem_addr(ring.base);
   const int p_lo = T.prog_off[w], n = T.prog_off[w + 1] - p_lo;
 
-  if (is_front) {
+  if (tid >= KVM_NT + 32) {
+    // ---- stream warp: issues the copies of the fetched tasks in list order, as soon as there are free stages.  It does nothing else:
+    // behind the dependency polls (an L2 round trip each, several microseconds when the copies saturate the memory system) a freed
+    // stage waited for its next copy, and the weights arrived at half the HBM rate.
+    if ((tid & 31) == 0) {
+      unsigned pit = 0, idle = 0;                // stage uses issued
+      bool leave = false;
+      // an error may leave stages unconsumed, and the front warp may have finished its list by then: watched here too
+      auto quit = [&]() { return (++idle & 1023u) == 0 && (kvm_ld_volatile_shared(&sctl[6]) || *(volatile int*)&S.err->code != 0 || kvm_globaltimer() > deadline); };
+      for (int ii = 0; ii < n && !leave; ++ii) {
+        KvmStSlot& sl = slots[ii % KVM_ST_SLOTS];
+        // The record may have come and gone if the task does not stream (its slot is refilled once it has finished); one that streams
+        // stays until its copies are issued here, so a kind read between two looks at the same position belongs to it.
+        int kind = 0;
+        while (true) {
+          const int seen = kvm_ld_volatile_shared(&sl.pos);
+          if (seen == ii) {
+            kind = kvm_ld_volatile_shared(&sl.kind);
+            if (kvm_ld_volatile_shared(&sl.pos) != ii) kind = 0;
+            break;
+          }
+          if (seen > ii) break;
+          if (quit()) { leave = true; break; }
+        }
+        if (leave || kind == 0) continue;
+        __threadfence_block();
+        const bool pre = sl.prefetch & 1;
+        // constants may run ahead; anything else waits until the task is ready
+        while (!pre && kvm_ld_volatile_shared(&sl.state) < 2) if (quit()) { leave = true; break; }
+        if (!pre) asm volatile("fence.proxy.async;" ::: "memory");      // data other workers wrote with plain stores, read here by bulk copies
+        const int nch = sl.nchunks;
+        for (int ci = 0; ci < nch && !leave; ++ci) {
+          while (pit >= ring.ns && !kvm_mbar_test(kvm_ring_empty(ring, pit), kvm_ring_parity(ring, pit) ^ 1u))
+            if (quit()) { leave = true; break; }
+          if (leave) break;
+          kvm_static_issue(S, sl, ring, pit, ci);
+          ++pit;
+        }
+      }
+      sctl[2] = (int)pit;
+    }
+  } else if (tid >= KVM_NT) {
+    // ---- front warp: fetches the records of the next tasks and finds them ready
     const int lane = tid & 31;
-    int fi = 0, ri = 0, ii = 0, ic = 0;        // next position to fetch / to mark ready / to stream; chunk inside the streamed task
-    unsigned pit = 0;                          // stage uses issued
+    int fi = 0, ri = 0;                        // next position to fetch / to mark ready
     int dep[5] = {-1, -1, -1, -1, -1}, dep_pos = -1;     // dependency entries of the task at `ri`
     bool stop = false;
     unsigned idle = 0;
-    // one pass of the copy issuer: lane 0 issues chunks of the oldest tasks that still have copies to issue while stages are free
-    auto stream_pass = [&]() -> bool {
-      if (ii >= fi) return false;
-      int lii = ii, lic = ic;
-      unsigned lpit = pit;
-      if (lane == 0) {
-        for (int guard = 0; guard < 6 && lii < fi; ++guard) {
-          KvmStSlot& sl = slots[lii % KVM_ST_SLOTS];
-          if (sl.kind == 0) { ++lii; lic = 0; continue; }
-          if (!(sl.prefetch || lii < ri)) break;             // constants may run ahead; anything else waits until the task is ready
-          if (!(lpit < ring.ns || kvm_mbar_test(kvm_ring_empty(ring, lpit), kvm_ring_parity(ring, lpit) ^ 1u))) break;
-          if (!sl.prefetch) asm volatile("fence.proxy.async;" ::: "memory");      // data other workers wrote with plain stores, read here by bulk copies
-          kvm_static_issue(S, sl, ring, lpit, lic);
-          ++lpit; ++lic;
-          if (lic >= sl.nchunks) { ++lii; lic = 0; }
-        }
-      }
-      lii = __shfl_sync(0xffffffffu, lii, 0); lic = __shfl_sync(0xffffffffu, lic, 0); lpit = __shfl_sync(0xffffffffu, lpit, 0);
-      const bool moved = lii != ii || lic != ic;
-      ii = lii; ic = lic; pit = lpit;
-      return moved;
-    };
-    while (!stop && (ri < n || ii < n)) {
+    while (!stop && ri < n) {
       bool progressed = false;
       // 1. fetch the next record into a free slot
-      if (fi < n && kvm_ld_volatile_shared(&slots[fi % KVM_ST_SLOTS].state) == 0) {
+      if (fi < n && __shfl_sync(0xffffffffu, lane == 0 ? kvm_ld_volatile_shared(&slots[fi % KVM_ST_SLOTS].state) : 0, 0) == 0) {      // the warp decides as one
         KvmStSlot& sl = slots[fi % KVM_ST_SLOTS];
         const int task = T.prog[p_lo + fi];
+        if (lane == 0) { *(volatile int*)&sl.pos = -1; __threadfence_block(); }      // see the stream warp
         const int32_t* rec = S.recs + (size_t)task * KVM_REC_WORDS;
         const int32_t w0 = rec[lane], w1 = lane < 16 ? rec[32 + lane] : 0;
         if (lane < 16) sl.desc[lane] = w0; else sl.args[lane - 16] = w0;
@@ -740,14 +804,14 @@ __global__ void __launch_bounds__(KVM_NT + 32, 1) kvm_static_kernel(KvmStaticSta
         }
         if (lane == 0) {
           if (use_ring) kvm_static_geometry(S, sl, (int)dyn - KVM_ST_HDR - ring_bytes); else { sl.kind = 0; sl.nchunks = 0; }
-          sl.state = 1;
+          __threadfence_block();
+          *(volatile int*)&sl.state = 1;
+          *(volatile int*)&sl.pos = fi;
         }
         __syncwarp();
         ++fi; progressed = true;
       }
-      // 2. stream ahead: chunks of the oldest tasks that still have copies to issue, as many as there are free stages
-      if (stream_pass()) progressed = true;
-      // 3. dependencies of the next task to become ready: its entries are held in registers (up to five per lane) and polled with
+      // 2. dependencies of the next task to become ready: its entries are held in registers (up to five per lane) and polled with
       //    plain loads, all in flight together; one acquire fence once they are all met
       if (ri < fi) {
         KvmStSlot& sl = slots[ri % KVM_ST_SLOTS];
@@ -760,10 +824,6 @@ __global__ void __launch_bounds__(KVM_NT + 32, 1) kvm_static_kernel(KvmStaticSta
         int seen[5];
 #pragma unroll
         for (int j = 0; j < 5; ++j) seen[j] = dep[j] >= 0 ? kvm_ld_relaxed(&T.progress[dep[j] >> KVM_ST_WAIT_BITS]) : 0;
-        // while those loads are in flight (an L2 round trip, longer when the memory system is saturated by the copies) keep
-        // refilling stages: a freed stage must not wait for the poll
-        if (ii < fi)
-          for (int sp = 0; sp < 6; ++sp) if (stream_pass()) progressed = true;
         bool met = true;
 #pragma unroll
         for (int j = 0; j < 5; ++j) if (dep[j] >= 0 && seen[j] < (dep[j] & ((1 << KVM_ST_WAIT_BITS) - 1))) met = false;
@@ -774,7 +834,7 @@ __global__ void __launch_bounds__(KVM_NT + 32, 1) kvm_static_kernel(KvmStaticSta
           ++ri; progressed = true;
         }
       }
-      // 4. failure / stall
+      // 3. failure / stall
       if (!progressed) {
         if ((++idle & 63u) == 0) {
           int e = 0;
@@ -791,13 +851,13 @@ __global__ void __launch_bounds__(KVM_NT + 32, 1) kvm_static_kernel(KvmStaticSta
     // leave: the compute group takes slots in order; the first one that is not ready tells it to go
     if (stop) {
       if (lane == 0) {
+        sctl[6] = 1;
         for (int k = 0; k < KVM_ST_SLOTS; ++k) {
           KvmStSlot& sl = slots[(ri + k) % KVM_ST_SLOTS];
           if (kvm_ld_volatile_shared(&sl.state) != 2) { sl.state = 3; break; }
         }
       }
     }
-    sctl[2] = (int)pit;
   } else {
     KvmCtx& c = *(KvmCtx*)(kvm_smem + KVM_ST_HDR - 128 - 288 - KVM_ST_CTX_BYTES);      // in shared memory (see kvm_sched.cuh)
     if (tid == 0) {
@@ -828,9 +888,14 @@ __global__ void __launch_bounds__(KVM_NT + 32, 1) kvm_static_kernel(KvmStaticSta
       if (go == 0) break;
       const int task = sl.task;
       unsigned long long t_task = 0;
-      if (tid == 0 && S.trace) { t_task = kvm_globaltimer(); S.t_start[task] = t_task; sctl[3] = 0; }
+      if (tid == 0 && S.trace) { t_task = kvm_globaltimer(); S.t_start[task] = t_task; sctl[3] = sctl[4] = 0; sctl[5] = (int)t_task; }
       const int op = sl.desc[0], kind = sl.kind, nch = sl.nchunks;
-      if (kind == 1) kvm_gemv_ring(c, sl.args, sl.lb, ring, cit, sl.R, nch, deadline, t_task, S.trace ? sctl + 3 : nullptr);
+      if (kind == 1) {
+        const int J = (sl.args[8] + 256 * kvm_gv_parts(sl.args[8]) - 1) / (256 * kvm_gv_parts(sl.args[8]));      // pieces of eight columns per thread
+        if (J == 1) kvm_gemv_ring<1>(c, sl.args, sl.lb, ring, cit, sl.R, nch, S.trace ? sctl + 3 : nullptr);
+        else if (J <= 3) kvm_gemv_ring<3>(c, sl.args, sl.lb, ring, cit, sl.R, nch, S.trace ? sctl + 3 : nullptr);
+        else kvm_gemv_ring_wide(c, sl.args, sl.lb, ring, cit, sl.R, nch);
+      }
       else if (kind == 3) kvm_gemv_mma_ring(c, sl.args, sl.lb, op == 301, ring, cit, sl.newrow, deadline, t_task, S.trace ? sctl + 3 : nullptr);
       else if (kind == 2) kvm_attn_part_ring(c, sl.args, sl.lb, op == 300, ring, cit, sl.j0, sl.j1, sl.newrow, deadline, t_task, S.trace ? sctl + 3 : nullptr);
       else if (op != 0 && go == 1) kvm_dispatch(c, op, sl.args, sl.aux);
@@ -841,7 +906,10 @@ __global__ void __launch_bounds__(KVM_NT + 32, 1) kvm_static_kernel(KvmStaticSta
       if (kind != 1 && kind != 3) asm volatile("fence.proxy.async;" ::: "memory");
       kvm_sync();
       if (tid == 0) {
-        if (S.trace) { S.t_end[task] = kvm_globaltimer(); S.t_smid[task] = (int)kvm_smid() | (sctl[3] << 8); }     // bits 8.. : detail of a streamed task
+        if (S.trace) {                                       // bits 8.. : detail of a streamed task (a GEMV: prologue | stage loop, a byte each in units of 0.2 us)
+          const int detail = kind == 1 ? min(255, (sctl[3] - sctl[5]) / 200) | min(255, (sctl[4] - sctl[3]) / 200) << 8 : sctl[3];
+          S.t_end[task] = kvm_globaltimer(); S.t_smid[task] = (int)kvm_smid() | (detail << 8);
+        }
         atomicAdd(&S.exec_count[task], 1);                   // no result needed: nothing waits for the old value
         const int pv = sl.desc[10];
         if (pv >= 0) {                                       // publish (include/mvm_task_abi.h:20-23): old + 1, else VERSION_GAP
@@ -862,7 +930,7 @@ __global__ void __launch_bounds__(KVM_NT + 32, 1) kvm_static_kernel(KvmStaticSta
   }
   __syncthreads();
   // copies issued but never consumed (an early exit): wait for them, bounded, before the shared memory goes away
-  if (use_ring && tid == KVM_NT) {
+  if (use_ring && tid == KVM_NT + 32) {
     const unsigned pit = (unsigned)sctl[2], cit = (unsigned)sctl[0];
     for (unsigned it = cit; it < pit; ++it) {
       const uint32_t bar = kvm_ring_full(ring, it), par = kvm_ring_parity(ring, it);

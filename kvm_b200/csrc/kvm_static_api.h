@@ -6,6 +6,7 @@
 #include "kvm_state.cuh"
 
 #define KVM_ST_STAGE 65536             // bytes of one stream stage
+#define KVM_ST_THREADS (KVM_NT + 64)   // 16 compute warps, the front warp, the stream warp
 #define KVM_ST_WAIT_BITS 20            // dependency entry: worker << 20 | tasks that worker must have finished
 
 struct KvmStaticState {
