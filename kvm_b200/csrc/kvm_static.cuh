@@ -78,18 +78,16 @@ __device__ __forceinline__ int kvm_ld_relaxed(const int* p) {
   return v;
 }
 
-// Wait for stage use `it` to land: lane 0 polls (bounded by the launch deadline and by an error recorded elsewhere), the verdict
-// is the same for the whole warp.  All 32 lanes must call it.
+// Wait for stage use `it` to land (bounded by the launch deadline and by an error recorded elsewhere); the verdict is the same for the
+// whole warp.  All 32 lanes poll: with one lane polling and a shuffle behind it the compiler kept that lane's path apart from the
+// others' through the arithmetic that follows, and the warp went through it twice (a GEMV phase took 57 us instead of 36).
 __device__ __forceinline__ bool kvm_ring_wait_warp(const KvmRing& ring, unsigned it, unsigned long long deadline, const KvmErrRec* err) {
-  int ok = 1;
-  if ((threadIdx.x & 31) == 0) {
-    const uint32_t bar = kvm_ring_full(ring, it), par = kvm_ring_parity(ring, it);
-    unsigned spins = 0;
-    while (!kvm_mbar_test(bar, par)) {
-      if ((++spins & 1023u) == 0 && (kvm_globaltimer() > deadline || *(volatile const int*)&err->code != 0)) { ok = 0; break; }      // an error elsewhere: the copies may never come
-    }
-  }
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+  const uint32_t bar = kvm_ring_full(ring, it), par = kvm_ring_parity(ring, it);
+  bool ok = true;
+  unsigned spins = 0;
+  while (!kvm_mbar_test(bar, par))
+    if ((++spins & 1023u) == 0 && (kvm_globaltimer() > deadline || *(volatile const int*)&err->code != 0)) { ok = false; break; }      // an error elsewhere: the copies may never come
+  return __all_sync(0xffffffffu, ok);
 }
 
 // ---- streamed GEMV, consumer side --------------------------------------------------------------------------------------------
@@ -303,6 +301,7 @@ __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a,
     }
   }
 }
+KVM_OP_FN void kvm_gemv_ring_3(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing ring, unsigned cit, int R, int NC, int* stamp) { kvm_gemv_ring<3>(c, a, lb, ring, cit, R, NC, stamp); }
 // rows of up to 32 Ki columns (what a stage holds) whose activations do not fit the registers beside the loop's: a function of its own
 KVM_OP_FN void kvm_gemv_ring_wide(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing ring, unsigned cit, int R, int NC) { kvm_gemv_ring<8>(c, a, lb, ring, cit, R, NC, nullptr); }
 
@@ -893,7 +892,7 @@ __global__ void __launch_bounds__(KVM_ST_THREADS, 1) kvm_static_kernel(KvmStatic
       if (kind == 1) {
         const int J = (sl.args[8] + 256 * kvm_gv_parts(sl.args[8]) - 1) / (256 * kvm_gv_parts(sl.args[8]));      // pieces of eight columns per thread
         if (J == 1) kvm_gemv_ring<1>(c, sl.args, sl.lb, ring, cit, sl.R, nch, S.trace ? sctl + 3 : nullptr);
-        else if (J <= 3) kvm_gemv_ring<3>(c, sl.args, sl.lb, ring, cit, sl.R, nch, S.trace ? sctl + 3 : nullptr);
+        else if (J <= 3) kvm_gemv_ring_3(c, sl.args, sl.lb, ring, cit, sl.R, nch, S.trace ? sctl + 3 : nullptr);
         else kvm_gemv_ring_wide(c, sl.args, sl.lb, ring, cit, sl.R, nch);
       }
       else if (kind == 3) kvm_gemv_mma_ring(c, sl.args, sl.lb, op == 301, ring, cit, sl.newrow, deadline, t_task, S.trace ? sctl + 3 : nullptr);
