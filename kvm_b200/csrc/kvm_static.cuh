@@ -18,6 +18,7 @@
 #pragma once
 #include "kvm_attn_tc.cuh"
 #include "kvm_dispatch.cuh"
+#include "kvm_ring_attn.cuh"
 #include "kvm_ops_decode.cuh"
 #include "kvm_static_api.h"
 
@@ -548,73 +549,58 @@ __device__ __forceinline__ void kvm_gemv_mma_ring(const KvmCtx& c, const int32_t
   else kvm_gemv_mma_ring_t<false>(c, a, lb, has_rows, ring, cit, deadline, t_task, stamp);
 }
 
-// ---- streamed split attention, consumer side ----------------------------------------------------------------------------------
-// Stage use `cit` holds the split's keys, `cit + 1` its values (the appended row left out).  Semantics as kvm_op_attn_decode_part
-// (runtime/ref_extra.py:421-498); the front warp has validated the geometry before it issued the copies.
-KVM_OP_FN void kvm_attn_part_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool qkn, const KvmRing ring, unsigned cit, int j0, int j1, int newrow,
-                                          unsigned long long deadline, unsigned long long t_task, int* stamp) {
-  KvmBuf q, kc, vc, lens, part, kn, vn, gam{};
-  bool ok = kvm_buf_local(c, lb, a, 0, KVM_M_FLT, q) && kvm_buf_local(c, lb, a, 1, KVM_M_FLT, kc) && kvm_buf_local(c, lb, a, 2, KVM_M_FLT, vc) &&
-            kvm_buf_local(c, lb, a, 3, KVM_M_I32, lens) && kvm_buf_local(c, lb, a, 4, KVM_M_F32, part) && kvm_buf_local(c, lb, a, 5, KVM_M_FLT, kn, true) &&
-            kvm_buf_local(c, lb, a, 6, KVM_M_FLT, vn, true);
-  if (ok && qkn) ok = kvm_buf(c, a[18], KVM_M_F32, gam);
-  const int b = a[7], kvh = a[8], s = a[9], S = a[10], H = a[11], Hkv = a[12], hd = a[13], Tmax = a[14], fl = a[17];
-  const float sc = kvm_bits_f32(a[15]), theta = kvm_bits_f32(a[16]);
-  const int G = H / Hkv;
-  if (ok) ok = kvm_mat_ok(c, q, b + 1, H * hd) && kvm_mat_ok(c, part, (long long)(b + 1) * S * H, hd + 2) && kvm_mat_ok(c, kn, b + 1, Hkv * hd) && kvm_mat_ok(c, vn, b + 1, Hkv * hd) &&
-            kvm_mat_ok(c, gam, 2, hd);
-  if (ok && ((fl & 1) && (!kn.p || !vn.p))) { c.fail(KVM_OPE_SHAPE, hd, fl); ok = false; }
-  const int p0 = ok ? ((const int*)lens.p)[b] : 0, nk = max(j1 - j0, 0);
-  unsigned char* sm = c.smem;
+// ---- streamed split attention, consumer side (kvm_ring_attn.cuh) --------------------------------------------------------------------
+// Stage use `cit` holds the split's keys, `cit + 1` its values (the appended row left out).  The front warp has validated the geometry
+// of the caches before it issued the copies; the other arguments are checked here.
+template <int HD, int GT>      // head dimension, query heads per key head at most
+KVM_OP_FN void kvm_attn_part_ring_t(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool qkn, const KvmRing ring, unsigned cit, int j0, int j1, int newrow) {
+  KvmPartArgs P;
+  const int bb = a[7], S = a[10], H = a[11], Hkv = a[12], hd = a[13];
+  bool ok;
+  {
+    KvmBuf q, kc, vc, lens, part, kn, vn, gam;
+    ok = kvm_buf_local(c, lb, a, 0, KVM_M_FLT, q) && kvm_buf_local(c, lb, a, 1, KVM_M_BF16, kc) && kvm_buf_local(c, lb, a, 2, KVM_M_BF16, vc) &&
+         kvm_buf_local(c, lb, a, 3, KVM_M_I32, lens) && kvm_buf_local(c, lb, a, 4, KVM_M_F32, part) && kvm_buf_local(c, lb, a, 5, KVM_M_FLT, kn, true) &&
+         kvm_buf_local(c, lb, a, 6, KVM_M_FLT, vn, true);
+    gam.p = c.smem; gam.ld = 0;
+    if (ok && qkn) ok = kvm_buf(c, a[18], KVM_M_F32, gam) && kvm_mat_ok(c, gam, 2, hd);
+    if (ok) ok = kvm_mat_ok(c, q, bb + 1, H * hd) && kvm_mat_ok(c, part, (long long)(bb + 1) * S * H, hd + 2) && kvm_mat_ok(c, kn, bb + 1, Hkv * hd) && kvm_mat_ok(c, vn, bb + 1, Hkv * hd);
+    if (ok && (!kn.p || !vn.p)) { c.fail(KVM_OPE_SHAPE, hd, a[17]); ok = false; }
+    P.lb = lb; P.a = a; P.qkn = qkn; P.gam = (const float*)gam.p; P.gam_ld = gam.ld; P.G = H / Hkv; P.nk = max(j1 - j0, 0); P.newrow = newrow;
+    P.p0 = ok ? ((const int*)lens.p)[bb] : 0;
+  }
+  const float theta = kvm_bits_f32(a[16]);
   unsigned char* Ks = kvm_ring_stage(ring, cit);
   unsigned char* Vs = kvm_ring_stage(ring, cit + 1);
-  auto wait_use = [&](unsigned it) {
-    const uint32_t bar = kvm_ring_full(ring, it), par = kvm_ring_parity(ring, it);
-    unsigned spins = 0;
-    while (!kvm_mbar_test(bar, par)) if ((++spins & 1023u) == 0 && (kvm_globaltimer() > deadline || *(volatile int*)&c.err->code != 0)) return false;
-    return true;
-  };
-  kvm_sync();                                              // the previous task is done with the scratch
   bool waited = true;
+  auto wk = [&]() { return kvm_ring_wait_warp(ring, cit, c.deadline, c.err); };
+  auto wv = [&]() { return kvm_ring_wait_warp(ring, cit + 1, c.deadline, c.err); };
   if (ok) {
-    KvmPartPro P;
-    P.q = q; P.kc = kc; P.vc = vc; P.kn = kn; P.vn = vn; P.gam = gam;
-    P.b = b; P.kvh = kvh; P.G = G; P.hd = hd; P.fl = fl; P.p0 = p0; P.base = (size_t)(b * Hkv + kvh) * Tmax; P.theta = theta; P.eps = qkn ? kvm_bits_f32(a[19]) : 0.0f;
-    P.appends = newrow >= 0;
-    P.rope_cache = c.rope_cache;
-    P.qs = (float*)(sm + KVM_AS_OFF_QS); P.inv = (float*)(sm + KVM_AS_OFF_INV); P.kns = (float*)(sm + KVM_AS_OFF_KNEW); P.vns = (float*)(sm + KVM_AS_OFF_VNEW);
-    P.rsq = (float*)(sm + KVM_AS_OFF_ML);
-    unsigned long long t_wait = 0;
-    auto prologue = [&]() {
-      kvm_part_prologue(P);
-      if (stamp && threadIdx.x == 0) stamp[0] = (int)min(255ull, (kvm_globaltimer() - t_task) / 100);      // trace detail, byte 0: start to end of the prologue (0.1 us)
-    };
-    float* pp = (float*)part.p;
-    auto emit = [&](int g, int cc, float M, float Lsum, float A) {
-      const size_t row = ((size_t)(b * S + s) * H + kvh * G + g) * part.ld;
-      pp[row + cc] = Lsum > 0.0f ? A : 0.0f;
-      if (cc == 0) { pp[row + hd] = Lsum > 0.0f ? M : KVM_ATTN_EMPTY_M_STREAM; pp[row + hd + 1] = Lsum; }
-    };
-    auto timed_wait = [&](unsigned it) {
-      const unsigned long long t0 = stamp && threadIdx.x == 0 ? kvm_globaltimer() : 0;
-      const bool r = wait_use(it);
-      if (stamp && threadIdx.x == 0) t_wait += kvm_globaltimer() - t0;
-      return r;
-    };
-    auto wk = [&]() { return timed_wait(cit); };
-    auto wv = [&]() { return timed_wait(cit + 1); };
-    if (G <= 1) waited = kvm_attn_part_core<1>(sm, Ks, Vs, nk, newrow, G, hd, sc, prologue, wk, wv, emit);
-    else if (G <= 2) waited = kvm_attn_part_core<2>(sm, Ks, Vs, nk, newrow, G, hd, sc, prologue, wk, wv, emit);
-    else if (G <= 4) waited = kvm_attn_part_core<4>(sm, Ks, Vs, nk, newrow, G, hd, sc, prologue, wk, wv, emit);
-    else waited = kvm_attn_part_core<8>(sm, Ks, Vs, nk, newrow, G, hd, sc, prologue, wk, wv, emit);
-    if (stamp && threadIdx.x == 0) stamp[0] |= (int)min(255ull, t_wait / 100) << 8;       // byte 1: waits for the keys and the values (0.1 us)
+    // theta^(-2i/hd) is a double-precision pow per frequency: computed once per (theta, head dimension) and launch, not per task
+    float* rc = c.rope_cache;
+    if (__float_as_int(rc[0]) != __float_as_int(theta) || __float_as_int(rc[1]) != hd) {
+      kvm_sync();                                          // every thread has looked at the key before anyone replaces it
+      for (int i = threadIdx.x; i < hd / 2; i += KVM_NT) rc[2 + i] = kvm_rope_inv(theta, i, hd);
+      if (threadIdx.x == 0) { rc[0] = theta; rc[1] = __int_as_float(hd); }
+      kvm_sync();
+    }
+    P.inv = rc + 2;
+    waited = kvm_ra_part<HD, GT>(P, c.smem, Ks, Vs, wk, wv);
   } else {
-    waited = wait_use(cit) && wait_use(cit + 1);
+    waited = wk() && wv();
   }
   if (!waited && *(volatile int*)&c.err->code == 0) kvm_stream_timeout(c, 1135);
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the appended row was written by threads; the next copies into these stages come after it
-  kvm_sync();
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the stages were written by threads; the next copies into them come after it
+  __syncwarp();
   if (waited && (threadIdx.x & 31) == 0) { kvm_mbar_arrive(kvm_ring_empty(ring, cit)); kvm_mbar_arrive(kvm_ring_empty(ring, cit + 1)); }
+}
+
+__device__ __forceinline__ void kvm_attn_part_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool qkn, const KvmRing ring, unsigned cit, int j0, int j1, int newrow) {
+  const int hd = a[13];
+  const bool few = a[11] <= 4 * a[12];
+  if (hd == 128) { if (few) kvm_attn_part_ring_t<128, 4>(c, a, lb, qkn, ring, cit, j0, j1, newrow); else kvm_attn_part_ring_t<128, 8>(c, a, lb, qkn, ring, cit, j0, j1, newrow); }
+  else if (hd == 64) { if (few) kvm_attn_part_ring_t<64, 4>(c, a, lb, qkn, ring, cit, j0, j1, newrow); else kvm_attn_part_ring_t<64, 8>(c, a, lb, qkn, ring, cit, j0, j1, newrow); }
+  else kvm_attn_part_ring_t<32, 8>(c, a, lb, qkn, ring, cit, j0, j1, newrow);
 }
 
 // ---- front warp: stream geometry of a fetched task (lane 0) ---------------------------------------------------------------------
@@ -641,16 +627,16 @@ static __device__ void kvm_static_geometry(const KvmDevState& S, KvmStSlot& sl, 
   } else if (op == 135 || op == 300) {
     const int kci = a[1], vci = a[2], li = a[3], b = a[7], kvh = a[8], s = a[9], Sp = a[10], H = a[11], Hkv = a[12], hd = a[13], Tmax = a[14], fl = a[17];
     if (kci < 0 || kci >= S.nbufs || vci < 0 || vci >= S.nbufs || li < 0 || li >= S.nbufs) return;
-    if (b < 0 || Hkv <= 0 || H <= 0 || H % Hkv || kvh < 0 || kvh >= Hkv || s < 0 || Sp <= 0 || s >= Sp || Tmax <= 0 || !(fl == 0 || fl == 1 || fl == 3)) return;
+    if (b < 0 || Hkv <= 0 || H <= 0 || H % Hkv || kvh < 0 || kvh >= Hkv || s < 0 || Sp <= 0 || s >= Sp || Tmax <= 0 || fl != 3) return;      // other flags: the op's own form
     const int G = H / Hkv;
-    if (G > 8 || (G & (G - 1)) || !(hd == 16 || hd == 32 || hd == 64 || hd == 128)) return;
+    if (G > 8 || !(hd == 32 || hd == 64 || hd == 128)) return;
     const KvmBuf kc = sl.lb[1], vc = sl.lb[2], lens = sl.lb[3];
     if (!kc.p || !vc.p || !lens.p || kc.dtype != KVM_BF16 || vc.dtype != KVM_BF16 || lens.dtype != KVM_I32 || kc.ld != hd || vc.ld != hd || ((uintptr_t)kc.p & 15) || ((uintptr_t)vc.p & 15)) return;
     if ((long long)(b + 1) * Hkv * Tmax > kc.rows || (long long)(b + 1) * Hkv * Tmax > vc.rows || hd > kc.cols || hd > vc.cols || lens.ld != lens.cols || b >= lens.rows * lens.cols) return;
     const int p0 = ((const int*)lens.p)[b], n = p0 + 1;
     if (p0 < 0 || n > Tmax) return;
     const int chunk = (n + Sp - 1) / Sp, j0 = s * chunk, j1 = min(n, s * chunk + chunk), nk = max(j1 - j0, 0);
-    if (nk * hd * 2 > KVM_ST_STAGE || kvm_attn_part_scratch(nk, G, hd) > scratch_bytes) return;
+    if (nk * hd * 2 > KVM_ST_STAGE || KVM_RA_BYTES > scratch_bytes) return;
     sl.kind = 2; sl.nchunks = 2; sl.j0 = j0; sl.j1 = j1;
     sl.newrow = ((fl & 1) && j0 <= n - 1 && n - 1 < j1) ? n - 1 - j0 : -1;
   }
@@ -896,8 +882,8 @@ __global__ void __launch_bounds__(KVM_ST_THREADS, 1) kvm_static_kernel(KvmStatic
         else kvm_gemv_ring_wide(c, sl.args, sl.lb, ring, cit, sl.R, nch);
       }
       else if (kind == 3) kvm_gemv_mma_ring(c, sl.args, sl.lb, op == 301, ring, cit, sl.newrow, deadline, t_task, S.trace ? sctl + 3 : nullptr);
-      else if (kind == 2) kvm_attn_part_ring(c, sl.args, sl.lb, op == 300, ring, cit, sl.j0, sl.j1, sl.newrow, deadline, t_task, S.trace ? sctl + 3 : nullptr);
-      else if (op != 0 && go == 1) kvm_dispatch(c, op, sl.args, sl.aux);
+      else if (kind == 2) kvm_attn_part_ring(c, sl.args, sl.lb, op == 300, ring, cit, sl.j0, sl.j1, sl.newrow);
+      else if (op != 0 && go == 1 && !(op == 136 && kvm_hot_merge(c, sl.args))) kvm_dispatch(c, op, sl.args, sl.aux);
       cit += (unsigned)nch;
       // Results that a later bulk copy or TMA load may read (cache rows appended by an attention split, operands of tensor-core ops)
       // need the writer's generic-to-async proxy fence.  A streamed GEMV writes activations only, which every consumer reads with
