@@ -202,7 +202,11 @@ static int kvm_plan_static(KvmExec* h, const std::vector<int>& base_versions, Kv
       any_stream = true;
       if (d.op_id == 301) any_rows = true;
       const int K = a[8];
-      if (K <= 0 || (K & 255) || K * 2 > KVM_ST_STAGE) all_fit = false;       // such a row does not stream through a stage: run the whole program without the ring
+      if (K <= 0 || K * 2 > KVM_ST_STAGE) all_fit = false;       // such a row does not stream through a stage: run the whole program without the ring
+      else if (K & 255) {                       // 16-byte pieces of a row are all the one-row consumer needs, with its scratch beside the ring
+        const KvmBuf* w = a[3] >= 0 && a[3] < (int)h->bufs.size() ? &h->bufs[a[3]] : nullptr;
+        if (d.op_id == 301 || (K & 7) || !w || (w->ld & 7) || ((uintptr_t)w->p & 15) || 272 + (long long)(a[7] - a[6]) * 16 * 4 + K * 2 > 32768) all_fit = false;
+      }
       if (a[3] >= 0 && a[3] < nb && !written[a[3]]) plan.stream[t] = 1;
     } else if (d.op_id == 135 || d.op_id == 300) {
       if (a[1] >= 0 && a[2] >= 0 && a[3] >= 0 && a[1] < nb && a[2] < nb && a[3] < nb && !written[a[1]] && !written[a[2]] && len_ok[t]) plan.stream[t] = 1;
