@@ -878,7 +878,7 @@ __global__ void __launch_bounds__(KVM_ST_THREADS, 1) kvm_static_kernel(KvmStatic
       if (kind == 1) {
         const int J = (sl.args[8] + 256 * kvm_gv_parts(sl.args[8]) - 1) / (256 * kvm_gv_parts(sl.args[8]));      // pieces of eight columns per thread
         if (J == 1) kvm_gemv_ring<1>(c, sl.args, sl.lb, ring, cit, sl.R, nch, S.trace ? sctl + 3 : nullptr);
-        else if (J <= 3) kvm_gemv_ring_3(c, sl.args, sl.lb, ring, cit, sl.R, nch, S.trace ? sctl + 3 : nullptr);
+        else if (J <= 3) kvm_gemv_ring<3>(c, sl.args, sl.lb, ring, cit, sl.R, nch, S.trace ? sctl + 3 : nullptr);
         else kvm_gemv_ring_wide(c, sl.args, sl.lb, ring, cit, sl.R, nch);
       }
       else if (kind == 3) kvm_gemv_mma_ring(c, sl.args, sl.lb, op == 301, ring, cit, sl.newrow, deadline, t_task, S.trace ? sctl + 3 : nullptr);
