@@ -208,6 +208,8 @@ static int kvm_plan_static(KvmExec* h, const std::vector<int>& base_versions, Kv
         if (d.op_id == 301 || (K & 7) || !w || (w->ld & 7) || ((uintptr_t)w->p & 15) || 272 + (long long)(a[7] - a[6]) * 16 * 4 + K * 2 > 32768) all_fit = false;
       }
       if (a[3] >= 0 && a[3] < nb && !written[a[3]]) plan.stream[t] = 1;
+    } else if (d.op_id == 45 || d.op_id == 47 || d.op_id == 48) {
+      all_fit = false;                          // their operand tiles want the ring's shared memory
     } else if (d.op_id == 135 || d.op_id == 300) {
       if (a[1] >= 0 && a[2] >= 0 && a[3] >= 0 && a[1] < nb && a[2] < nb && a[3] < nb && !written[a[1]] && !written[a[2]] && len_ok[t]) plan.stream[t] = 1;
     }
