@@ -5,6 +5,8 @@
 // Products run on mma.sync m16n8k16 (bf16 operands, float32 sums) at float32 precision: a float32 operand is split into three bf16
 // terms of eight bits each and the products of terms whose orders sum to less than three are added (the rest is below 2^-24); a bf16
 // operand is its own single term.  Scores of bf16 inputs are therefore exact products, and the probabilities keep float32 precision.
+// The matrix unit truncates where it adds to the accumulator, so a running sum in it drifts towards zero with every instruction: the
+// terms of sixteen products are added from zero, smallest first, and the running sums are float32 adds.
 //
 // A warp owns sixteen rows of the task's block from the scores to the output (flash form, 32 keys at a time, nothing but operands in
 // shared memory).  Warps left over share the other side: KG groups of warps take every KG-th key tile and are added up at the end in
@@ -98,20 +100,30 @@ __device__ __forceinline__ void kvm_am_scores(float (&s)[4][4], const __nv_bfloa
   const __nv_bfloat16* bp = B + (nb + (lane & 7) + ((lane >> 4) << 3)) * P + ((lane >> 3) & 1) * 8;
 #pragma unroll(HD >= 128 && NT > 1 ? 1 : 2)
   for (int ks = 0; ks < HD / 16; ++ks) {
+    float d[4][4];
+    if (NT > 1)
 #pragma unroll
-    for (int i = 0; i < NT; ++i) {
+      for (int n = 0; n < 4; ++n) d[n][0] = d[n][1] = d[n][2] = d[n][3] = 0.0f;
+    float (&to)[4][4] = NT > 1 ? d : s;
+#pragma unroll
+    for (int i = NT - 1; i >= 0; --i) {
       uint32_t a[4];
       kvm_am_ldm4(a, ap + (size_t)i * arows * P + ks * 16);
 #pragma unroll
-      for (int j = 0; j < NT - i; ++j)
+      for (int j = NT - 1 - i; j >= 0; --j)
 #pragma unroll
         for (int np = 0; np < 2; ++np) {
           uint32_t b[4];
           kvm_am_ldm4(b, bp + (size_t)j * brows * P + np * 16 * P + ks * 16);
-          kvm_am_mma(s[2 * np], a, b[0], b[1]);
-          kvm_am_mma(s[2 * np + 1], a, b[2], b[3]);
+          kvm_am_mma(to[2 * np], a, b[0], b[1]);
+          kvm_am_mma(to[2 * np + 1], a, b[2], b[3]);
         }
     }
+    if (NT > 1)
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[n][e] += d[n][e];
   }
 }
 // acc[16 x NCOL] += p[16 x 32] times B rows kb.. (32 of them), columns n0..
@@ -129,14 +141,18 @@ __device__ __forceinline__ void kvm_am_accum(float (&acc)[KvmAm<HD>::NCOL / 8][4
       a[i][2] = kvm_am_term2(p[2 * kk + 1][0], p[2 * kk + 1][1]); a[i][3] = kvm_am_term2(p[2 * kk + 1][2], p[2 * kk + 1][3]);
     }
 #pragma unroll
-    for (int np = 0; np < KvmAm<HD>::NCOL / 16; ++np)
+    for (int np = 0; np < KvmAm<HD>::NCOL / 16; ++np) {
+      float d[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
 #pragma unroll
-      for (int j = 0; j < NT; ++j) {
+      for (int j = NT - 1; j >= 0; --j) {
         uint32_t b[4];
         kvm_am_ldm4t(b, bp + (size_t)j * brows * P + kk * 16 * P + np * 16);
 #pragma unroll
-        for (int i = 0; i < 3 - j; ++i) { kvm_am_mma(acc[2 * np], a[i], b[0], b[1]); kvm_am_mma(acc[2 * np + 1], a[i], b[2], b[3]); }
+        for (int i = 2 - j; i >= 0; --i) { kvm_am_mma(d[0], a[i], b[0], b[1]); kvm_am_mma(d[1], a[i], b[2], b[3]); }
       }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { acc[2 * np][e] += d[0][e]; acc[2 * np + 1][e] += d[1][e]; }
+    }
   }
 }
 // Output rows of a warp: row lane/4 (+8) of the block at global row r0, columns col0 + ...; rows from `valid` on and columns from hd on are padding.
