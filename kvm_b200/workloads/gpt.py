@@ -319,7 +319,7 @@ class _Emit:
                    ['opt_step'], [dst], self.prio, f'{tag}window.{dst}')
         x = B('x0', N, d)
         self._rowwise = {x}
-        self.rows('embedding_fwd', tag + 'embed', N, c.norm_rows, {'ids': ids, 'wte': 'w.wte', 'wpe': 'w.wpe', 'out': x, 'T': T, 'd': d},
+        self.rows('embedding_fwd', tag + 'embed', N, c.norm_rows if N > 4 * c.norm_rows else 4 * c.norm_rows, {'ids': ids, 'wte': 'w.wte', 'wpe': 'w.wpe', 'out': x, 'T': T, 'd': d},
                   ['w.wte', 'w.wpe'], [x], vec_r=[ids])
         saved = []
         for l in range(L):
