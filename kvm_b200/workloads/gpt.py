@@ -106,6 +106,11 @@ def param_shapes(c: GPTConfig):
     return out
 
 
+def opt_chunk(c: GPTConfig) -> int:
+    """Elements per optimizer chunk: the parameters are updated side by side, about two chunks per SM."""
+    return Graph.spread(sum(rows * cols for _, rows, cols, _, _ in param_shapes(c)) // 2, c.flat_chunk)
+
+
 def dp_exchange_layout(c: GPTConfig, world: int):
     """Layout of the in-launch gradient exchange of data parallelism over `world` ranks, the same on every rank: the gradient arena
     ({parameter: element offset}, 64-element aligned, and its length), the exchange chunks [(parameter, e0, e1)] (the optimizer's
@@ -116,7 +121,7 @@ def dp_exchange_layout(c: GPTConfig, world: int):
         tmp.buffer('w.' + name, rows, cols)
         arena[name] = off
         off += -(-rows * cols // 64) * 64
-        chunks += [(name, e0, e1) for e0, e1 in tmp.flat_chunks('w.' + name, c.flat_chunk)]
+        chunks += [(name, e0, e1) for e0, e1 in tmp.flat_chunks('w.' + name, opt_chunk(c))]
     width = -(-max(e1 - e0 for _, e0, e1 in chunks) // 4) * 4
     return arena, off, chunks, width, -(-len(chunks) // world)
 
@@ -174,10 +179,10 @@ class _Emit:
         return ('wb.' if self.bf else 'w.') + name
 
     # ---- op helpers (each emits the tile tasks of one logical op)
-    def flat(self, op, bufs_r, bufs_w, n_elems, args, tag):
+    def flat(self, op, bufs_r, bufs_w, n_elems, args, tag, chunk=None):
         """Elementwise op over equally shaped buffers, chunked on row boundaries."""
         g = self.g
-        for i, (e0, e1) in enumerate(g.flat_chunks(bufs_w[0], self.c.flat_chunk)):
+        for i, (e0, e1) in enumerate(g.flat_chunks(bufs_w[0], chunk or g.spread(n_elems, self.c.flat_chunk))):
             rd = [(b, *g.region_of(b, e0, e1)) for b in bufs_r]
             wr = [(b, *g.region_of(b, e0, e1)) for b in bufs_w]
             g.task(op, {**args, 'e0': e0, 'e1': e1}, rd, wr, self.prio, f'{tag}.{i}')
@@ -310,7 +315,7 @@ class _Emit:
         if self.bf:
             for name, (rows, cols, mat) in self.params.items():
                 if mat:
-                    self.flat('round_bf16', ['w.' + name], ['wb.' + name], rows * cols, {'x': 'w.' + name, 'out': 'wb.' + name}, tag + 'shadow.' + name)
+                    self.flat('round_bf16', ['w.' + name], ['wb.' + name], rows * cols, {'x': 'w.' + name, 'out': 'wb.' + name}, tag + 'shadow.' + name, opt_chunk(c))
             if c.tied:
                 self.flat('round_bf16', ['w.wte'], ['wb.wte'], V * d, {'x': 'w.wte', 'out': 'wb.wte'}, tag + 'shadow.wte')
         ids, tgt = B('ids', N, 1, 'i32'), B('tgt', N, 1, 'i32')
@@ -417,7 +422,7 @@ class _Emit:
         # ---------------- clip + AdamW, bracketed by the two publishes of `weights`
         chunks = []
         for name, (rows, cols, _) in self.params.items():
-            for e0, e1 in g.flat_chunks('w.' + name, c.flat_chunk):
+            for e0, e1 in g.flat_chunks('w.' + name, opt_chunk(c)):
                 chunks.append((name, e0, e1))
         if self.dp_fused:
             self.dp_exchange(tag, chunks)

@@ -40,6 +40,9 @@ class _Records:
             self.n = k
 
 
+SMS = 148        # workers of the executor on a B200: one CTA per SM
+
+
 class Graph:
     def __init__(self, name='train'):
         self.name = name
@@ -109,6 +112,12 @@ class Graph:
         if e0 // c == (e1 - 1) // c:
             return (e0 // c, e0 // c + 1), (e0 % c, (e1 - 1) % c + 1)
         return (e0 // c, -(-e1 // c)), ALL
+
+    @staticmethod
+    def spread(n, chunk, least=4096):
+        """Chunk length for a phase of `n` elements: `chunk`, or less where that would leave SMs without a task.  Below 4096 elements a
+        task is all fixed cost (3-4 us)."""
+        return min(chunk, max(least, -(-n // SMS)))
 
     def flat_chunks(self, buf, target):
         """Flat ranges [e0,e1) of about `target` elements covering `buf`, cut on row boundaries (or inside single rows when a row

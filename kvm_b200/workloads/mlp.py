@@ -67,7 +67,8 @@ def build_mlps(c: MLPConfig, steps: int) -> Graph:
                        prio, f'{tag}.{m0 // 64}.{n0 // 64}')
 
     def flat(op, tag, bufs, n, extra, reads, writes, prio=10):
-        for i, (e0, e1) in enumerate(g.flat_chunks(writes[0], c.flat_chunk)):      # chunks on row boundaries: no false dependencies
+        # the same phase of all the models side by side (most of their elements are width x width)
+        for i, (e0, e1) in enumerate(g.flat_chunks(writes[0], g.spread(n * sum(v * v for v in c.widths) // width ** 2, c.flat_chunk))):      # chunks on row boundaries: no false dependencies
             g.task(op, dict(bufs, e0=e0, e1=e1, **extra), [(b, *g.region_of(b, e0, e1)) for b in reads], [(b, *g.region_of(b, e0, e1)) for b in writes], prio, f'{tag}.{i}')
 
     for mi, w in enumerate(c.widths):
