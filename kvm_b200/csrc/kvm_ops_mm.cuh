@@ -175,10 +175,106 @@ static __device__ __noinline__ void kvm_mm_simt_t(const KvmCtx& c, const KvmMmAr
       }
     }
 }
+// Tiles of 32x32 at most (what the training graphs cut a product into that would occupy few SMs, so that its length counts and not its
+// rate).  Eight warps multiply, a thread owns 2 rows x 2 columns; the other eight stage, two chunks ahead in registers.  The product is
+// rounded before it is added; packed FMAs do both with one rounding each, x * y + (-0) and the sum.  The constant comes from constant
+// memory, since the compiler contracts a packed multiply and add into one FMA when it sees them.
+// What bounds it: shared memory delivers 128 bytes a cycle, 32 cycles per k for the eight warps' two 8-byte loads; the 64x64 form
+// above takes four times its share of latency per k at this size.  At K = 512 a tile takes 19 us, of which
+// 5 are the call and the first loads (64x64 form: 27-30 us for such a tile, 39 us for a whole one).
+static __constant__ unsigned long long kvm_mm_nzero2 = 0x8000000080000000ull;      // (-0, -0)
+template <bool VEC>
+static __device__ __noinline__ void kvm_mm_simt_32(const KvmCtx& c, const KvmMmArgs& g) {
+  extern __shared__ __align__(1024) unsigned char kvm_smem[];
+  unsigned char* sm = kvm_smem + (uint32_t)(c.smem - kvm_smem);      // the compiler sees shared memory (through the context's pointer every access is a generic one)
+  const bool ta = g.flags & 1, tb = g.flags & 2;
+  const int mb = g.m0, nb = g.n0, m_end = min(mb + g.tm, g.M), n_end = min(nb + g.tn, g.N), K = g.K, nch = (K + 31) / 32;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  kvm_sync();                                               // whatever used the scratch before is done with it
+  if (tid >= 256) {
+    const int t = tid & 255, am = ta ? (t & 7) * 4 : t >> 3, ak = ta ? t >> 3 : (t & 7) * 4, bn = tb ? t >> 3 : (t & 7) * 4, bk = tb ? (t & 7) * 4 : t >> 3;
+    const KvmBuf ga = g.a, gb = g.b;
+    const bool ro = g.round_ops;
+    float xa[4][4], xb[4][4];
+    auto fetch = [&](int i, float (&va)[4], float (&vb)[4]) {
+      if (i >= nch) return;
+      const int k0 = i * 32;
+      if (ta) kvm_sm_fetch<VEC>(ga, ro, k0 + ak, mb + am, K, m_end, va); else kvm_sm_fetch<VEC>(ga, ro, mb + am, k0 + ak, m_end, K, va);
+      if (tb) kvm_sm_fetch<VEC>(gb, ro, nb + bn, k0 + bk, n_end, K, vb); else kvm_sm_fetch<VEC>(gb, ro, k0 + bk, nb + bn, K, n_end, vb);
+    };
+    auto put1 = [&](unsigned char* st, int o, int k, bool along_k, const float (&v)[4]) {      // element (o, k) of a [k][32] array, four along k or along o
+      const int q = (k >> 2) & 7;
+      if (along_k) {
+        const int at = (((o >> 2) ^ q) << 4) + (o & 3) * 4;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) *(float*)(st + (k + j) * 128 + at) = v[j];
+      } else *(float4*)(st + k * 128 + (((o >> 2) ^ q) << 4)) = make_float4(v[0], v[1], v[2], v[3]);
+    };
+    auto put = [&](int i, const float (&va)[4], const float (&vb)[4]) {
+      if (i >= nch) return;
+      unsigned char* st = sm + (i & 1) * 8192;
+      put1(st, am, ak, !ta, va); put1(st + 4096, bn, bk, tb, vb);
+    };
+#pragma unroll
+    for (int u = 0; u < 4; ++u) fetch(u, xa[u], xb[u]);
+    put(0, xa[0], xb[0]);
+    fetch(4, xa[0], xb[0]);
+#pragma unroll 1
+    for (int i = 0; i < nch; i += 4)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (i + u >= nch) break;
+        kvm_sync();                                         // chunk i + u is in its buffer
+        put(i + u + 1, xa[(u + 1) & 3], xb[(u + 1) & 3]);
+        fetch(i + u + 5, xa[(u + 1) & 3], xb[(u + 1) & 3]);
+      }
+    return;
+  }
+  const int rg = (warp & 1) * 8 + (lane & 7), cg = (warp >> 1) * 4 + (lane >> 3);      // rows 2 rg, + 1; columns 2 cg, + 1
+  const bool active = mb + (warp & 1) * 16 < m_end && nb + (warp >> 1) * 8 < n_end;
+  const unsigned long long nzero = kvm_mm_nzero2;
+  unsigned long long acc0 = 0ull, acc1 = 0ull;
+#pragma unroll 1
+  for (int i = 0; i < nch; ++i) {
+    kvm_sync();                                             // chunk i is in its buffer
+    if (!active) continue;
+    const unsigned char* st = sm + (i & 1) * 8192;
+    const unsigned char* xp = st + (rg & 1) * 8;
+    const unsigned char* yp = st + 4096 + (cg & 1) * 8;
+    const int kmax = min(32, K - i * 32);
+    auto step = [&](int k, int q) {
+      const float2 x = *(const float2*)(xp + k * 128 + (((rg >> 1) ^ q) << 4));
+      const unsigned long long y = *(const unsigned long long*)(yp + k * 128 + (((cg >> 1) ^ q) << 4));
+      unsigned long long x0, x1, p0, p1;
+      asm("mov.b64 %0, {%1, %1};" : "=l"(x0) : "f"(x.x));
+      asm("mov.b64 %0, {%1, %1};" : "=l"(x1) : "f"(x.y));
+      asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p0) : "l"(x0), "l"(y), "l"(nzero));
+      asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p1) : "l"(x1), "l"(y), "l"(nzero));
+      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(acc0) : "l"(p0), "l"(acc0));
+      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(acc1) : "l"(p1), "l"(acc1));
+    };
+    if (kmax == 32) {
+#pragma unroll 1
+      for (int k4 = 0; k4 < 32; k4 += 8)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) step(k4 + k, ((k4 + k) >> 2) & 7);
+    } else
+      for (int k = 0; k < kmax; ++k) step(k, (k >> 2) & 7);
+  }
+  if (!active) return;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const float2 v = r ? *(float2*)&acc1 : *(float2*)&acc0;
+    const int m = mb + 2 * rg + r, n = nb + 2 * cg;
+    if (m < m_end && n < n_end) kvm_st(g.out, (size_t)m * g.out.ld + n, kvm_mm_epilogue(g, v.x, m, n));
+    if (m < m_end && n + 1 < n_end) kvm_st(g.out, (size_t)m * g.out.ld + n + 1, kvm_mm_epilogue(g, v.y, m, n + 1));
+  }
+}
 static __device__ void kvm_mm_simt(const KvmCtx& c, const KvmMmArgs& g) {
   // vector loads: float32 operands as they are (no rounding), rows and tile origin on 16-byte boundaries
   const bool vec = !g.round_ops && g.a.dtype == KVM_F32 && g.b.dtype == KVM_F32 && ((g.a.ld | g.b.ld | g.m0 | g.n0) & 3) == 0 && kvm_vec_ok(g.a) && kvm_vec_ok(g.b);
-  if (vec) kvm_mm_simt_t<true>(c, g); else kvm_mm_simt_t<false>(c, g);
+  if (min(g.tm, g.M - g.m0) <= 32 && min(g.tn, g.N - g.n0) <= 32) { if (vec) kvm_mm_simt_32<true>(c, g); else kvm_mm_simt_32<false>(c, g); }
+  else if (vec) kvm_mm_simt_t<true>(c, g); else kvm_mm_simt_t<false>(c, g);
 }
 
 KVM_OP_FN void kvm_op_matmul_tile(const KvmCtx& c, const int32_t* a) {

@@ -193,7 +193,8 @@ class _Emit:
         if self.bf:
             op, tm, tn = 'matmul_mma_bf16', 128, 256
         else:
-            op, tm, tn = 'matmul_tile', 64, 64
+            op, tm = 'matmul_tile', g.f32_tile((M, N))
+            tn = tm
         ta, tb, acc = flags & 1, flags & 2, flags & 4
         for m0 in range(0, M, tm):
             m1 = min(m0 + tm, M)
@@ -210,8 +211,8 @@ class _Emit:
                 wr = [(out, (m0, m1), (n0, n1))]
                 if pre:
                     wr.append((pre, (m0, m1), (n0, n1)))
-                g.task(op, {'a': a, 'b': w, 'out': out, 'bias': bias, 'res': res, 'pre': pre, 'm0': m0, 'n0': n0, 'M': M, 'N': N, 'K': K,
-                            'flags': flags, 'alpha': alpha}, rd, wr, min(self.prio, 7) if ta else self.prio, f'{tag}.{m0 // tm}.{n0 // tn}')
+                g.task(op, {'a': a, 'b': w, 'out': out, 'bias': bias, 'res': res, 'pre': pre, 'm0': m0, 'n0': n0, 'M': m1 if tm == 32 else M, 'N': n1 if tm == 32 else N,
+                            'K': K, 'flags': flags, 'alpha': alpha}, rd, wr, min(self.prio, 7) if ta else self.prio, f'{tag}.{m0 // tm}.{n0 // tn}')
 
     def rows(self, op, tag, N, per, args, reads, writes, vec_r=(), vec_w=()):
         """Row-block tasks over [0,N): matrices in reads/writes are touched on rows [r0,r1); vec_* are [N]-long flat vectors."""

@@ -55,16 +55,20 @@ def build_mlps(c: MLPConfig, steps: int) -> Graph:
         xs.append(g.buffer(f'x.{s}', B, D, init=seeded(f'x.{s}', 1.0, 'normal')))
         ys.append(g.data(f'y.{s}', rng.integers(0, C, size=(B, 1), dtype=np.int32), 'i32'))
 
+    width = None                                 # of the model whose tasks are being added
+
     def mm(tag, a, b, out, M, N, K, flags=0, bias=None, pre=None, prio=10):
-        for m0 in range(0, M, 64):
-            for n0 in range(0, N, 64):
-                m1, n1 = min(m0 + 64, M), min(n0 + 64, N)
+        # the models run side by side: the products of all of them, each with this one's shape in its own width
+        t = g.f32_tile(*((v if M == width else M, v if N == width else N) for v in c.widths))
+        for m0 in range(0, M, t):
+            for n0 in range(0, N, t):
+                m1, n1 = min(m0 + t, M), min(n0 + t, N)
                 ra = (a, (0, K), (m0, m1)) if flags & 1 else (a, (m0, m1), (0, K))
                 rb = (b, (n0, n1), (0, K)) if flags & 2 else (b, (0, K), (n0, n1))
-                g.task('matmul_tile', {'a': a, 'b': b, 'out': out, 'bias': bias, 'res': None, 'pre': pre, 'm0': m0, 'n0': n0, 'M': M, 'N': N, 'K': K,
-                                       'flags': flags, 'alpha': 1.0},
+                g.task('matmul_tile', {'a': a, 'b': b, 'out': out, 'bias': bias, 'res': None, 'pre': pre, 'm0': m0, 'n0': n0, 'M': m1 if t == 32 else M,
+                                       'N': n1 if t == 32 else N, 'K': K, 'flags': flags, 'alpha': 1.0},
                        [ra, rb, (bias, (0, 1), (n0, n1)) if bias else None], [(out, (m0, m1), (n0, n1)), (pre, (m0, m1), (n0, n1)) if pre else None],
-                       prio, f'{tag}.{m0 // 64}.{n0 // 64}')
+                       prio, f'{tag}.{m0 // t}.{n0 // t}')
 
     def flat(op, tag, bufs, n, extra, reads, writes, prio=10):
         # the same phase of all the models side by side (most of their elements are width x width)
@@ -72,6 +76,7 @@ def build_mlps(c: MLPConfig, steps: int) -> Graph:
             g.task(op, dict(bufs, e0=e0, e1=e1, **extra), [(b, *g.region_of(b, e0, e1)) for b in reads], [(b, *g.region_of(b, e0, e1)) for b in writes], prio, f'{tag}.{i}')
 
     for mi, w in enumerate(c.widths):
+        width = w
         p = f'm{mi}.'
         shapes = {'w1': (D, w), 'b1': (1, w), 'w2': (w, w), 'b2': (1, w), 'w3': (w, C), 'b3': (1, C)}
         for n, (r, cc) in shapes.items():
