@@ -36,7 +36,8 @@ __device__ __forceinline__ void kvm_st4(const KvmBuf& b, size_t i, float4 v) {
 }
 
 // ---- layernorm forward, float32 rows -------------------------------------------------------------------------------------------
-// A warp per row, NV float4 per lane; gamma and beta wait in shared memory, the next row is in flight while this one is reduced.
+// A warp per row, NV float4 per lane (pairs of them make up eight neighbouring columns: the general body's order of summation); gamma and beta wait in shared memory, the next row is in flight while this one is reduced.
+__device__ __forceinline__ int kvm_hot_ln_col(int t) { return (threadIdx.x & 31) * 8 + (t >> 1) * 256 + (t & 1) * 4; }      // first column of a lane's piece t
 template <int NV>
 __device__ __forceinline__ void kvm_hot_ln_fwd_t(const KvmBuf& x, const KvmBuf& out, float* mean, float* rstd, const float* gs, int r0, int r1, int d, float eps) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -45,7 +46,7 @@ __device__ __forceinline__ void kvm_hot_ln_fwd_t(const KvmBuf& x, const KvmBuf& 
   float4 nx[NV];
   auto load = [&](int r) {
 #pragma unroll
-    for (int t = 0; t < NV; ++t) { const int k = lane * 4 + t * 128; nx[t] = (r < r1 && k < d) ? *(const float4*)(xp + (size_t)r * x.ld + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+    for (int t = 0; t < NV; ++t) { const int k = kvm_hot_ln_col(t); nx[t] = (r < r1 && k < d) ? *(const float4*)(xp + (size_t)r * x.ld + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
   };
   if (AHEAD) load(r0 + warp);
 #pragma unroll 1
@@ -54,18 +55,18 @@ __device__ __forceinline__ void kvm_hot_ln_fwd_t(const KvmBuf& x, const KvmBuf& 
     float s = 0.0f, q = 0.0f;
     if (!AHEAD) load(r);
 #pragma unroll
-    for (int t = 0; t < NV; ++t) { v[t] = nx[t]; s += (v[t].x + v[t].y) + (v[t].z + v[t].w); }
+    for (int t = 0; t < NV; ++t) { v[t] = nx[t]; s += v[t].x; s += v[t].y; s += v[t].z; s += v[t].w; }
     if (AHEAD) load(r + KVM_NWARPS);
     const float mu = kvm_warp_sum(s) / d;
 #pragma unroll
-    for (int t = 0; t < NV; ++t) if (lane * 4 + t * 128 < d) {
+    for (int t = 0; t < NV; ++t) if (kvm_hot_ln_col(t) < d) {
       v[t].x -= mu; v[t].y -= mu; v[t].z -= mu; v[t].w -= mu;
-      q += (v[t].x * v[t].x + v[t].y * v[t].y) + (v[t].z * v[t].z + v[t].w * v[t].w);
+      q += v[t].x * v[t].x; q += v[t].y * v[t].y; q += v[t].z * v[t].z; q += v[t].w * v[t].w;
     }
     const float rs = 1.0f / sqrtf(kvm_warp_sum(q) / d + eps);
 #pragma unroll
     for (int t = 0; t < NV; ++t) {
-      const int k = lane * 4 + t * 128;
+      const int k = kvm_hot_ln_col(t);
       if (k < d) {
         const float4 g = *(const float4*)(gs + k), b = *(const float4*)(gs + 1024 + k);
         kvm_st4(out, (size_t)r * out.ld + k, make_float4(v[t].x * rs * g.x + b.x, v[t].y * rs * g.y + b.y, v[t].z * rs * g.z + b.z, v[t].w * rs * g.w + b.w));
@@ -105,16 +106,16 @@ __device__ __forceinline__ void kvm_hot_ln_bwd_t(const KvmBuf& x, const KvmBuf& 
     const float* xp = (const float*)x.p + (size_t)r * x.ld;
     float* op = (float*)dx.p + (size_t)r * dx.ld;
 #pragma unroll
-    for (int t = 0; t < NV; ++t) { const int k = lane * 4 + t * 128; xv[t] = k < d ? *(const float4*)(xp + k) : zero; }
+    for (int t = 0; t < NV; ++t) { const int k = kvm_hot_ln_col(t); xv[t] = k < d ? *(const float4*)(xp + k) : zero; }
 #pragma unroll
     for (int t = 0; t < NV; ++t) {
-      const int k = lane * 4 + t * 128;
+      const int k = kvm_hot_ln_col(t);
       if (YB) yb[t] = k < d ? *(const uint2*)((const __nv_bfloat16*)dy.p + (size_t)r * dy.ld + k) : make_uint2(0u, 0u);
       else yf[t] = k < d ? *(const float4*)((const float*)dy.p + (size_t)r * dy.ld + k) : zero;
     }
     const float mu = mean[r], rs = rstd[r];
     auto grad = [&](int t) {                       // dy * gamma of this lane's piece t
-      const int k = lane * 4 + t * 128;
+      const int k = kvm_hot_ln_col(t);
       const float4 y = YB ? kvm_bf16x4(yb[YB ? t : 0]) : yf[YB ? 0 : t];
       if (k >= d) return zero;
       const float4 g = *(const float4*)(gs + k);
@@ -125,14 +126,14 @@ __device__ __forceinline__ void kvm_hot_ln_bwd_t(const KvmBuf& x, const KvmBuf& 
     for (int t = 0; t < NV; ++t) {
       const float4 g = grad(t);
       xv[t] = make_float4((xv[t].x - mu) * rs, (xv[t].y - mu) * rs, (xv[t].z - mu) * rs, (xv[t].w - mu) * rs);
-      s1 += (g.x + g.y) + (g.z + g.w);
-      s2 += (g.x * xv[t].x + g.y * xv[t].y) + (g.z * xv[t].z + g.w * xv[t].w);
+      s1 += g.x; s2 += g.x * xv[t].x; s1 += g.y; s2 += g.y * xv[t].y;
+      s1 += g.z; s2 += g.z * xv[t].z; s1 += g.w; s2 += g.w * xv[t].w;
     }
     s1 = kvm_warp_sum(s1) / d;
     s2 = kvm_warp_sum(s2) / d;
 #pragma unroll
     for (int t = 0; t < NV; ++t) {
-      const int k = lane * 4 + t * 128;
+      const int k = kvm_hot_ln_col(t);
       if (k < d) {
         const float4 g = grad(t);
         const float4 o = acc ? *(const float4*)(op + k) : zero;
