@@ -144,7 +144,7 @@ __device__ __forceinline__ void kvm_tc_store32(const KvmMmArgs& g, const float (
     if (g.pre.p) kvm_st8(g.pre, (size_t)m * g.pre.ld + n + j0, v);
     if (g.flags & 8) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = g.out.dtype == KVM_BF16 ? kvm_gelu_s(v[j]) : kvm_gelu(v[j]);
+      for (int j = 0; j < 8; ++j) v[j] = kvm_gelu(v[j]);
     }
     if (g.res.p) { kvm_ld8(g.res, (size_t)m * g.res.ld + n + j0, t);
 #pragma unroll
@@ -201,7 +201,7 @@ static __device__ void kvm_tc_epilogue_staged(const KvmCtx& c, const KvmMmArgs& 
         if (g.pre.p) kvm_st8(g.pre, (size_t)m * g.pre.ld + n, v);
         if (g.flags & 8) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = g.out.dtype == KVM_BF16 ? kvm_gelu_s(v[j]) : kvm_gelu(v[j]);
+          for (int j = 0; j < 8; ++j) v[j] = kvm_gelu(v[j]);
         }
         if (g.res.p) { kvm_ld8(g.res, (size_t)m * g.res.ld + n, t);
 #pragma unroll
@@ -522,7 +522,7 @@ static __device__ __forceinline__ void kvm_tce_epilogue(const KvmCtx& c, const K
             if (g.pre.p) kvm_st8(g.pre, (size_t)m * g.pre.ld + n, v);
             if (g.flags & 8) {
 #pragma unroll
-              for (int j = 0; j < 8; ++j) v[j] = g.out.dtype == KVM_BF16 ? kvm_gelu_s(v[j]) : kvm_gelu(v[j]);
+              for (int j = 0; j < 8; ++j) v[j] = kvm_gelu(v[j]);
             }
             if (g.res.p) { kvm_ld8(g.res, (size_t)m * g.res.ld + n, t);
 #pragma unroll
