@@ -3,16 +3,16 @@
 // of include/mvm_static.h:1-17,43-51 (list schedule -> per-worker records, cross-worker watermark waits) and its worker loop
 // include/mvm_static.cuh:161-229 (fetch the next record ahead, poll the watermarks, dispatch, publish own progress).
 //
-// One CTA per SM as in the dynamic kernel: 16 compute warps + one FRONT warp.  The front warp walks the worker's list ahead of the
-// compute group: it fetches task records into a four-slot shared-memory ring, polls the task's dependencies (pairs of
+// One CTA per SM as in the dynamic kernel: 16 compute warps, a FRONT warp and a STREAM warp.  The front warp walks the worker's list
+// ahead of the compute group: it fetches task records into a four-slot shared-memory ring, polls the task's dependencies (pairs of
 // (worker, tasks that worker must have finished), lanes in parallel over the pairs), and marks the slot ready.  A worker's
 // progress word is one release store per finished task; nothing else is written to global memory for scheduling.
 //
-// Because a worker knows its next tasks, the front warp also STREAMS AHEAD: for decode GEMVs and split decode attention it
-// issues the bulk copies of the task's weight rows / cache rows into a shared-memory stage ring as soon as stages are free,
-// BEFORE the task's dependencies are resolved (weights and old cache rows do not change during a launch; the host marks a task
-// whose streamed operand is written by some task of the batch, and its copies then wait for the dependencies like everything
-// else).  The dependency wait then only gates the prologue and the arithmetic, so HBM keeps streaming across phase boundaries.
+// Because a worker knows its next tasks, the stream warp STREAMS AHEAD: for decode GEMVs and split decode attention it issues the
+// bulk copies of the task's weight rows / cache rows into a shared-memory stage ring as soon as stages are free, BEFORE the task's
+// dependencies are resolved (weights and old cache rows do not change during a launch; the host marks a task whose streamed operand
+// is written by some task of the batch, and its copies then wait for the dependencies like everything else).  The dependency wait
+// then only gates the prologue and the arithmetic, so HBM keeps streaming across phase boundaries.
 //
 // Every wait is bounded (time limit); on expiry KVM_ERR_TIMEOUT is recorded, every CTA leaves, copies in flight are awaited.
 #pragma once
@@ -302,9 +302,8 @@ __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a,
     }
   }
 }
-KVM_OP_FN void kvm_gemv_ring_3(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing ring, unsigned cit, int R, int NC, int* stamp) { kvm_gemv_ring<3>(c, a, lb, ring, cit, R, NC, stamp); }
-// rows of up to 32 Ki columns (what a stage holds) whose activations do not fit the registers beside the loop's: a function of its own
-KVM_OP_FN void kvm_gemv_ring_wide(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing ring, unsigned cit, int R, int NC) { kvm_gemv_ring<8>(c, a, lb, ring, cit, R, NC, nullptr); }
+// rows of more than 12288 columns (their staging bounds them to 16 Ki): the activations beside the loop do not fit the kernel's registers, a function of its own
+KVM_OP_FN void kvm_gemv_ring_wide(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing ring, unsigned cit, int R, int NC) { kvm_gemv_ring<4>(c, a, lb, ring, cit, R, NC, nullptr); }
 
 // ---- streamed GEMV on tensor cores (gemv_bf16 with one activation row, gemv_bf16_rows with up to eight), consumer side --------------
 // D[16 x 8] += A[16 x 16] B[16 x 8] (mma.sync m16n8k16, bf16 operands, float32 accumulate) with A = activations (rows = activation
