@@ -1,0 +1,48 @@
+"""GPU parity at the sizes where the small-shape kernel forms can go wrong: 32x32 exact matmul tiles, attention of ragged sequences and every
+head dimension, streamed decode rows that are no multiple of 256 columns and odd query-head groups."""
+import numpy as np
+import pytest
+
+from tests.parity import compare, run_both
+from tests.test_gpu_attention import attn_bundle
+from tests.test_gpu_gemm import gemm_bundle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize('flags', [0, 1, 2, 3])
+@pytest.mark.parametrize('shape', [(1, 1, 1), (32, 32, 512), (31, 17, 33), (32, 10, 100), (7, 32, 200), (32, 32, 127)])
+def test_matmul_tile_32_is_bit_exact(kvm_lib, flags, shape):
+    M, N, K = shape
+    ex, vm, res = run_both(gemm_bundle('matmul_tile', M, N, K, flags, 'f32', 'f32', bias=True))
+    assert np.array_equal(ex.read_buffer('out'), vm.buffer('out').a)
+    ex.close()
+
+
+@pytest.mark.parametrize('case', [(1, 5, 1, 1, 16, 'f32'), (2, 17, 2, 1, 32, 'f32'), (1, 129, 3, 1, 64, 'f32'), (1, 257, 2, 2, 128, 'f32'), (1, 257, 2, 1, 64, 'bf16'),
+                                  (1, 300, 2, 1, 128, 'bf16'), (3, 33, 1, 1, 32, 'bf16')])
+def test_attention_ragged(kvm_lib, case):
+    B, T, H, Hkv, hd, dt = case
+    ex, vm, res = run_both(attn_bundle(B, T, H, Hkv, hd, dt))
+    assert ex.tc_task_count() == 0
+    compare(ex, vm, 2e-5 if dt == 'f32' else 6e-3)
+    ex.close()
+
+
+# hidden, heads, kv heads, head dim, ffn: seven query heads per key head; rows of 8 .. more than 12288 columns; one head each
+@pytest.mark.parametrize('widths', [(448, 14, 2, 32, 712), (896, 14, 2, 64, 1096), (72, 1, 1, 128, 12552), (264, 6, 2, 64, 520), (128, 8, 1, 128, 136)])
+@pytest.mark.parametrize('qk_norm', [False, True])
+def test_decode_streams_odd_widths(kvm_lib, widths, qk_norm):
+    from kvm_b200.executor import Executor
+    from kvm_b200.workloads.decode import DecodeConfig, build_decode
+    from oracle.vm_np import VM
+    hidden, heads, kv, hd, ffn = widths
+    b = build_decode(DecodeConfig(hidden=hidden, heads=heads, kv_heads=kv, head_dim=hd, ffn=ffn, vocab=304, ctx=70, init_std=0.05, qk_norm=qk_norm)).to_bundle()
+    vm = VM(b).run()
+    with Executor() as ex:
+        ex.load(b)
+        assert ex.run().done == len(b.tasks)
+        assert ex.plan_info()[:2] == (True, True)
+        for name in ('u0.logits', 'u0.l1.x2'):
+            ref = vm.buffer(name).a
+            assert np.abs(ex.read_buffer(name) - ref).max() <= 1e-2 * np.abs(ref).max(), name
