@@ -267,7 +267,7 @@ __device__ __forceinline__ void kvm_hot_delta_t(const KvmBuf& o, const KvmBuf& d
           const uint32_t x[4] = {ov[u][i].x, ov[u][i].y, ov[u][i].z, ov[u][i].w}, y[4] = {dv[u][i].x, dv[u][i].y, dv[u][i].z, dv[u][i].w};
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            if (B) s += __uint_as_float(x[j] << 16) * __uint_as_float(y[j] << 16) + __uint_as_float(x[j] & 0xffff0000u) * __uint_as_float(y[j] & 0xffff0000u);
+            if (B) { s += __uint_as_float(x[j] << 16) * __uint_as_float(y[j] << 16); s += __uint_as_float(x[j] & 0xffff0000u) * __uint_as_float(y[j] & 0xffff0000u); }
             else s += __uint_as_float(x[j]) * __uint_as_float(y[j]);
           }
         }
@@ -292,7 +292,7 @@ __device__ __forceinline__ bool kvm_hot_delta(const KvmCtx& c, const int32_t* a)
 
 // ---- cross entropy of long bf16 rows (forward and gradient in one op) -------------------------------------------------------------------
 // A row is fetched once, by a bulk copy into shared memory that runs while the row before it is worked on (two row buffers; with
-// room for one only, the next copy starts when the row is done), and read from there three times: maximum, sum, gradient.  Maximum
+// room for one only, the next copy starts when the row is done), and read from there twice: maximum and sum, gradient.  Maximum
 // and sum take one barrier each.  Bound by HBM (read + write, 4 bytes per logit: 4.6 us for 50304 of them at an SM's share) with
 // the exponentials (two per logit, 16 a cycle: 3.2 us) beside it; the loop it replaces read the row twice from HBM, 19 us a row.
 __device__ __forceinline__ bool kvm_hot_ce_fused(const KvmCtx& c, const int32_t* a) {
@@ -324,38 +324,36 @@ __device__ __forceinline__ bool kvm_hot_ce_fused(const KvmCtx& c, const int32_t*
     const int t = tp[r];
     if (!kvm_mbar_wait(bar, (phase0 + r - r0) & 1)) ok = false;
     if (two && tid == 0 && r + 1 < r1) fetch(r + 1);   // the other buffer was last read before the barrier at the end of the previous row
-    __nv_bfloat162 mx = __halves2bfloat162(__ushort_as_bfloat16(0xff80), __ushort_as_bfloat16(0xff80));
-#pragma unroll 4
-    for (int k = tid * 8; k < V; k += KVM_NT * 8) {
-      const uint4 v = *(const uint4*)(row + k * 2);
-      const __nv_bfloat162* h = (const __nv_bfloat162*)&v;
-      mx = __hmax2(mx, __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
-    }
-    float m = kvm_warp_max(fmaxf(__bfloat162float(mx.x), __bfloat162float(mx.y)));
-    float* rr = red + ((r - r0) & 1) * 32;
-    if (lane == 0) rr[warp] = m;
-    kvm_sync();
-    m = rr[0];
-#pragma unroll
-    for (int w = 1; w < KVM_NWARPS; ++w) m = fmaxf(m, rr[w]);
-    const float m2 = m * KVM_LOG2E;
-    float s = 0.0f;
+    float m = -INFINITY, s = 0.0f;                     // online (max, sum) per thread, as the general body
 #pragma unroll 2
     for (int k = tid * 8; k < V; k += KVM_NT * 8) {
       const uint4 v = *(const uint4*)(row + k * 2);
       const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-      float e[4];
+      float x[8];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) e[i] = kvm_ex2(fmaf(__uint_as_float(w[i] << 16), KVM_LOG2E, -m2)) + kvm_ex2(fmaf(__uint_as_float(w[i] & 0xffff0000u), KVM_LOG2E, -m2));
-      s += (e[0] + e[1]) + (e[2] + e[3]);
+      for (int i = 0; i < 4; ++i) { x[2 * i] = __uint_as_float(w[i] << 16); x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+      float mm = x[0];
+#pragma unroll
+      for (int j = 1; j < 8; ++j) mm = fmaxf(mm, x[j]);
+      if (mm > m) { s *= __expf(m - mm); m = mm; }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s += __expf(x[j] - m);
     }
+    float* rr = red + ((r - r0) & 1) * 32;
+    float M = kvm_warp_max(m);
+    if (lane == 0) rr[warp] = M;
+    kvm_sync();
+    M = rr[0];
+#pragma unroll
+    for (int w = 1; w < KVM_NWARPS; ++w) M = fmaxf(M, rr[w]);
+    s = m == -INFINITY ? 0.0f : s * __expf(m - M);
     s = kvm_warp_sum(s);
     if (lane == 0) rr[16 + warp] = s;
     kvm_sync();
     s = 0.0f;
 #pragma unroll
     for (int w = 0; w < KVM_NWARPS; ++w) s += rr[16 + w];
-    const float lse = m + logf(s), l2 = lse * KVM_LOG2E;
+    const float lse = M + logf(s);
     if (tid == 0) { ((float*)ls.p)[r] = lse; ((float*)rl.p)[r] = lse - __bfloat162float(*(const __nv_bfloat16*)(row + t * 2)); }
     __nv_bfloat16* out = (__nv_bfloat16*)dl.p + (size_t)r * dl.ld;
 #pragma unroll 2
@@ -366,7 +364,7 @@ __device__ __forceinline__ bool kvm_hot_ce_fused(const KvmCtx& c, const int32_t*
       uint32_t* ow = (uint32_t*)&o;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        float p = kvm_ex2(fmaf(__uint_as_float(w[i] << 16), KVM_LOG2E, -l2)), q = kvm_ex2(fmaf(__uint_as_float(w[i] & 0xffff0000u), KVM_LOG2E, -l2));
+        float p = __expf(__uint_as_float(w[i] << 16) - lse), q = __expf(__uint_as_float(w[i] & 0xffff0000u) - lse);
         if (k + 2 * i == t) p -= 1.0f;
         if (k + 2 * i + 1 == t) q -= 1.0f;
         const __nv_bfloat162 h = __floats2bfloat162_rn(p * f, q * f);
@@ -542,7 +540,7 @@ __device__ __forceinline__ bool kvm_hot(const KvmCtx& c, int op, const int32_t* 
     case 35: return kvm_hot_ln_fwd(c, a);
     case 37: return kvm_hot_ln_bwd(c, a);
     case 39: return kvm_hot_norm_params(c, a);
-    case 41: return !a[5] && kvm_hot_map<2, true>(c, a[0], a[1], a[2], a[3], a[4], [](const float (&v)[2]) { return __fmul_rn(v[1], kvm_gelu_grad_s(v[0])); });
+    case 41: return !a[5] && kvm_hot_map<2, true>(c, a[0], a[1], a[2], a[3], a[4], [](const float (&v)[2]) { return __fmul_rn(v[1], kvm_gelu_grad(v[0])); });
     case 46: return kvm_hot_delta(c, a);
     case 54: return kvm_hot_adamw(c, a);
     case 55: return kvm_hot_gradnorm(c, a);

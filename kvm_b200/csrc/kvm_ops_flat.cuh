@@ -59,13 +59,6 @@ __device__ __forceinline__ float kvm_gelu_grad(float x) {
   float t = tanhf(0.7978845608028654f * (x + 0.044715f * x * x * x));
   return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * 0.7978845608028654f * (1.0f + 3.0f * 0.044715f * x * x);
 }
-// The derivative through the logistic form (0.5 (1 + tanh u) = 1 / (1 + exp(-2u))), two fast special-function calls per value
-// instead of the thirty-odd instructions of tanhf; relative error about 1e-6.  For results that are stored as bf16 (4e-3).
-__device__ __forceinline__ float kvm_gelu_sig(float x) { return __fdividef(1.0f, 1.0f + __expf(-1.5957691216057308f * (x + 0.044715f * x * x * x))); }
-__device__ __forceinline__ float kvm_gelu_grad_s(float x) {
-  const float s = kvm_gelu_sig(x);
-  return s + x * s * (1.0f - s) * 1.5957691216057308f * (1.0f + 3.0f * 0.044715f * x * x);
-}
 __device__ __forceinline__ float kvm_sigmoid(float x) {
   float e = expf(-fabsf(x));
   return x >= 0 ? 1.0f / (1.0f + e) : e / (1.0f + e);
