@@ -101,7 +101,6 @@ __device__ __forceinline__ bool kvm_ring_wait_warp(const KvmRing& ring, unsigned
 // in registers, since a spilled one costs an L2 round trip per stage (the stages leave 28 KB of L1 for 512 threads' local memory).
 // Partial sums are added in part order.  Semantics as kvm_op_gemv_bf16 (runtime/ref_extra.py:398-415).  Always consumes its nchunks
 // stage uses, also after an error.
-__device__ __forceinline__ float kvm_silu_fast(float x) { return __fdividef(x, 1.0f + __expf(-x)); }      // for values that are rounded to bf16 next
 __device__ __forceinline__ unsigned long long kvm_pack2(float lo, float hi) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
 __device__ __forceinline__ void kvm_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
 __device__ __forceinline__ uint4 kvm_pack_bf16x8(const float (&v)[8]) {
@@ -230,7 +229,7 @@ __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a,
       for (int j = 0; j < J; ++j) {
         float t[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) t[i] = kvm_bf16_round(pro == 1 ? v[j][i] * rs * u[j][i] : pro == 2 ? kvm_silu_fast(v[j][i]) * u[j][i] : v[j][i]);
+        for (int i = 0; i < 8; ++i) t[i] = kvm_bf16_round(pro == 1 ? v[j][i] * rs * u[j][i] : pro == 2 ? kvm_silu(v[j][i]) * u[j][i] : v[j][i]);
         put(j, t);
       }
     } else {

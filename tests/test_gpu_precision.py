@@ -1,0 +1,41 @@
+"""Distances of the streamed and reduced-order kernel forms from float64 evaluations of the same op on the same stored inputs.  Bounds follow
+from the storage type (half a unit of bf16) or from the number of float32 roundings on the path; none is a measured value."""
+import numpy as np
+import pytest
+
+from kvm_b200.executor import Executor
+from kvm_b200.workloads.graph import Graph
+from oracle.ops_np import bf16_round
+
+pytestmark = pytest.mark.gpu
+
+
+def run(g):
+    ex = Executor()
+    ex.load(g.to_bundle())
+    ex.run()
+    return ex
+
+
+def gemv_task(g, op, x, w, out, n0, n1, K, pro=0, x2=None, gamma=None):
+    rows = {'r0': 0, 'r1': 1} if op == 'gemv_bf16_rows' else {}
+    g.task(op, {'x': x, 'x2': x2, 'gamma': gamma, 'w': w, 'out': out, 'res': None, 'n0': n0, 'n1': n1, 'K': K, 'pro': pro, 'eps': 1e-6, **rows}, [x], [(out, (0, 1), (n0, n1))])
+
+
+@pytest.mark.parametrize('op', ['gemv_bf16', 'gemv_bf16_rows'])
+def test_swiglu_activations_are_the_rounded_values(kvm_lib, op):
+    # weight row n picks activation n alone: the output is bf16(silu(x) * x2), far tails included (silu(-87) is a normal float32)
+    K = 1024
+    x = np.concatenate([np.linspace(-95, 95, K // 2), np.random.default_rng(1).standard_normal(K // 2) * 3]).astype(np.float32)
+    g = Graph('silu')
+    g.data('x', x[None]), g.data('u', np.full((1, K), 1.5, np.float32)), g.data('w', np.eye(K, dtype=np.float32), 'bf16'), g.buffer('o', 1, K)
+    for n in range(0, K, 128):
+        gemv_task(g, op, 'x', 'w', 'o', n, n + 128, K, pro=2, x2='u')
+    ex = run(g)
+    assert ex.plan_info()[:2] == (True, True)
+    x = x.astype(np.float64)
+    ref = 1.5 * x / (1 + np.exp(-x))
+    got = ex.read_buffer('o')[0].astype(np.float64)
+    # half a unit of bf16 (normal and subnormal), and the float32 evaluation's few units on top
+    assert (np.abs(got - ref) <= 2.0 ** -8 * (1 + 2.0 ** -10) * np.abs(ref) + 2.0 ** -134).all()
+    ex.close()
