@@ -22,18 +22,20 @@ def gemv_task(g, op, x, w, out, n0, n1, K, pro=0, x2=None, gamma=None):
     g.task(op, {'x': x, 'x2': x2, 'gamma': gamma, 'w': w, 'out': out, 'res': None, 'n0': n0, 'n1': n1, 'K': K, 'pro': pro, 'eps': 1e-6, **rows}, [x], [(out, (0, 1), (n0, n1))])
 
 
-@pytest.mark.parametrize('op', ['gemv_bf16', 'gemv_bf16_rows'])
-def test_swiglu_activations_are_the_rounded_values(kvm_lib, op):
-    # weight row n picks activation n alone: the output is bf16(silu(x) * x2), far tails included (silu(-87) is a normal float32)
-    K = 1024
+@pytest.mark.parametrize('op,K', [('gemv_bf16', 1024), ('gemv_bf16', 4864), ('gemv_bf16', 12296), ('gemv_bf16_rows', 1024)])
+def test_swiglu_activations_are_the_rounded_values(kvm_lib, op, K):
+    # weight row n picks one activation alone: the output is bf16(silu(x) * x2), far tails included (silu(-87) is a normal float32)
     x = np.concatenate([np.linspace(-95, 95, K // 2), np.random.default_rng(1).standard_normal(K // 2) * 3]).astype(np.float32)
+    pick = np.linspace(0, K - 1, 512).astype(int)
+    w = np.zeros((512, K), np.float32)
+    w[np.arange(512), pick] = 1
     g = Graph('silu')
-    g.data('x', x[None]), g.data('u', np.full((1, K), 1.5, np.float32)), g.data('w', np.eye(K, dtype=np.float32), 'bf16'), g.buffer('o', 1, K)
-    for n in range(0, K, 128):
-        gemv_task(g, op, 'x', 'w', 'o', n, n + 128, K, pro=2, x2='u')
+    g.data('x', x[None]), g.data('u', np.full((1, K), 1.5, np.float32)), g.data('w', w, 'bf16'), g.buffer('o', 1, 512)
+    for n in range(0, 512, 64):
+        gemv_task(g, op, 'x', 'w', 'o', n, n + 64, K, pro=2, x2='u')
     ex = run(g)
     assert ex.plan_info()[:2] == (True, True)
-    x = x.astype(np.float64)
+    x = x[pick].astype(np.float64)
     ref = 1.5 * x / (1 + np.exp(-x))
     got = ex.read_buffer('o')[0].astype(np.float64)
     # half a unit of bf16 (normal and subnormal), and the float32 evaluation's few units on top
