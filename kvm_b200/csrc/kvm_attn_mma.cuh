@@ -101,10 +101,8 @@ __device__ __forceinline__ void kvm_am_scores(float (&s)[4][4], const __nv_bfloa
 #pragma unroll(HD >= 128 && NT > 1 ? 1 : 2)
   for (int ks = 0; ks < HD / 16; ++ks) {
     float d[4][4];
-    if (NT > 1)
 #pragma unroll
-      for (int n = 0; n < 4; ++n) d[n][0] = d[n][1] = d[n][2] = d[n][3] = 0.0f;
-    float (&to)[4][4] = NT > 1 ? d : s;
+    for (int n = 0; n < 4; ++n) d[n][0] = d[n][1] = d[n][2] = d[n][3] = 0.0f;
 #pragma unroll
     for (int i = NT - 1; i >= 0; --i) {
       uint32_t a[4];
@@ -115,15 +113,14 @@ __device__ __forceinline__ void kvm_am_scores(float (&s)[4][4], const __nv_bfloa
         for (int np = 0; np < 2; ++np) {
           uint32_t b[4];
           kvm_am_ldm4(b, bp + (size_t)j * brows * P + np * 16 * P + ks * 16);
-          kvm_am_mma(to[2 * np], a, b[0], b[1]);
-          kvm_am_mma(to[2 * np + 1], a, b[2], b[3]);
+          kvm_am_mma(d[2 * np], a, b[0], b[1]);
+          kvm_am_mma(d[2 * np + 1], a, b[2], b[3]);
         }
     }
-    if (NT > 1)
 #pragma unroll
-      for (int n = 0; n < 4; ++n)
+    for (int n = 0; n < 4; ++n)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[n][e] += d[n][e];
+      for (int e = 0; e < 4; ++e) s[n][e] += d[n][e];
   }
 }
 // acc[16 x NCOL] += p[16 x 32] times B rows kb.. (32 of them), columns n0..

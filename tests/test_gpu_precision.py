@@ -41,3 +41,31 @@ def test_swiglu_activations_are_the_rounded_values(kvm_lib, op, K):
     # half a unit of bf16 (normal and subnormal), and the float32 evaluation's few units on top
     assert (np.abs(got - ref) <= 2.0 ** -8 * (1 + 2.0 ** -10) * np.abs(ref) + 2.0 ** -134).all()
     ex.close()
+
+
+def lse_bias(got, ref):
+    """Mean signed error in units of the float32 spacing at the references' size."""
+    return float((got - ref).mean() / np.spacing(np.abs(ref).mean().astype(np.float32)))
+
+
+@pytest.mark.parametrize('T,hd', [(300, 128), (200, 64), (130, 32)])
+def test_attention_scores_do_not_drift(kvm_lib, T, hd):
+    # Products of one sign: a sum kept in the matrix unit's accumulator loses part of a unit with every instruction.  Sixteen products
+    # added from zero lose half a unit of their own sum on average, which is 16 / hd of the score: half a unit of the score altogether;
+    # the float32 adds between them round to nearest, without a mean.
+    rng = np.random.default_rng(0)
+    q, k = (bf16_round(np.abs(rng.standard_normal((T, hd)) * 3).astype(np.float32)) for _ in range(2))
+    g = Graph('attn')
+    g.data('q', q, 'bf16'), g.data('k', k, 'bf16'), g.data('v', k, 'bf16'), g.buffer('o', T, hd), g.buffer('lse', T, 1)
+    for q0 in range(0, T, 128):
+        q1 = min(q0 + 128, T)
+        g.task('attn_fwd', {'q': 'q', 'k': 'k', 'v': 'v', 'o': 'o', 'lse': 'lse', 'b': 0, 'h': 0, 'q0': q0, 'T': T, 'H': 1, 'Hkv': 1, 'hd': hd, 'scale': hd ** -0.5},
+               ['q'], [('o', (q0, q1), (0, hd)), ('lse', (q0, q1))])
+    ex = run(g)
+    assert ex.tc_task_count() == 0
+    s = q.astype(np.float64) @ k.astype(np.float64).T * np.float64(np.float32(hd ** -0.5))
+    s[np.triu_indices(T, 1)] = -np.inf
+    m = s.max(1, keepdims=True)
+    ref = (m + np.log(np.exp(s - m).sum(1, keepdims=True)))[:, 0]
+    assert abs(lse_bias(ex.read_buffer('lse')[:, 0], ref)) <= 0.5
+    ex.close()
