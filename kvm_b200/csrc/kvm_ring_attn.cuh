@@ -4,12 +4,12 @@
 // A split is a few microseconds of HBM time, so what bounds it is the length of its dependency chain.  One warp owns sixteen keys from
 // the scores to the weighted sum of the values; warps meet at three barriers only:
 //   prologue   warp g rotates (and normalises) query head g into a bf16 tile, warp 8 the appended key, warp 9 the appended value
-//   scores     mma.sync m16n8k16 with the query heads as rows (queries and keys are bf16: the products are exact, float32 sums);
+//   scores     mma.sync m16n8k16 with the query heads as rows (queries and keys are bf16: the products are exact, summed sixteen at a time);
 //              both operands are read 16 bytes per lane at the same k offsets (a dot product does not care about the order of k)
 //   softmax    over the warp's sixteen keys by two shuffles; probabilities stay float32
 //   values     lane = HD / 32 columns for all heads, probabilities broadcast from shared memory
 //   merge      each warp scales its sums by exp(own maximum - split's maximum) and parks them in the keys' stage; one pass adds the
-//              sixteen warps up in order
+//              sixteen warps up in pairs
 // (The form it replaces, one softmax over the split by all warps with ten barriers, took 18-24 us a task, eight of them in the prologue.)
 #pragma once
 #include "kvm_decode_stream.cuh"
@@ -29,6 +29,13 @@ struct KvmPartArgs {
 #define KVM_RA_PS 2048
 #define KVM_RA_ML (KVM_RA_PS + 8192)
 #define KVM_RA_BYTES (KVM_RA_ML + 1024)
+
+// d = rows g (0..7) of A[16 x 16] B[16 x 8], columns 2t and 2t + 1; rows 8 to 15 of A are zero.
+__device__ __forceinline__ void kvm_ra_mma(float (&d)[2], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+  float pad0, pad1;
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(pad0), "=f"(pad1) : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1), "f"(0.0f));
+}
 
 // Rotated row of one head: lane handles the pairs (i, i + HD/2), i = lane, lane + 32, ...  put(column, value).
 template <int HD, class Put>
@@ -111,19 +118,24 @@ __device__ __forceinline__ bool kvm_ra_part(const KvmPartArgs& P, unsigned char*
   const float sc = kvm_bits_f32(P.a[15]);
 #pragma unroll 1
   for (int k0 = warp * 16; k0 < nk; k0 += 256) {
-    float s[2][4];
+    float s[2][2];
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt) {
-      s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.0f;
+      // sixteen products from zero, float32 adds in pairs between them: the matrix unit truncates where it adds to an accumulator, so a
+      // sum kept there over a whole row drifts towards zero (the tile's rows 8 to 15 hold no head)
       const unsigned char* kr = Ks + (size_t)(k0 + nt * 8 + g) * HD * 2 + t * 16;
+      float d[HD / 16][2];
 #pragma unroll
       for (int ch = 0; ch < HD / 32; ++ch) {
         const uint4 kf = *(const uint4*)(kr + ch * 64);
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                     : "+f"(s[nt][0]), "+f"(s[nt][1]), "+f"(s[nt][2]), "+f"(s[nt][3]) : "r"(qf[ch].x), "r"(0u), "r"(qf[ch].y), "r"(0u), "r"(kf.x), "r"(kf.y));
-        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-                     : "+f"(s[nt][0]), "+f"(s[nt][1]), "+f"(s[nt][2]), "+f"(s[nt][3]) : "r"(qf[ch].z), "r"(0u), "r"(qf[ch].w), "r"(0u), "r"(kf.z), "r"(kf.w));
+        kvm_ra_mma(d[2 * ch], qf[ch].x, qf[ch].y, kf.x, kf.y);
+        kvm_ra_mma(d[2 * ch + 1], qf[ch].z, qf[ch].w, kf.z, kf.w);
       }
+#pragma unroll
+      for (int w = 1; w < HD / 16; w *= 2)
+#pragma unroll
+        for (int i = 0; i < HD / 16; i += 2 * w) { d[i][0] += d[i + w][0]; d[i][1] += d[i + w][1]; }
+      s[nt][0] = d[0][0]; s[nt][1] = d[0][1];
     }
     // lane (g, t): scores of head g for the keys k0 + 2t, + 1 and k0 + 8 + 2t, + 1
     float mx = KVM_ATTN_EMPTY_M_STREAM;
@@ -193,11 +205,15 @@ __device__ __forceinline__ bool kvm_ra_part(const KvmPartArgs& P, unsigned char*
   const KvmBuf part = P.lb[4];
   for (int e = threadIdx.x; e < G * HD; e += KVM_NT) {
     const int h = e / HD, cc = e % HD;
-    float A = 0.0f;
+    float A[KVM_NWARPS];
 #pragma unroll
-    for (int w = 0; w < KVM_NWARPS; ++w) A += red[((size_t)w * G + h) * HD + cc];
+    for (int w = 0; w < KVM_NWARPS; ++w) A[w] = red[((size_t)w * G + h) * HD + cc];
+#pragma unroll
+    for (int n = 1; n < KVM_NWARPS; n *= 2)
+#pragma unroll
+      for (int w = 0; w < KVM_NWARPS; w += 2 * n) A[w] += A[w + n];
     float* row = (float*)part.p + ((size_t)(b * P.a[10] + P.a[9]) * P.a[11] + kvh * G + h) * part.ld;
-    row[cc] = A;
+    row[cc] = A[0];
     if (cc == 0) {
       float Mh = KVM_ATTN_EMPTY_M_STREAM, L = 0.0f;
       for (int w = 0; w < KVM_NWARPS; ++w) Mh = fmaxf(Mh, ml[w * 8 + h].x);

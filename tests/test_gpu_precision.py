@@ -69,3 +69,33 @@ def test_attention_scores_do_not_drift(kvm_lib, T, hd):
     ref = (m + np.log(np.exp(s - m).sum(1, keepdims=True)))[:, 0]
     assert abs(lse_bias(ex.read_buffer('lse')[:, 0], ref)) <= 0.5
     ex.close()
+
+
+@pytest.mark.parametrize('hd,G', [(128, 4), (128, 8), (64, 7), (32, 8)])
+def test_split_scores_do_not_drift(kvm_lib, hd, G):
+    # The same for the split decode attention.  Queries are rotated back from positive bf16 values, which the kernel's rotation and
+    # rounding restore exactly.
+    rng = np.random.default_rng(0)
+    n, S, theta, half = 1000, 8, 1e4, hd // 2
+    pos, keys = bf16_round(np.abs(rng.standard_normal((G, hd)) * 3).astype(np.float32)), bf16_round(np.abs(rng.standard_normal((n, hd)) * 3).astype(np.float32))
+    ang = np.float64(n - 1) * np.float32(theta ** (-2.0 * np.arange(half) / hd)).astype(np.float64)
+    a, b = pos[:, :half].astype(np.float64), pos[:, half:].astype(np.float64)
+    q = np.concatenate([a * np.cos(ang) + b * np.sin(ang), b * np.cos(ang) - a * np.sin(ang)], 1).astype(np.float32)
+    g = Graph('part')
+    g.data('q', q.reshape(1, -1)), g.data('kc', keys, 'bf16'), g.data('vc', keys, 'bf16'), g.data('lens', np.array([[n - 1]], np.int32), 'i32'), g.buffer('part', S * G, hd + 2)
+    g.buffer('new', 1, hd)
+    for s in range(S):
+        g.task('attn_decode_part', {'q': 'q', 'kc': 'kc', 'vc': 'vc', 'lens': 'lens', 'part': 'part', 'knew': 'new', 'vnew': 'new', 'b': 0, 'kvh': 0, 's': s, 'S': S, 'H': G, 'Hkv': 1,
+                                    'hd': hd, 'Tmax': n, 'scale': hd ** -0.5, 'theta': theta, 'flags': 3}, ['q'], [('part', (s * G, s * G + G))])
+    g.buffer('w', 8, 256, 'bf16'), g.buffer('x', 1, 256), g.buffer('y', 1, 8)
+    gemv_task(g, 'gemv_bf16', 'x', 'w', 'y', 0, 8, 256)          # a program with a streamed GEMV runs on the static path, its splits from the ring
+    ex = run(g)
+    assert ex.plan_info()[:2] == (True, True)
+    keys[n - 1] = 0                                               # the appended key
+    s = pos.astype(np.float64) @ keys.astype(np.float64).T * np.float64(np.float32(hd ** -0.5))
+    s = s.reshape(G, S, n // S)
+    m = s.max(2)
+    ref = (m + np.log(np.exp(s - m[..., None]).sum(2))).T
+    part = ex.read_buffer('part').reshape(S, G, hd + 2).astype(np.float64)
+    assert abs(lse_bias(part[..., hd] + np.log(part[..., hd + 1]), ref)) <= 0.5
+    ex.close()
