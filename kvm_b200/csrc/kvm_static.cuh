@@ -99,7 +99,7 @@ __device__ __forceinline__ bool kvm_ring_wait_warp(const KvmRing& ring, unsigned
 // transposing reduction (nine shuffles for eight rows).
 // What bounds it: a 64 KB stage is 1.5 us of an SM's share of HBM and about 700 issue cycles here; every value of the loop has to stay
 // in registers, since a spilled one costs an L2 round trip per stage (the stages leave 28 KB of L1 for 512 threads' local memory).
-// Partial sums are added in part order.  Semantics as kvm_op_gemv_bf16 (runtime/ref_extra.py:398-415).  Always consumes its nchunks
+// Partial sums are added in pairs.  Semantics as kvm_op_gemv_bf16 (runtime/ref_extra.py:398-415).  Always consumes its nchunks
 // stage uses, also after an error.
 __device__ __forceinline__ unsigned long long kvm_pack2(float lo, float hi) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
 __device__ __forceinline__ void kvm_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
@@ -190,7 +190,7 @@ __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a,
         for (int i = 0; i < 4; ++i) xs[PACK ? 0 : j][i] = kvm_pack2(t[2 * i], t[2 * i + 1]);
     };
     ok = kvm_gv_args_ok(c, a, lb);
-    if (ok && a[5] >= 0 && tid < rows) rv = kvm_ld(lb[5], a[6] + tid);
+    if (ok && a[5] >= 0 && (lane & 15) == 0 && tid / 16 < rows) rv = kvm_ld(lb[5], a[6] + tid / 16);
     const KvmBuf x = lb[0];
     bool f32 = x.dtype == KVM_F32 && kvm_vec_ok(x);
     const float* up = nullptr;                             // the prologue's second operand: gamma or the up projection
@@ -322,11 +322,16 @@ __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a,
   kvm_sync();
   if (ok && waited) {
     const KvmBuf out = lb[4];
-    for (int i = tid; i < rows; i += KVM_NT) {
-      float sum = 0.0f;
-      for (int p = 0; p < KP; ++p) sum += parts[p * rows + i];
-      if (a[5] >= 0) sum = __fadd_rn(sum, i == tid ? rv : kvm_ld(lb[5], a[6] + i));
-      kvm_st(out, a[6] + i, sum);
+    // sixteen lanes per row (KP of them hold a part), added in pairs
+    for (int base = warp * 2; base < rows; base += 2 * KVM_NWARPS) {
+      const int i = base + (lane >> 4);
+      float sum = i < rows && (lane & 15) < KP ? parts[(lane & 15) * rows + i] : 0.0f;
+#pragma unroll
+      for (int o = 1; o < 16; o *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if ((lane & 15) == 0 && i < rows) {
+        if (a[5] >= 0) sum = __fadd_rn(sum, base == warp * 2 ? rv : kvm_ld(lb[5], a[6] + i));
+        kvm_st(out, a[6] + i, sum);
+      }
     }
   }
 }

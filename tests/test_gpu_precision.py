@@ -99,3 +99,20 @@ def test_split_scores_do_not_drift(kvm_lib, hd, G):
     part = ex.read_buffer('part').reshape(S, G, hd + 2).astype(np.float64)
     assert abs(lse_bias(part[..., hd] + np.log(part[..., hd + 1]), ref)) <= 0.5
     ex.close()
+
+
+def test_gemv_sums_in_pairs(kvm_lib):
+    # Terms of random sign: an addition in which partial sums of all terms meet adds (c * sum)^2 to the error's variance, c = 0.41 * 2^-24
+    # the rms of a rounding relative to the rounded value.  A row of 4096 passes a chain of four products (2.5 such levels on average),
+    # the halves of a packed sum (1), five shuffles and sixteen parts in pairs (4).  Parts one after the other would count 8.5.
+    K, levels = 4096, 2.5 + 1 + 5 + 4
+    rng = np.random.default_rng(1)
+    x, w = bf16_round(rng.standard_normal(K).astype(np.float32)), bf16_round((rng.standard_normal((512, K)) * 0.02).astype(np.float32))
+    g = Graph('gemv')
+    g.data('x', x[None]), g.data('w', w, 'bf16'), g.buffer('o', 1, 512)
+    for n in range(0, 512, 64):
+        gemv_task(g, 'gemv_bf16', 'x', 'w', 'o', n, n + 64, K)
+    ex = run(g)
+    ref = w.astype(np.float64) @ x.astype(np.float64)
+    assert np.linalg.norm(ex.read_buffer('o')[0] - ref) <= 0.41 * 2.0 ** -24 * levels ** 0.5 * np.linalg.norm(ref)
+    ex.close()
