@@ -517,15 +517,21 @@ __device__ __forceinline__ bool kvm_hot_adamw(const KvmCtx& c, const int32_t* a)
 __device__ __forceinline__ bool kvm_hot_gradnorm(const KvmCtx& c, const int32_t* a) {
   KvmBuf g, part;
   const int slot = a[2], e0 = a[3], e1 = a[4];
-  if (!kvm_hot_buf(c, a[0], KVM_F32, g) || !kvm_hot_buf(c, a[1], KVM_F32, part) || slot < 0 || !kvm_hot_range(e0, e1, 4) || !kvm_hot_flat(g, e1) || !kvm_hot_flat(part, slot + 1)) return false;
+  if (!kvm_hot_buf(c, a[0], KVM_F32, g) || !kvm_hot_buf(c, a[1], KVM_F32, part) || slot < 0 || !kvm_hot_range(e0, e1, 8) || !kvm_hot_flat(g, e1) || !kvm_hot_flat(part, slot + 1)) return false;
   double s = 0.0;
   const char* const in[1] = {(const char*)g.p};
   const int eb[1] = {4};
-  kvm_stream<1, 4 * KVM_NT * 4>(c, in, eb, e0, e1, [&](const char* const (&st)[1], int, int n) {
+  kvm_stream<1, 2 * KVM_NT * 8>(c, in, eb, e0, e1, [&](const char* const (&st)[1], int, int n) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = (u * KVM_NT + (int)threadIdx.x) * 4;
-      if (k < n) { const float4 v = *(const float4*)(st[0] + k * 4); s += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w); }
+    for (int u = 0; u < 2; ++u) {                      // eight squares in sequence, as the general body
+      const int k = (u * KVM_NT + (int)threadIdx.x) * 8;
+      if (k < n) {
+        const float4 v = *(const float4*)(st[0] + k * 4), w = *(const float4*)(st[0] + k * 4 + 16);
+        float q = 0.0f;
+        q += v.x * v.x; q += v.y * v.y; q += v.z * v.z; q += v.w * v.w;
+        q += w.x * w.x; q += w.y * w.y; q += w.z * w.z; q += w.w * w.w;
+        s += q;
+      }
     }
   });
   s = kvm_block_sum(s, (double*)c.smem);
