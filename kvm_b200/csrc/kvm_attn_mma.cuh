@@ -5,8 +5,9 @@
 // Products run on mma.sync m16n8k16 (bf16 operands, float32 sums) at float32 precision: a float32 operand is split into three bf16
 // terms of eight bits each and the products of terms whose orders sum to less than three are added (the rest is below 2^-24); a bf16
 // operand is its own single term.  Scores of bf16 inputs are therefore exact products, and the probabilities keep float32 precision.
-// The matrix unit truncates where it adds to the accumulator, so a running sum in it drifts towards zero with every instruction: the
-// terms of sixteen products are added from zero, smallest first, and the running sums are float32 adds.
+// The matrix unit truncates where it adds to the accumulator, so a running sum in it drifts towards zero with every instruction: sixteen
+// products of the leading terms are added from zero, those of all other terms (2^-8 of them) in an accumulator of their own, and the two
+// and the running sums meet in float32 adds.
 //
 // A warp owns sixteen rows of the task's block from the scores to the output (flash form, 32 keys at a time, nothing but operands in
 // shared memory).  Warps left over share the other side: KG groups of warps take every KG-th key tile and are added up at the end in
@@ -100,9 +101,12 @@ __device__ __forceinline__ void kvm_am_scores(float (&s)[4][4], const __nv_bfloa
   const __nv_bfloat16* bp = B + (nb + (lane & 7) + ((lane >> 4) << 3)) * P + ((lane >> 3) & 1) * 8;
 #pragma unroll(HD >= 128 && NT > 1 ? 1 : 2)
   for (int ks = 0; ks < HD / 16; ++ks) {
-    float d[4][4];
+    float d[4][4], lo[NT > 1 ? 4 : 1][4];      // products of the leading terms | of all others
 #pragma unroll
-    for (int n = 0; n < 4; ++n) d[n][0] = d[n][1] = d[n][2] = d[n][3] = 0.0f;
+    for (int n = 0; n < 4; ++n) {
+      d[n][0] = d[n][1] = d[n][2] = d[n][3] = 0.0f;
+      if (NT > 1) lo[NT > 1 ? n : 0][0] = lo[NT > 1 ? n : 0][1] = lo[NT > 1 ? n : 0][2] = lo[NT > 1 ? n : 0][3] = 0.0f;
+    }
 #pragma unroll
     for (int i = NT - 1; i >= 0; --i) {
       uint32_t a[4];
@@ -113,14 +117,14 @@ __device__ __forceinline__ void kvm_am_scores(float (&s)[4][4], const __nv_bfloa
         for (int np = 0; np < 2; ++np) {
           uint32_t b[4];
           kvm_am_ldm4(b, bp + (size_t)j * brows * P + np * 16 * P + ks * 16);
-          kvm_am_mma(d[2 * np], a, b[0], b[1]);
-          kvm_am_mma(d[2 * np + 1], a, b[2], b[3]);
+          if (i + j == 0) { kvm_am_mma(d[2 * np], a, b[0], b[1]); kvm_am_mma(d[2 * np + 1], a, b[2], b[3]); }
+          else { kvm_am_mma(lo[NT > 1 ? 2 * np : 0], a, b[0], b[1]); kvm_am_mma(lo[NT > 1 ? 2 * np + 1 : 0], a, b[2], b[3]); }
         }
     }
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) s[n][e] += d[n][e];
+      for (int e = 0; e < 4; ++e) s[n][e] += NT > 1 ? d[n][e] + lo[NT > 1 ? n : 0][e] : d[n][e];
   }
 }
 // acc[16 x NCOL] += p[16 x 32] times B rows kb.. (32 of them), columns n0..
@@ -139,16 +143,19 @@ __device__ __forceinline__ void kvm_am_accum(float (&acc)[KvmAm<HD>::NCOL / 8][4
     }
 #pragma unroll
     for (int np = 0; np < KvmAm<HD>::NCOL / 16; ++np) {
-      float d[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
+      float d[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}}, lo[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};
 #pragma unroll
       for (int j = NT - 1; j >= 0; --j) {
         uint32_t b[4];
         kvm_am_ldm4t(b, bp + (size_t)j * brows * P + kk * 16 * P + np * 16);
 #pragma unroll
-        for (int i = 2 - j; i >= 0; --i) { kvm_am_mma(d[0], a[i], b[0], b[1]); kvm_am_mma(d[1], a[i], b[2], b[3]); }
+        for (int i = 2 - j; i >= 0; --i) {
+          if (i + j == 0) { kvm_am_mma(d[0], a[i], b[0], b[1]); kvm_am_mma(d[1], a[i], b[2], b[3]); }
+          else { kvm_am_mma(lo[0], a[i], b[0], b[1]); kvm_am_mma(lo[1], a[i], b[2], b[3]); }
+        }
       }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { acc[2 * np][e] += d[0][e]; acc[2 * np + 1][e] += d[1][e]; }
+      for (int e = 0; e < 4; ++e) { acc[2 * np][e] += d[0][e] + lo[0][e]; acc[2 * np + 1][e] += d[1][e] + lo[1][e]; }
     }
   }
 }

@@ -116,3 +116,32 @@ def test_gemv_sums_in_pairs(kvm_lib):
     ref = w.astype(np.float64) @ x.astype(np.float64)
     assert np.linalg.norm(ex.read_buffer('o')[0] - ref) <= 0.41 * 2.0 ** -24 * levels ** 0.5 * np.linalg.norm(ref)
     ex.close()
+
+
+@pytest.mark.parametrize('T,hd', [(200, 32), (257, 64)])
+def test_attention_gradients_do_not_shrink(kvm_lib, T, hd):
+    # dq of float32 inputs: scores, their gradient and the weighted sum of the keys each lose half a unit (2^-25 to 2^-24) of their sum
+    # on average where the products of the leading terms are added; every other addition is rounded to nearest.  Projected on the result
+    # the roundings average out and the losses add up: at most 2^-23.
+    rng = np.random.default_rng(0)
+    q, k, v, do = (rng.standard_normal((T, hd)).astype(np.float32) for _ in range(4))
+    Q, K, V, D = (a.astype(np.float64) for a in (q, k, v, do))
+    sc = np.float64(np.float32(hd ** -0.5))
+    s = Q @ K.T * sc
+    s[np.triu_indices(T, 1)] = -np.inf
+    m = s.max(1, keepdims=True)
+    lse = (m + np.log(np.exp(s - m).sum(1, keepdims=True))).astype(np.float32)
+    delta = ((np.exp(s - lse.astype(np.float64)) @ V) * D).sum(1, keepdims=True).astype(np.float32)
+    dS = np.exp(s - lse.astype(np.float64)) * (D @ V.T - delta.astype(np.float64))
+    g = Graph('attn')
+    for n, a in (('q', q), ('k', k), ('v', v), ('do', do), ('lse', lse), ('delta', delta)):
+        g.data(n, a)
+    g.buffer('dq', T, hd), g.buffer('dk', T, hd), g.buffer('dv', T, hd)
+    for r0 in range(0, T, 128):
+        r1, args = min(r0 + 128, T), {'q': 'q', 'k': 'k', 'v': 'v', 'do': 'do', 'lse': 'lse', 'delta': 'delta', 'b': 0, 'T': T, 'H': 1, 'hd': hd, 'scale': hd ** -0.5}
+        g.task('attn_bwd_dq', {**args, 'dq': 'dq', 'h': 0, 'q0': r0, 'Hkv': 1}, ['q'], [('dq', (r0, r1), (0, hd))])
+        g.task('attn_bwd_dkv', {**args, 'dk': 'dk', 'dv': 'dv', 'kvh': 0, 'k0': r0}, ['q'], [('dk', (r0, r1), (0, hd)), ('dv', (r0, r1), (0, hd))])
+    ex = run(g)
+    for name, ref in (('dq', dS @ K * sc), ('dk', dS.T @ Q * sc)):
+        assert abs(((ex.read_buffer(name) - ref) * ref).sum() / (ref * ref).sum()) <= 2.0 ** -23, name
+    ex.close()
