@@ -165,74 +165,118 @@ __device__ __forceinline__ bool kvm_hot_ln_bwd(const KvmCtx& c, const int32_t* a
 }
 
 // ---- column sums (and the parameter gradients of a norm) -------------------------------------------------------------------------------
-// 64 columns at a time: a thread owns 4 neighbouring columns of every 32nd row, four rows' loads in flight (float32 rows: 16 bytes
-// per thread and row instead of the 4 of one column per thread, which left the loop at 10 KB/us).  Row groups are added in a fixed
-// order through shared memory.
+// 64 columns at a time.  Rows come through shared memory, copied sixteen bytes at a time, 72 to 112 KB in flight (one column per thread straight from global memory left the loop at 10 KB/us); they are added from there by eight row
+// groups of a thread per column, in the general body's order.  Bound by HBM: 8192 rows of 64 columns take 43 us for a column sum of bf16
+// rows and 111 us for the parameter gradients of a norm in the 162M step (94 and 301 in the general body; 55 and 124 with 32 row groups
+// straight from global memory, which summed in another order).
+__device__ __forceinline__ void kvm_cp_async(uint32_t dst, const void* src, int bytes) {      // 16 or 4
+  if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+template <int MODE, bool XB, bool YB> struct KvmColStage {
+  static constexpr int S = MODE == 0 && XB ? 128 : 64, DEPTH = MODE == 0 ? 8 : 4;      // rows of a stage, stages (of 16 KB, 24 or 32 KB for two operands)
+  static constexpr int XR = XB ? 128 : 256, YR = MODE == 0 ? 0 : YB ? 128 : 256;      // bytes of a staged row
+  static constexpr int OFF_Y = S * XR, OFF_M = OFF_Y + S * YR, BYTES = OFF_M + (MODE == 1 ? S * 8 : 0);      // x | dy | mean | rstd
+  static constexpr int SCRATCH = DEPTH * BYTES + KVM_NT * 8;           // and the row groups' sums
+};
 template <int MODE, bool XB, bool YB>
-__device__ __forceinline__ void kvm_hot_colreduce_t(float* red, const KvmBuf& x, const KvmBuf& dy, const float* mean, const float* rstd, float* o1, float* o2, int R, int c0, int c1, int acc) {
-  const int cq = threadIdx.x & 15, rg = threadIdx.x >> 4;
-  constexpr int U = MODE == 0 ? 8 : 4;
+__device__ __forceinline__ bool kvm_hot_colreduce_t(const KvmCtx& c, const KvmBuf& x, const KvmBuf& dy, const float* mean, const float* rstd, float* o1, float* o2, int R, int c0, int c1, int acc) {
+  typedef KvmColStage<MODE, XB, YB> G;
+  if (c.smem_bytes < G::SCRATCH) return false;
+  const int tid = threadIdx.x, col = tid & 63, rg = tid >> 6, ns = (R + G::S - 1) / G::S;
+  const uint32_t base = kvm_smem_addr(c.smem);
+  float* red = (float*)(c.smem + G::DEPTH * G::BYTES);
 #pragma unroll 1
   for (int cb = c0; cb < c1; cb += 64) {
-    const int col = cb + cq * 4;
-    float4 s1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), s2 = s1;
-    if (col < c1) {
-      auto ldx = [&](int r) { return XB ? kvm_bf16x4(*(const uint2*)((const __nv_bfloat16*)x.p + (size_t)r * x.ld + col)) : *(const float4*)((const float*)x.p + (size_t)r * x.ld + col); };
-      auto ldy = [&](int r) { return YB ? kvm_bf16x4(*(const uint2*)((const __nv_bfloat16*)dy.p + (size_t)r * dy.ld + col)) : *(const float4*)((const float*)dy.p + (size_t)r * dy.ld + col); };
-      auto add = [&](float4 xv, float4 gv, float mu, float rs) {
-        if (MODE == 0) { s1.x += xv.x; s1.y += xv.y; s1.z += xv.z; s1.w += xv.w; }
-        else {
-          s1.x += gv.x * (xv.x - mu) * rs; s1.y += gv.y * (xv.y - mu) * rs; s1.z += gv.z * (xv.z - mu) * rs; s1.w += gv.w * (xv.w - mu) * rs;
-          s2.x += gv.x; s2.y += gv.y; s2.z += gv.z; s2.w += gv.w;
+    const int w = min(64, c1 - cb);
+    auto issue = [&](int st) {                         // one group of copies, empty past the last stage
+      if (st < ns) {
+        const int r0 = st * G::S;
+        const uint32_t dst = base + (st & (G::DEPTH - 1)) * G::BYTES;
+#pragma unroll
+        for (int i = tid; i < G::S * G::XR / 16; i += KVM_NT) {
+          const int r = i / (G::XR / 16), k = i % (G::XR / 16) * (XB ? 8 : 4);
+          if (r0 + r < R && k < w) kvm_cp_async(dst + r * G::XR + k * (XB ? 2 : 4), (const char*)x.p + ((size_t)(r0 + r) * x.ld + cb + k) * (XB ? 2 : 4), 16);
         }
-      };
-      int r = rg;
-#pragma unroll 1
-      for (; r + (U - 1) * 32 < R; r += U * 32) {
-        float4 xv[U], gv[MODE == 1 ? U : 1];
-        float mu[MODE == 1 ? U : 1], rs[MODE == 1 ? U : 1];
+        if (MODE == 1)
 #pragma unroll
-        for (int u = 0; u < U; ++u) { xv[u] = ldx(r + u * 32); if (MODE == 1) { gv[u] = ldy(r + u * 32); mu[u] = mean ? mean[r + u * 32] : 0.0f; rs[u] = rstd[r + u * 32]; } }
-#pragma unroll
-        for (int u = 0; u < U; ++u) { if (MODE == 1) add(xv[u], gv[u], mu[u], rs[u]); else add(xv[u], xv[u], 0.0f, 0.0f); }
+          for (int i = tid; i < G::S * G::YR / 16; i += KVM_NT) {
+            const int r = i / (MODE == 1 ? G::YR / 16 : 1), k = i % (MODE == 1 ? G::YR / 16 : 1) * (YB ? 8 : 4);
+            if (r0 + r < R && k < w) kvm_cp_async(dst + G::OFF_Y + r * G::YR + k * (YB ? 2 : 4), (const char*)dy.p + ((size_t)(r0 + r) * dy.ld + cb + k) * (YB ? 2 : 4), 16);
+          }
+        if (MODE == 1 && tid < 2 * G::S && r0 + (tid & (G::S - 1)) < R) kvm_cp_async(dst + G::OFF_M + tid * 4, (tid < G::S ? mean : rstd) + r0 + (tid & (G::S - 1)), 4);
       }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    kvm_sync();                                        // the scratch is free
+#pragma unroll
+    for (int st = 0; st < G::DEPTH - 1; ++st) issue(st);
+    float s1 = 0.0f, s2 = 0.0f;
 #pragma unroll 1
-      for (; r < R; r += 32) { if (MODE == 1) add(ldx(r), ldy(r), mean ? mean[r] : 0.0f, rstd[r]); else { const float4 v = ldx(r); add(v, v, 0.0f, 0.0f); } }
+    for (int st = 0; st < ns; ++st) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(G::DEPTH - 2) : "memory");
+      kvm_sync();                                      // the stage has landed for everyone, and everyone is done with the one before
+      issue(st + G::DEPTH - 1);
+      const unsigned char* sm = c.smem + (st & (G::DEPTH - 1)) * G::BYTES;
+      const int left = R - st * G::S;
+      auto ldx = [&](int r) { return XB ? __bfloat162float(*(const __nv_bfloat16*)(sm + r * G::XR + col * 2)) : *(const float*)(sm + r * G::XR + col * 4); };
+      auto ldy = [&](int r) { return YB ? __bfloat162float(*(const __nv_bfloat16*)(sm + G::OFF_Y + r * G::YR + col * 2)) : *(const float*)(sm + G::OFF_Y + r * G::YR + col * 4); };
+      const float* mu = (const float*)(sm + G::OFF_M);
+      auto add = [&](float xv, float gv, float m, float rs) { if (MODE == 0) s1 += xv; else { s1 += gv * (xv - m) * rs; s2 += gv; } };
+      if (col < w) {
+        if (left >= G::S) {                            // a whole stage: eight rows' values before the first of them is added
+#pragma unroll
+          for (int b = 0; b < G::S; b += 64) {
+            float xv[8], gv[8], mv[8], rv[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              const int r = b + u * 8 + rg;
+              xv[u] = ldx(r);
+              gv[u] = MODE == 1 ? ldy(r) : 0.0f; mv[u] = MODE == 1 ? mu[r] : 0.0f; rv[u] = MODE == 1 ? mu[G::S + r] : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) add(xv[u], gv[u], mv[u], rv[u]);
+          }
+        } else {
+#pragma unroll 1
+          for (int r = rg; r < left; r += 8) add(ldx(r), MODE == 1 ? ldy(r) : 0.0f, MODE == 1 ? mu[r] : 0.0f, MODE == 1 ? mu[G::S + r] : 0.0f);
+        }
+      }
     }
+    red[tid] = s1;
+    if (MODE == 1) red[KVM_NT + tid] = s2;
     kvm_sync();
-    *(float4*)(red + rg * 64 + cq * 4) = s1;
-    if (MODE == 1) *(float4*)(red + 2048 + rg * 64 + cq * 4) = s2;
-    kvm_sync();
-    if (threadIdx.x < (MODE == 1 ? 128 : 64)) {
-      const int k = threadIdx.x & 63, w = threadIdx.x >> 6, cc = cb + k;
+    if (tid < (MODE == 1 ? 128 : 64)) {
+      const int k = tid & 63, m = tid >> 6, cc = cb + k;
       float t = 0.0f;
 #pragma unroll
-      for (int g = 0; g < 32; ++g) t += red[w * 2048 + g * 64 + k];
-      float* o = w ? o2 : o1;
-      if (cc < c1 && o) o[cc] = acc ? __fadd_rn(o[cc], t) : t;
+      for (int g = 0; g < 8; ++g) t += red[m * KVM_NT + g * 64 + k];
+      float* o = m ? o2 : o1;
+      if (cc < c1) o[cc] = acc ? __fadd_rn(o[cc], t) : t;
     }
   }
+  return true;
 }
+// columns [c0, c1) in pieces of sixteen bytes
+__device__ __forceinline__ bool kvm_hot_cols(const KvmBuf& b, int c0, int c1) { return ((c0 | c1 | b.ld) & (b.dtype == KVM_BF16 ? 7 : 3)) == 0; }
 __device__ __forceinline__ bool kvm_hot_colsum(const KvmCtx& c, const int32_t* a) {
   KvmBuf x, out;
   const int R = a[2], c0 = a[3], c1 = a[4];
   if (!kvm_hot_float(c, a[0], x) || !kvm_hot_buf(c, a[1], KVM_F32, out)) return false;
-  if (R < 0 || c0 < 0 || c1 < c0 || ((c0 | c1) & 3) || !kvm_hot_mat(x, R, c1) || !kvm_hot_flat(out, c1)) return false;
+  if (R < 0 || c0 < 0 || c1 < c0 || !kvm_hot_cols(x, c0, c1) || !kvm_hot_mat(x, R, c1) || !kvm_hot_flat(out, c1)) return false;
   KvmBuf none{};
-  if (x.dtype == KVM_BF16) kvm_hot_colreduce_t<0, true, false>((float*)c.smem, x, none, nullptr, nullptr, (float*)out.p, nullptr, R, c0, c1, a[5]);
-  else kvm_hot_colreduce_t<0, false, false>((float*)c.smem, x, none, nullptr, nullptr, (float*)out.p, nullptr, R, c0, c1, a[5]);
-  return true;
+  if (x.dtype == KVM_BF16) return kvm_hot_colreduce_t<0, true, false>(c, x, none, nullptr, nullptr, (float*)out.p, nullptr, R, c0, c1, a[5]);
+  return kvm_hot_colreduce_t<0, false, false>(c, x, none, nullptr, nullptr, (float*)out.p, nullptr, R, c0, c1, a[5]);
 }
 __device__ __forceinline__ bool kvm_hot_norm_params(const KvmCtx& c, const int32_t* a) {
   KvmBuf x, dy, mean, rstd, dg, db;
   const int R = a[6], d = a[7], c0 = a[8], c1 = a[9];
   if (!kvm_hot_buf(c, a[0], KVM_F32, x) || !kvm_hot_float(c, a[1], dy) || !kvm_hot_buf(c, a[2], KVM_F32, mean) || !kvm_hot_buf(c, a[3], KVM_F32, rstd) || !kvm_hot_buf(c, a[4], KVM_F32, dg) ||
       !kvm_hot_buf(c, a[5], KVM_F32, db)) return false;
-  if (R < 0 || c0 < 0 || c1 < c0 || c1 > d || ((c0 | c1) & 3) || !kvm_hot_mat(x, R, d) || !kvm_hot_mat(dy, R, d) || !kvm_hot_flat(mean, R) || !kvm_hot_flat(rstd, R) || !kvm_hot_flat(dg, d) ||
+  if (R < 0 || c0 < 0 || c1 < c0 || c1 > d || !kvm_hot_cols(x, c0, c1) || !kvm_hot_cols(dy, c0, c1) || !kvm_hot_mat(x, R, d) || !kvm_hot_mat(dy, R, d) || !kvm_hot_flat(mean, R) || !kvm_hot_flat(rstd, R) || !kvm_hot_flat(dg, d) ||
       !kvm_hot_flat(db, d)) return false;
-  if (dy.dtype == KVM_BF16) kvm_hot_colreduce_t<1, false, true>((float*)c.smem, x, dy, (const float*)mean.p, (const float*)rstd.p, (float*)dg.p, (float*)db.p, R, c0, c1, a[10]);
-  else kvm_hot_colreduce_t<1, false, false>((float*)c.smem, x, dy, (const float*)mean.p, (const float*)rstd.p, (float*)dg.p, (float*)db.p, R, c0, c1, a[10]);
-  return true;
+  if (dy.dtype == KVM_BF16) return kvm_hot_colreduce_t<1, false, true>(c, x, dy, (const float*)mean.p, (const float*)rstd.p, (float*)dg.p, (float*)db.p, R, c0, c1, a[10]);
+  return kvm_hot_colreduce_t<1, false, false>(c, x, dy, (const float*)mean.p, (const float*)rstd.p, (float*)dg.p, (float*)db.p, R, c0, c1, a[10]);
 }
 
 // ---- attention delta: sum over a head's columns of o * dO -----------------------------------------------------------------------------

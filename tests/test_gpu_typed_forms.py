@@ -37,3 +37,22 @@ def test_gradnorm_partial(kvm_lib, n):
         for slot in (0, 1):
             g.task('gradnorm_partial', {'g': f'g{i}', 'partial': f'p{i}', 'slot': slot, 'e0': 8 * slot, 'e1': n + 8 * slot}, [f'g{i}'], [(f'p{i}', (0, 1), (slot, slot + 1))])
     same_bits(g)
+
+
+# rows around a row group, a stage (64 rows, 128 of a bf16 column sum) and the stages in flight; columns around a block of 64, and too few
+# for a 16-byte piece of bf16
+@pytest.mark.parametrize('R', [1, 7, 9, 63, 65, 128, 129, 513, 1030])
+@pytest.mark.parametrize('D,c0', [(4, 0), (68, 0), (136, 8)])
+def test_column_reductions(kvm_lib, R, D, c0):
+    g = Graph('columns')
+    g.data('x', normal(1, R, D)), g.data('xb', normal(2, R, D), 'bf16'), g.data('dy', normal(3, R, D)), g.data('dyb', normal(4, R, D), 'bf16')
+    g.data('mean', normal(5, R, 1)), g.data('rstd', np.abs(normal(6, R, 1)) + 0.5)
+    for src in ('x', 'xb'):
+        for acc in (0, 1):
+            out = g.data(f'sum.{src}.{acc}', normal(7, 1, D))
+            g.task('colsum', {'x': src, 'out': out, 'R': R, 'c0': c0, 'c1': D, 'acc': acc}, [src], [out])
+    for src, dy in (('x', 'dy'), ('x', 'dyb'), ('xb', 'dy'), ('xb', 'dyb')):
+        for acc in (0, 1):
+            dg, db = g.data(f'dg.{src}.{dy}.{acc}', normal(8, 1, D)), g.data(f'db.{src}.{dy}.{acc}', normal(9, 1, D))
+            g.task('norm_bwd_params', {'x': src, 'dy': dy, 'mean': 'mean', 'rstd': 'rstd', 'dgamma': dg, 'dbeta': db, 'R': R, 'd': D, 'c0': c0, 'c1': D, 'acc': acc}, [src, dy], [dg, db])
+    same_bits(g)
