@@ -271,10 +271,14 @@ __device__ __forceinline__ bool kvm_hot_colsum(const KvmCtx& c, const int32_t* a
 __device__ __forceinline__ bool kvm_hot_norm_params(const KvmCtx& c, const int32_t* a) {
   KvmBuf x, dy, mean, rstd, dg, db;
   const int R = a[6], d = a[7], c0 = a[8], c1 = a[9];
-  if (!kvm_hot_buf(c, a[0], KVM_F32, x) || !kvm_hot_float(c, a[1], dy) || !kvm_hot_buf(c, a[2], KVM_F32, mean) || !kvm_hot_buf(c, a[3], KVM_F32, rstd) || !kvm_hot_buf(c, a[4], KVM_F32, dg) ||
+  if (!kvm_hot_float(c, a[0], x) || !kvm_hot_float(c, a[1], dy) || !kvm_hot_buf(c, a[2], KVM_F32, mean) || !kvm_hot_buf(c, a[3], KVM_F32, rstd) || !kvm_hot_buf(c, a[4], KVM_F32, dg) ||
       !kvm_hot_buf(c, a[5], KVM_F32, db)) return false;
   if (R < 0 || c0 < 0 || c1 < c0 || c1 > d || !kvm_hot_cols(x, c0, c1) || !kvm_hot_cols(dy, c0, c1) || !kvm_hot_mat(x, R, d) || !kvm_hot_mat(dy, R, d) || !kvm_hot_flat(mean, R) || !kvm_hot_flat(rstd, R) || !kvm_hot_flat(dg, d) ||
       !kvm_hot_flat(db, d)) return false;
+  if (x.dtype == KVM_BF16) {
+    if (dy.dtype == KVM_BF16) return kvm_hot_colreduce_t<1, true, true>(c, x, dy, (const float*)mean.p, (const float*)rstd.p, (float*)dg.p, (float*)db.p, R, c0, c1, a[10]);
+    return false;                                  // bf16 x with a float32 gradient: the general body
+  }
   if (dy.dtype == KVM_BF16) return kvm_hot_colreduce_t<1, false, true>(c, x, dy, (const float*)mean.p, (const float*)rstd.p, (float*)dg.p, (float*)db.p, R, c0, c1, a[10]);
   return kvm_hot_colreduce_t<1, false, false>(c, x, dy, (const float*)mean.p, (const float*)rstd.p, (float*)dg.p, (float*)db.p, R, c0, c1, a[10]);
 }
