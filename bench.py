@@ -840,7 +840,7 @@ def run_alone_more(device, pk):
                 e.flat(op, [a], [o], N * F, {'x': a, 'out': o}, f'{op}{r}')
         mem(name, g, 4 * N * F * per)
     # ---- column reductions at the step's granularity (64 columns x all rows per task): bias gradients (colsum of a bf16 [N, F]
-    #      activation gradient) and the norm layers' dgamma / dbeta (x and dy bf16, mean and rstd per row)
+    #      activation gradient) and the norm layers' dgamma / dbeta (x float32, dy bf16, as in the training step; mean and rstd per row)
     from kvm_b200.workloads.graph import Graph
     g = Graph('alone')
     reps = 3
@@ -852,12 +852,12 @@ def run_alone_more(device, pk):
     mem('colsum', g, reps * N * F * 2)
     g = Graph('alone')
     for r in range(reps):
-        x, dy = g.buffer(f'x{r}', N, F, 'bf16', sd(r + 1, 1.0)), g.buffer(f'dy{r}', N, F, 'bf16', sd(r + 11, 1.0))
+        x, dy = g.buffer(f'x{r}', N, F, init=sd(r + 1, 1.0)), g.buffer(f'dy{r}', N, F, 'bf16', sd(r + 11, 1.0))
         mu, rs = g.buffer(f'mu{r}', 1, N, init=sd(r + 21, 1.0)), g.buffer(f'rs{r}', 1, N, init=sd(r + 31, 1.0))
         dg, db = g.buffer(f'dg{r}', 1, F), g.buffer(f'db{r}', 1, F)
         for c0 in range(0, F, cfg.col_chunk):
             g.task('norm_bwd_params', {'x': x, 'dy': dy, 'mean': mu, 'rstd': rs, 'dgamma': dg, 'dbeta': db, 'R': N, 'd': F, 'c0': c0, 'c1': min(c0 + cfg.col_chunk, F), 'acc': 0})
-    mem('norm_bwd_params', g, reps * N * F * 4)
+    mem('norm_bwd_params', g, reps * N * F * 6)
     return out
 
 
