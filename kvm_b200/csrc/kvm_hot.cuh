@@ -484,45 +484,29 @@ __device__ __forceinline__ void kvm_stream(const KvmCtx& c, const char* const (&
 }
 __device__ __forceinline__ bool kvm_hot_range(int e0, int e1, int align) { return e0 >= 0 && e1 > e0 && ((e0 | e1) & (align - 1)) == 0; }
 
-// Elementwise map over inputs of one storage type: 8 KB of each input per stage, 16 bytes per thread.
-template <int NI, bool B, class F>
-__device__ __forceinline__ void kvm_hot_map_t(const KvmCtx& c, const char* const (&in)[NI], void* out, int e0, int e1, F f) {
-  constexpr int E = B ? 8 : 4;
-  int eb[NI];
-#pragma unroll
-  for (int n = 0; n < NI; ++n) eb[n] = B ? 2 : 4;
-  kvm_stream<NI, KVM_NT * E>(c, in, eb, e0, e1, [&](const char* const (&part)[NI], int i, int n) {
-    const int k = (int)threadIdx.x * E;
-    if (k >= n) return;
-    uint4 x[NI], w;
-#pragma unroll
-    for (int m = 0; m < NI; ++m) x[m] = *(const uint4*)(part[m] + k * (B ? 2 : 4));
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float lo[NI], hi[NI];
-#pragma unroll
-      for (int m = 0; m < NI; ++m) {
-        const uint32_t u = j == 0 ? x[m].x : j == 1 ? x[m].y : j == 2 ? x[m].z : x[m].w;
-        lo[m] = B ? __uint_as_float(u << 16) : __uint_as_float(u);
-        hi[m] = __uint_as_float(u & 0xffff0000u);
-      }
-      if (B) ((__nv_bfloat162*)&w)[j] = __floats2bfloat162_rn(f(lo), f(hi));
-      else ((uint32_t*)&w)[j] = __float_as_uint(f(lo));
-    }
-    *(uint4*)((char*)out + (size_t)(i + k) * (B ? 2 : 4)) = w;
-  });
-}
-// Two inputs and an output of one storage type (or one input: `second` < 0).
-template <int NI, bool B, class F>
-__device__ __forceinline__ bool kvm_hot_map(const KvmCtx& c, int i0, int i1, int o, int e0, int e1, F f) {
+// Elementwise map of two inputs and an output of one storage type: 8 KB of each input per stage, 16 bytes per thread.  The output may be one
+// of the inputs: an element is written after its stage has landed, by the thread that reads it, and later stages are other elements.
+template <bool B, class F>
+__device__ __forceinline__ bool kvm_hot_map2(const KvmCtx& c, int i0, int i1, int o, int e0, int e1, F f) {
+  constexpr int E = B ? 8 : 4, EB = B ? 2 : 4;
   KvmBuf x, y, z;
   const int dt = B ? KVM_BF16 : KVM_F32;
-  if (!kvm_hot_range(e0, e1, B ? 8 : 4) || !kvm_hot_buf(c, i0, dt, x) || (NI == 2 && !kvm_hot_buf(c, i1, dt, y)) || !kvm_hot_buf(c, o, dt, z) || !kvm_hot_flat(x, e1) ||
-      (NI == 2 && !kvm_hot_flat(y, e1)) || !kvm_hot_flat(z, e1)) return false;
-  const char* in[NI];
-  in[0] = (const char*)x.p;
-  if (NI == 2) in[NI - 1] = (const char*)y.p;
-  kvm_hot_map_t<NI, B>(c, in, z.p, e0, e1, f);
+  if (!kvm_hot_range(e0, e1, E) || !kvm_hot_buf(c, i0, dt, x) || !kvm_hot_buf(c, i1, dt, y) || !kvm_hot_buf(c, o, dt, z) || !kvm_hot_flat(x, e1) || !kvm_hot_flat(y, e1) || !kvm_hot_flat(z, e1)) return false;
+  const char* const in[2] = {(const char*)x.p, (const char*)y.p};
+  const int eb[2] = {EB, EB};
+  kvm_stream<2, KVM_NT * E>(c, in, eb, e0, e1, [&](const char* const (&part)[2], int i, int n) {
+    const int k = (int)threadIdx.x * E;
+    if (k >= n) return;
+    const uint4 u = *(const uint4*)(part[0] + k * EB), v = *(const uint4*)(part[1] + k * EB);
+    const uint32_t p[4] = {u.x, u.y, u.z, u.w}, q[4] = {v.x, v.y, v.z, v.w};
+    uint4 w;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (B) ((__nv_bfloat162*)&w)[j] = __floats2bfloat162_rn(f(__uint_as_float(p[j] << 16), __uint_as_float(q[j] << 16)), f(__uint_as_float(p[j] & 0xffff0000u), __uint_as_float(q[j] & 0xffff0000u)));
+      else ((uint32_t*)&w)[j] = __float_as_uint(f(__uint_as_float(p[j]), __uint_as_float(q[j])));
+    }
+    *(uint4*)((char*)z.p + (size_t)(i + k) * EB) = w;
+  });
   return true;
 }
 // f32 -> bf16
@@ -594,7 +578,8 @@ __device__ __forceinline__ bool kvm_hot(const KvmCtx& c, int op, const int32_t* 
     case 35: return kvm_hot_ln_fwd(c, a);
     case 37: return kvm_hot_ln_bwd(c, a);
     case 39: return kvm_hot_norm_params(c, a);
-    case 41: return !a[5] && kvm_hot_map<2, true>(c, a[0], a[1], a[2], a[3], a[4], [](const float (&v)[2]) { return __fmul_rn(v[1], kvm_gelu_grad(v[0])); });
+    case 41: return !a[5] && kvm_hot_map2<true>(c, a[0], a[1], a[2], a[3], a[4], [](float x, float dy) { return __fmul_rn(dy, kvm_gelu_grad(x)); });
+    case 42: return kvm_hot_map2<false>(c, a[0], a[1], a[2], a[3], a[4], [](float x, float y) { return __fadd_rn(x, y); });
     case 46: return kvm_hot_delta(c, a);
     case 54: return kvm_hot_adamw(c, a);
     case 55: return kvm_hot_gradnorm(c, a);

@@ -56,3 +56,22 @@ def test_column_reductions(kvm_lib, R, D, c0):
             dg, db = g.data(f'dg.{src}.{dy}.{acc}', normal(8, 1, D)), g.data(f'db.{src}.{dy}.{acc}', normal(9, 1, D))
             g.task('norm_bwd_params', {'x': src, 'dy': dy, 'mean': 'mean', 'rstd': 'rstd', 'dgamma': dg, 'dbeta': db, 'R': R, 'd': D, 'c0': c0, 'c1': D, 'acc': acc}, [src, dy], [dg, db])
     same_bits(g)
+
+
+# a stage is 2048 float32 or 4096 bf16 elements, four of them in flight; ranges that end inside a stage or start off its grid, outputs in
+# place, and ranges that are no multiple of the typed forms' pieces
+@pytest.mark.parametrize('e0,e1', [(0, 8), (8, 4104), (0, 4096), (16, 16408), (0, 40960), (4, 5000), (3, 4099)])
+def test_elementwise(kvm_lib, e0, e1):
+    n = -(-e1 // 8) * 8
+    g = Graph('elementwise')
+    for dt in ('f32', 'bf16'):
+        for place in ('new', 'first', 'second'):
+            a, b = g.data(f'a.{dt}.{place}', normal(1, 1, n), dt), g.data(f'b.{dt}.{place}', normal(2, 1, n), dt)
+            for op, args in (('residual_add', {'a': a, 'b': b}), ('gelu_bwd', {'x': a, 'dy': b})):
+                src = {k: g.data(f'{v}.{op}', normal(3 + i, 1, n), dt) for i, (k, v) in enumerate(args.items())}
+                out = g.buffer(f'out.{dt}.{place}.{op}', 1, n, dt) if place == 'new' else list(src.values())[place == 'second']
+                extra = {'out': out} if op == 'residual_add' else {'dx': out, 'acc': 0}
+                g.task(op, {**src, **extra, 'e0': e0, 'e1': e1}, list(src.values()), [out])
+    x, o = g.data('x', normal(5, 1, n)), g.buffer('rounded', 1, n, 'bf16')
+    g.task('round_bf16', {'x': x, 'out': o, 'e0': e0, 'e1': e1}, [x], [o])
+    same_bits(g)
