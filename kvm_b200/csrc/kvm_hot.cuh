@@ -571,21 +571,22 @@ __device__ __forceinline__ bool kvm_hot_gradnorm(const KvmCtx& c, const int32_t*
   return true;
 }
 
-// The typed form of op `op`, if there is one for these buffers.  BIG: programs with long rows (the ready-queue kernel).
-template <bool BIG>
-__device__ __forceinline__ bool kvm_hot(const KvmCtx& c, int op, const int32_t* a) {
+// The inlined form of op `op`, if there is one for this task: tcgen05 attention where the host planned it, a typed form where the buffers
+// allow it.
+__device__ __forceinline__ bool kvm_hot(const KvmCtx& c, int op, const int32_t* a, const int4& aux) {
   switch (op) {
     case 35: return kvm_hot_ln_fwd(c, a);
     case 37: return kvm_hot_ln_bwd(c, a);
     case 39: return kvm_hot_norm_params(c, a);
     case 41: return !a[5] && kvm_hot_map2<true>(c, a[0], a[1], a[2], a[3], a[4], [](float x, float dy) { return __fmul_rn(dy, kvm_gelu_grad(x)); });
     case 42: return kvm_hot_map2<false>(c, a[0], a[1], a[2], a[3], a[4], [](float x, float y) { return __fadd_rn(x, y); });
+    case 45: case 47: case 48: return kvm_attn_tc(c, op, a, aux);
     case 46: return kvm_hot_delta(c, a);
     case 54: return kvm_hot_adamw(c, a);
     case 55: return kvm_hot_gradnorm(c, a);
     case 61: return kvm_hot_colsum(c, a);
     case 113: return kvm_hot_round_bf16(c, a);
-    case 127: return BIG && kvm_hot_ce_fused(c, a);
+    case 127: return kvm_hot_ce_fused(c, a);
     default: return false;
   }
 }

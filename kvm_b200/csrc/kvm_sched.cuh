@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(KVM_EXEC_THREADS, 1) kvm_exec_kernel(KvmDevSta
       const int op = sl.desc[0];
       const bool tile = sl.kind == 1;
       if (tile) { if (go == 1) kvm_tce_tile(c, sl.args); ++tiles; }
-      else if (op != 0 && go == 1 && !kvm_attn_tc(c, op, sl.args, sl.aux) && !kvm_hot<true>(c, op, sl.args)) kvm_dispatch(c, op, sl.args, sl.aux);
+      else if (op != 0 && go == 1 && !kvm_hot(c, op, sl.args, sl.aux)) kvm_dispatch(c, op, sl.args, sl.aux);
       // this task's generic-proxy writes (global results, shared scratch) ordered before any later TMA access to them
       asm volatile("fence.proxy.async;" ::: "memory");
       kvm_sync();                       // every thread's writes happen before thread 0's fence below (barrier, then a cumulative gpu-scope fence)

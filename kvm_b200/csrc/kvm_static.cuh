@@ -494,7 +494,7 @@ KVM_OP_FN void kvm_gemv_mma_ring_t(const KvmCtx& c, const int32_t* a, const KvmB
   if (ok && !staged && pro == 1) kvm_stage_rms(sx);
   if (ok && !staged && L.full_x) kvm_stage_rows(sx, 0, K);
   kvm_sync();
-  unsigned long long t_pro = 0, t_wait = 0, t_first = 0;
+  unsigned long long t_pro = 0, t_wait = 0;
   if (stamp && tid == 0) t_pro = kvm_globaltimer();
   bool waited = true;
   const int npairs = KC / 64;
@@ -503,7 +503,7 @@ KVM_OP_FN void kvm_gemv_mma_ring_t(const KvmCtx& c, const int32_t* a, const KvmB
     unsigned long long tw = 0;
     if (stamp && tid == 0) tw = kvm_globaltimer();
     if (waited && !kvm_ring_wait_warp(ring, it, deadline, c.err)) waited = false;
-    if (stamp && tid == 0) { const unsigned long long d = kvm_globaltimer() - tw; t_wait += d; if (it == cit) t_first = d; }
+    if (stamp && tid == 0) t_wait += kvm_globaltimer() - tw;
     if (!waited) return;                                   // warp-uniform; the warp still takes part in every barrier of the task
     if (ok) {
       const unsigned char* wrow = kvm_ring_stage(ring, it) + (size_t)g * KC * 2 + t * 16;
@@ -558,7 +558,6 @@ KVM_OP_FN void kvm_gemv_mma_ring_t(const KvmCtx& c, const int32_t* a, const KvmB
   }
   __syncwarp();
   if (stamp && tid == 0) {      // trace detail, one byte each in units of 0.2 us: prologue | stage loop (waits included) | waits for stages
-    (void)t_first;
     stamp[0] = (int)min(255ull, (t_pro - t_task) / 200) | ((int)min(255ull, (kvm_globaltimer() - t_pro) / 200) << 8) | ((int)min(255ull, t_wait / 200) << 16);
   }
   if (!waited && *(volatile int*)&c.err->code == 0) kvm_stream_timeout(c, 1301);
