@@ -736,7 +736,7 @@ static __device__ void kvm_argmax_rows(const KvmCtx& c, const KvmBuf& lg, const 
 #pragma unroll 4
     for (int k = k0 + threadIdx.x; k < V; k += KVM_NT) {
       float v = kvm_ld(lg, (size_t)r * lg.ld + k);
-      if (v > bv || (v == bv && k < bi)) { bv = v; bi = k; }
+      if (v > bv) { bv = v; bi = k; }              // a thread's columns ascend; -inf never wins, a row of nothing else gives column 0
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) {

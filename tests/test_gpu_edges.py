@@ -46,3 +46,19 @@ def test_decode_streams_odd_widths(kvm_lib, widths, qk_norm):
         for name in ('u0.logits', 'u0.l1.x2'):
             ref = vm.buffer(name).a
             assert np.abs(ex.read_buffer(name) - ref).max() <= 1e-2 * np.abs(ref).max(), name
+
+
+# rows of masked logits: all columns -inf, NaN before them, and a single finite value, around the 8192 columns that a pass in pieces takes
+@pytest.mark.parametrize('V', [8191, 8192, 8200, 16390])
+def test_argmax_of_masked_rows(kvm_lib, V):
+    from kvm_b200.workloads.graph import Graph
+    rows = np.full((4, V), -np.inf, np.float32)
+    rows[1, :100] = np.nan
+    rows[2, V - 1] = 0.0
+    rows[3, [5000, V - 2]] = 1.0
+    g = Graph('argmax')
+    g.data('l', rows), g.buffer('t', 4, 1, 'i32')
+    g.task('argmax', {'logits': 'l', 'out': 't', 'r0': 0, 'r1': 4, 'V': V}, ['l'], ['t'])
+    ex, vm, res = run_both(g.to_bundle())
+    assert ex.read_buffer('t').ravel().tolist() == [0, 0, V - 1, 5000] == vm.buffer('t').a.ravel().tolist()
+    ex.close()
