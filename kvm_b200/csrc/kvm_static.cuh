@@ -24,6 +24,7 @@
 
 #define KVM_ST_SLOTS 4                 // record ring depth (tasks fetched ahead)
 #define KVM_ST_HDR 3072                // header bytes: slots, control words, barriers
+#define KVM_ST_WAITED 4                // stamp[0] end of the prologue, [1] of the stage loop, [2] start of the task, [4] waits for stages so far (ns)
 #define KVM_ST_ARRIVALS 16             // arrivals that free a stage: every compute warp, once it is done with the stage (or has nothing to do with it)
 
 struct KvmStSlot {
@@ -170,7 +171,7 @@ __device__ __forceinline__ bool kvm_gv_args_ok(const KvmCtx& c, const int32_t* a
   return ok;
 }
 
-template <int J>
+template <int J, bool TR>      // TR: notes its times in `stamp` (KVM_ST_WAITED)
 __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing ring, unsigned cit, int R, int NC, int* stamp) {
   const int K = a[8], rows = a[7] - a[6], KP = kvm_gv_parts(K);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = warp & (KP - 1), rg = warp / KP, m = R * KP / KVM_NWARPS;      // rows rg*m .. of a stage
@@ -275,12 +276,14 @@ __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a,
       }
     }
   }
-  if (stamp && tid == 0) stamp[0] = (int)kvm_globaltimer();
+  if (TR && tid == 0) stamp[0] = (int)kvm_globaltimer();
   bool waited = true;
   constexpr int RB = J <= 1 ? 4 : 1;          // rows whose loads are in flight together
 #pragma unroll 1
   for (int ci = 0; ci < NC; ++ci) {
+    const int t0 = TR ? (int)kvm_globaltimer() : 0;
     if (!kvm_ring_wait_warp(ring, cit + ci, c.deadline, c.err)) { waited = false; break; }      // warp-uniform
+    if (TR && tid == 0) stamp[KVM_ST_WAITED] += (int)kvm_globaltimer() - t0;
     const unsigned char* st = kvm_ring_stage(ring, cit + ci) + (size_t)(rg * m) * (K * 2);
     const int left = min(m, rows - ci * R - rg * m);
     float s[8];
@@ -318,7 +321,7 @@ __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a,
     if ((lane & 3) == 0 && (lane >> 2) < left) parts[part * rows + ci * R + rg * m + (lane >> 2)] = t;
   }
   if (!waited && *(volatile int*)&c.err->code == 0) kvm_stream_timeout(c, 1134);
-  if (stamp && tid == 0) stamp[1] = (int)kvm_globaltimer();
+  if (TR && tid == 0) stamp[1] = (int)kvm_globaltimer();
   kvm_sync();
   if (ok && waited) {
     const KvmBuf out = lb[4];
@@ -336,7 +339,17 @@ __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a,
   }
 }
 // rows of more than 12288 columns (their staging bounds them to 16 Ki): the activations beside the loop do not fit the kernel's registers, a function of its own
-KVM_OP_FN void kvm_gemv_ring_wide(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing ring, unsigned cit, int R, int NC) { kvm_gemv_ring<4>(c, a, lb, ring, cit, R, NC, nullptr); }
+KVM_OP_FN void kvm_gemv_ring_wide(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing ring, unsigned cit, int R, int NC) { kvm_gemv_ring<4, false>(c, a, lb, ring, cit, R, NC, nullptr); }
+// Pieces of eight columns per thread.
+__device__ __forceinline__ int kvm_gv_pieces(int K) { return (K + 256 * kvm_gv_parts(K) - 1) / (256 * kvm_gv_parts(K)); }
+// A traced task: a copy of its own, called, so that tracing costs an untraced program nothing (tests of a switch inside the loops cost
+// three users' decode step 1.83 -> 1.88 ms, a small model's 0.59 -> 0.62).
+KVM_OP_FN void kvm_gemv_ring_traced(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing ring, unsigned cit, int R, int NC, int* stamp) {
+  const int J = kvm_gv_pieces(a[8]);
+  if (J == 1) kvm_gemv_ring<1, true>(c, a, lb, ring, cit, R, NC, stamp);
+  else if (J <= 3) kvm_gemv_ring<3, true>(c, a, lb, ring, cit, R, NC, stamp);
+  else kvm_gemv_ring<4, true>(c, a, lb, ring, cit, R, NC, stamp);
+}
 
 // ---- streamed GEMV on tensor cores (gemv_bf16 with one activation row, gemv_bf16_rows with up to eight), consumer side --------------
 // D[16 x 8] += A[16 x 16] B[16 x 8] (mma.sync m16n8k16, bf16 operands, float32 accumulate) with A = activations (rows = activation
@@ -470,8 +483,7 @@ KVM_OP_FN void kvm_stage_rows(const KvmStageX& s, int kb, int kn) {
   }
 }
 template <bool CHUNKED>      // the k-chunk layout (accumulators of eight row groups live over the task) or the whole-row layout, a function each
-KVM_OP_FN void kvm_gemv_mma_ring_t(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool has_rows, const KvmRing ring, unsigned cit, unsigned long long deadline,
-                                   unsigned long long t_task, int* stamp) {
+KVM_OP_FN void kvm_gemv_mma_ring_t(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool has_rows, const KvmRing ring, unsigned cit, int* stamp) {
   KvmBuf x, x2, gm, w, out, res;
   const int n0 = a[6], n1 = a[7], K = a[8], pro = a[9], r0 = has_rows ? a[11] : 0, r1 = has_rows ? a[12] : 1;
   const float eps = kvm_bits_f32(a[10]);
@@ -494,16 +506,14 @@ KVM_OP_FN void kvm_gemv_mma_ring_t(const KvmCtx& c, const int32_t* a, const KvmB
   if (ok && !staged && pro == 1) kvm_stage_rms(sx);
   if (ok && !staged && L.full_x) kvm_stage_rows(sx, 0, K);
   kvm_sync();
-  unsigned long long t_pro = 0, t_wait = 0;
-  if (stamp && tid == 0) t_pro = kvm_globaltimer();
+  if (stamp && tid == 0) stamp[0] = (int)kvm_globaltimer();
   bool waited = true;
   const int npairs = KC / 64;
   // one stage use: wait for it, multiply it into acc (x columns from xk0 of the staged rows), release it
   auto consume = [&](unsigned it, float (&acc)[4], int xk0) {
-    unsigned long long tw = 0;
-    if (stamp && tid == 0) tw = kvm_globaltimer();
-    if (waited && !kvm_ring_wait_warp(ring, it, deadline, c.err)) waited = false;
-    if (stamp && tid == 0) t_wait += kvm_globaltimer() - tw;
+    const int t0 = stamp && tid == 0 ? (int)kvm_globaltimer() : 0;
+    if (waited && !kvm_ring_wait_warp(ring, it, c.deadline, c.err)) waited = false;
+    if (stamp && tid == 0) stamp[KVM_ST_WAITED] += (int)kvm_globaltimer() - t0;
     if (!waited) return;                                   // warp-uniform; the warp still takes part in every barrier of the task
     if (ok) {
       const unsigned char* wrow = kvm_ring_stage(ring, it) + (size_t)g * KC * 2 + t * 16;
@@ -557,9 +567,7 @@ KVM_OP_FN void kvm_gemv_mma_ring_t(const KvmCtx& c, const int32_t* a, const KvmB
     for (int rg = 0; rg < 8; ++rg) if (rg < ng) put_parts(rg, acc[rg]);
   }
   __syncwarp();
-  if (stamp && tid == 0) {      // trace detail, one byte each in units of 0.2 us: prologue | stage loop (waits included) | waits for stages
-    stamp[0] = (int)min(255ull, (t_pro - t_task) / 200) | ((int)min(255ull, (kvm_globaltimer() - t_pro) / 200) << 8) | ((int)min(255ull, t_wait / 200) << 16);
-  }
+  if (stamp && tid == 0) stamp[1] = (int)kvm_globaltimer();
   if (!waited && *(volatile int*)&c.err->code == 0) kvm_stream_timeout(c, 1301);
   kvm_sync();
   if (ok && *(volatile int*)&c.err->code == 0)            // a warp that gave up has recorded the timeout before the barrier
@@ -574,17 +582,16 @@ KVM_OP_FN void kvm_gemv_mma_ring_t(const KvmCtx& c, const int32_t* a, const KvmB
     }
 }
 
-__device__ __forceinline__ void kvm_gemv_mma_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool has_rows, const KvmRing ring, unsigned cit, int nkc,
-                                                  unsigned long long deadline, unsigned long long t_task, int* stamp) {
-  if (nkc > 1) kvm_gemv_mma_ring_t<true>(c, a, lb, has_rows, ring, cit, deadline, t_task, stamp);
-  else kvm_gemv_mma_ring_t<false>(c, a, lb, has_rows, ring, cit, deadline, t_task, stamp);
+__device__ __forceinline__ void kvm_gemv_mma_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool has_rows, const KvmRing ring, unsigned cit, int nkc, int* stamp) {
+  if (nkc > 1) kvm_gemv_mma_ring_t<true>(c, a, lb, has_rows, ring, cit, stamp);
+  else kvm_gemv_mma_ring_t<false>(c, a, lb, has_rows, ring, cit, stamp);
 }
 
 // ---- streamed split attention, consumer side (kvm_ring_attn.cuh) --------------------------------------------------------------------
 // Stage use `cit` holds the split's keys, `cit + 1` its values (the appended row left out).  The front warp has validated the geometry
 // of the caches before it issued the copies; the other arguments are checked here.
-template <int HD, int GT>      // head dimension, query heads per key head at most
-KVM_OP_FN void kvm_attn_part_ring_t(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool qkn, const KvmRing ring, unsigned cit, int j0, int j1, int newrow) {
+template <int HD, int GT, bool TR>      // head dimension, query heads per key head at most, traced
+KVM_OP_FN void kvm_attn_part_ring_t(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool qkn, const KvmRing ring, unsigned cit, int j0, int j1, int newrow, int* stamp) {
   KvmPartArgs P;
   const int bb = a[7], S = a[10], H = a[11], Hkv = a[12], hd = a[13];
   bool ok;
@@ -604,8 +611,17 @@ KVM_OP_FN void kvm_attn_part_ring_t(const KvmCtx& c, const int32_t* a, const Kvm
   unsigned char* Ks = kvm_ring_stage(ring, cit);
   unsigned char* Vs = kvm_ring_stage(ring, cit + 1);
   bool waited = true;
-  auto wk = [&]() { return kvm_ring_wait_warp(ring, cit, c.deadline, c.err); };
-  auto wv = [&]() { return kvm_ring_wait_warp(ring, cit + 1, c.deadline, c.err); };
+  auto wait = [&](unsigned it) {
+    const int t0 = TR ? (int)kvm_globaltimer() : 0;
+    const bool landed = kvm_ring_wait_warp(ring, it, c.deadline, c.err);
+    if (TR && threadIdx.x == 0) {
+      if (it == cit) stamp[0] = t0;                        // the prologue ends where the wait for the keys begins
+      stamp[KVM_ST_WAITED] += (int)kvm_globaltimer() - t0;
+    }
+    return landed;
+  };
+  auto wk = [&]() { return wait(cit); };
+  auto wv = [&]() { return wait(cit + 1); };
   if (ok) {
     // theta^(-2i/hd) is a double-precision pow per frequency: computed once per (theta, head dimension) and launch, not per task
     float* rc = c.rope_cache;
@@ -626,12 +642,17 @@ KVM_OP_FN void kvm_attn_part_ring_t(const KvmCtx& c, const int32_t* a, const Kvm
   if (waited && (threadIdx.x & 31) == 0) { kvm_mbar_arrive(kvm_ring_empty(ring, cit)); kvm_mbar_arrive(kvm_ring_empty(ring, cit + 1)); }
 }
 
-__device__ __forceinline__ void kvm_attn_part_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool qkn, const KvmRing ring, unsigned cit, int j0, int j1, int newrow) {
+template <bool TR>
+__device__ __forceinline__ void kvm_attn_part_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool qkn, const KvmRing ring, unsigned cit, int j0, int j1, int newrow, int* stamp) {
   const int hd = a[13];
   const bool few = a[11] <= 4 * a[12];
-  if (hd == 128) { if (few) kvm_attn_part_ring_t<128, 4>(c, a, lb, qkn, ring, cit, j0, j1, newrow); else kvm_attn_part_ring_t<128, 8>(c, a, lb, qkn, ring, cit, j0, j1, newrow); }
-  else if (hd == 64) { if (few) kvm_attn_part_ring_t<64, 4>(c, a, lb, qkn, ring, cit, j0, j1, newrow); else kvm_attn_part_ring_t<64, 8>(c, a, lb, qkn, ring, cit, j0, j1, newrow); }
-  else kvm_attn_part_ring_t<32, 8>(c, a, lb, qkn, ring, cit, j0, j1, newrow);
+  if (hd == 128) { if (few) kvm_attn_part_ring_t<128, 4, TR>(c, a, lb, qkn, ring, cit, j0, j1, newrow, stamp); else kvm_attn_part_ring_t<128, 8, TR>(c, a, lb, qkn, ring, cit, j0, j1, newrow, stamp); }
+  else if (hd == 64) { if (few) kvm_attn_part_ring_t<64, 4, TR>(c, a, lb, qkn, ring, cit, j0, j1, newrow, stamp); else kvm_attn_part_ring_t<64, 8, TR>(c, a, lb, qkn, ring, cit, j0, j1, newrow, stamp); }
+  else kvm_attn_part_ring_t<32, 8, TR>(c, a, lb, qkn, ring, cit, j0, j1, newrow, stamp);
+}
+// Traced splits: called from a function of their own, so that the kernel's task loop does not grow by them.
+KVM_OP_FN void kvm_attn_part_ring_traced(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool qkn, const KvmRing ring, unsigned cit, int j0, int j1, int newrow, int* stamp) {
+  kvm_attn_part_ring<true>(c, a, lb, qkn, ring, cit, j0, j1, newrow, stamp);
 }
 
 // ---- front warp: stream geometry of a fetched task (lane 0) ---------------------------------------------------------------------
@@ -710,7 +731,7 @@ __global__ void __launch_bounds__(KVM_ST_THREADS, 1) kvm_static_kernel(KvmStatic
   const KvmDevState& S = T.D;
   KvmStSlot* slots = (KvmStSlot*)kvm_smem;
   int* ctl = (int*)(kvm_smem + KVM_ST_SLOTS * sizeof(KvmStSlot));          // as in the dynamic kernel: ctl[0] = TMEM base, tensor-core barriers from ctl[8]
-  int* sctl = ctl + 96;                                                     // static path's own words: [0] consumer stage-use count, [1] tasks finished, [2] producer stage-use count, [3..5] trace, [6] leave
+  int* sctl = ctl + 96;                                                     // static path's own words: [0] consumer stage-use count, [1] tasks finished, [2] producer stage-use count, [3..5] and [7] trace, [6] leave
   const uint32_t sbar = kvm_smem_addr(kvm_smem + KVM_ST_HDR - 128);         // stream ring barriers: full[3] | empty[3]
   const int tid = threadIdx.x;
   const int w = blockIdx.x;
@@ -887,14 +908,14 @@ __global__ void __launch_bounds__(KVM_ST_THREADS, 1) kvm_static_kernel(KvmStatic
       c.smem_bytes = (int)dyn - used - (use_ring ? ring_bytes : 0);
     }
     unsigned cit = 0;
-    int finished = 0;
-    for (int i = 0; i < n; ++i) {
+    int i = 0;
+    for (; i < n; ++i) {
       KvmStSlot& sl = slots[i % KVM_ST_SLOTS];
       if (tid == 0) {
         unsigned polls = 0;
         int st;
         while ((st = kvm_ld_volatile_shared(&sl.state)) < 2) {
-          if ((++polls & 1023u) == 0 && kvm_globaltimer() > deadline + S.timeout_ns) { st = 3; break; }      // the front warp always answers first
+          if ((++polls & 1023u) == 0 && kvm_globaltimer() > c.deadline + 2 * S.timeout_ns) { st = 3; break; }      // the front warp always answers first
         }
         sl.go = st == 3 ? 0 : (*(volatile int*)&S.err->code == 0 ? 1 : 2);
         c.task = sl.task;
@@ -903,17 +924,20 @@ __global__ void __launch_bounds__(KVM_ST_THREADS, 1) kvm_static_kernel(KvmStatic
       const int go = kvm_ld_volatile_shared(&sl.go);
       if (go == 0) break;
       const int task = sl.task;
-      unsigned long long t_task = 0;
-      if (tid == 0 && S.trace) { t_task = kvm_globaltimer(); S.t_start[task] = t_task; sctl[3] = sctl[4] = 0; sctl[5] = (int)t_task; }
+      if (tid == 0 && S.trace) { const unsigned long long t_task = kvm_globaltimer(); S.t_start[task] = t_task; sctl[3] = sctl[4] = sctl[3 + KVM_ST_WAITED] = 0; sctl[5] = (int)t_task; }
       const int op = sl.desc[0], kind = sl.kind, nch = sl.nchunks;
       if (kind == 1) {
-        const int J = (sl.args[8] + 256 * kvm_gv_parts(sl.args[8]) - 1) / (256 * kvm_gv_parts(sl.args[8]));      // pieces of eight columns per thread
-        if (J == 1) kvm_gemv_ring<1>(c, sl.args, sl.lb, ring, cit, sl.R, nch, S.trace ? sctl + 3 : nullptr);
-        else if (J <= 3) kvm_gemv_ring<3>(c, sl.args, sl.lb, ring, cit, sl.R, nch, S.trace ? sctl + 3 : nullptr);
+        const int J = kvm_gv_pieces(sl.args[8]);
+        if (S.trace) kvm_gemv_ring_traced(c, sl.args, sl.lb, ring, cit, sl.R, nch, sctl + 3);
+        else if (J == 1) kvm_gemv_ring<1, false>(c, sl.args, sl.lb, ring, cit, sl.R, nch, nullptr);
+        else if (J <= 3) kvm_gemv_ring<3, false>(c, sl.args, sl.lb, ring, cit, sl.R, nch, nullptr);
         else kvm_gemv_ring_wide(c, sl.args, sl.lb, ring, cit, sl.R, nch);
       }
-      else if (kind == 3) kvm_gemv_mma_ring(c, sl.args, sl.lb, op == 301, ring, cit, sl.newrow, deadline, t_task, S.trace ? sctl + 3 : nullptr);
-      else if (kind == 2) kvm_attn_part_ring(c, sl.args, sl.lb, op == 300, ring, cit, sl.j0, sl.j1, sl.newrow);
+      else if (kind == 3) kvm_gemv_mma_ring(c, sl.args, sl.lb, op == 301, ring, cit, sl.newrow, S.trace ? sctl + 3 : nullptr);
+      else if (kind == 2) {
+        if (S.trace) kvm_attn_part_ring_traced(c, sl.args, sl.lb, op == 300, ring, cit, sl.j0, sl.j1, sl.newrow, sctl + 3);
+        else kvm_attn_part_ring<false>(c, sl.args, sl.lb, op == 300, ring, cit, sl.j0, sl.j1, sl.newrow, nullptr);
+      }
       else if (op != 0 && go == 1 && !(op == 136 && kvm_hot_merge(c, sl.args))) kvm_dispatch(c, op, sl.args, sl.aux);
       cit += (unsigned)nch;
       // Results that a later bulk copy or TMA load may read (cache rows appended by an attention split, operands of tensor-core ops)
@@ -922,8 +946,10 @@ __global__ void __launch_bounds__(KVM_ST_THREADS, 1) kvm_static_kernel(KvmStatic
       if (kind != 1 && kind != 3) asm volatile("fence.proxy.async;" ::: "memory");
       kvm_sync();
       if (tid == 0) {
-        if (S.trace) {                                       // bits 8.. : detail of a streamed task (a GEMV: prologue | stage loop, a byte each in units of 0.2 us)
-          const int detail = kind == 1 ? min(255, (sctl[3] - sctl[5]) / 200) | min(255, (sctl[4] - sctl[3]) / 200) << 8 : sctl[3];
+        if (S.trace) {                                       // bits 8.. : detail of a streamed task (kvm_trace_detail)
+          const int pro = sctl[3] ? sctl[3] - sctl[5] : 0, waits = sctl[3 + KVM_ST_WAITED];
+          const int detail = kind == 1 || kind == 3 ? min(255, pro / 200) | min(255, (sctl[4] - sctl[3]) / 200) << 8 | min(255, waits / 200) << 16
+                           : kind == 2 ? min(255, pro / 100) | min(255, waits / 100) << 8 : 0;
           S.t_end[task] = kvm_globaltimer(); S.t_smid[task] = (int)kvm_smid() | (detail << 8);
         }
         atomicAdd(&S.exec_count[task], 1);                   // no result needed: nothing waits for the old value
@@ -940,9 +966,8 @@ __global__ void __launch_bounds__(KVM_ST_THREADS, 1) kvm_static_kernel(KvmStatic
         sctl[0] = (int)cit;
         sl.state = 0;
       }
-      ++finished;
     }
-    if (tid == 0) { sctl[1] = finished; atomicAdd(S.done, finished); }
+    if (tid == 0) { sctl[1] = i; atomicAdd(S.done, i); }
   }
   __syncthreads();
   // copies issued but never consumed (an early exit): wait for them, bounded, before the shared memory goes away

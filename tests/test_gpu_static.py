@@ -229,3 +229,43 @@ def test_decode_batch_as_rows_equals_per_user_decode(kvm_lib):
             execs, observed = ex.task_counts()
             assert (execs == 1).all() and np.array_equal(observed, br.tasks['indegree'])
         assert got == ref, (qkn, got, ref)
+
+
+def test_trace_detail_of_streamed_tasks(kvm_lib):
+    """Prologue, stage loop and waits of every kind of streamed task, within the task's own time (kvm_trace_detail's units)."""
+    from kvm_b200.executor import Executor
+    from kvm_b200.workloads.graph import Graph
+    g, kinds, K, rows = Graph('detail'), [], 2048, 148 * 256
+    g.buffer('w', rows, K, 'bf16', {'kind': 'seeded', 'seed': 1, 'scale': 0.02, 'dist': 'normal'})
+    g.buffer('wide', 16, 12544, 'bf16', {'kind': 'seeded', 'seed': 2, 'scale': 0.02, 'dist': 'normal'})
+    for n, r, c in (('x', 1, K), ('xw', 1, 12544), ('o', 1, rows), ('ow', 1, 16), ('q', 1, 512), ('kv', 1, 128), ('part', 32, 130)):
+        g.buffer(n, r, c, init={'kind': 'fill', 'value': 0.5} if n[0] in 'xqk' else None)
+    for n in ('kc', 'vc'):
+        g.buffer(n, 2048, 128, 'bf16', {'kind': 'seeded', 'seed': 3, 'scale': 1.0, 'dist': 'normal'})
+    g.data('lens', np.array([[2000]], np.int32), 'i32')
+    common = {'x2': None, 'gamma': None, 'res': None, 'pro': 0, 'eps': 0.0}
+    for n in range(0, rows, 256):
+        g.task('gemv_bf16', {**common, 'x': 'x', 'w': 'w', 'out': 'o', 'n0': n, 'n1': n + 256, 'K': K}, ['x'], [('o', (0, 1), (n, n + 256))])
+        kinds.append('gemv')
+    g.task('gemv_bf16', {**common, 'x': 'xw', 'w': 'wide', 'out': 'ow', 'n0': 0, 'n1': 16, 'K': 12544}, ['xw'], ['ow'])
+    kinds.append('gemv')
+    for s in range(8):
+        g.task('attn_decode_part', {'q': 'q', 'kc': 'kc', 'vc': 'vc', 'lens': 'lens', 'part': 'part', 'knew': 'kv', 'vnew': 'kv', 'b': 0, 'kvh': 0, 's': s, 'S': 8, 'H': 4, 'Hkv': 1,
+                                    'hd': 128, 'Tmax': 2048, 'scale': 0.1, 'theta': 1e4, 'flags': 3}, ['q'], [('part', (s * 4, s * 4 + 4))])
+        kinds.append('part')
+    b = g.to_bundle()
+    kinds = np.array([{134: 'gemv', 135: 'part'}.get(int(o), '') for o in b.tasks['op_id']])
+    with Executor(trace=True) as ex:
+        ex.load(b)
+        ex.run()
+        assert ex.plan_info()[:2] == (True, True)
+        st, en, _ = ex.trace()
+        d = ex.trace_detail()
+    us = (en.astype(np.int64) - st.astype(np.int64)) / 1e3
+    first, second, third = d & 255, d >> 8 & 255, d >> 16 & 255
+    gemv, part = kinds == 'gemv', kinds == 'part'
+    assert (first[part] > 0).all() and (first[part] * 0.1 + second[part] * 0.1 <= us[part] + 0.2).all()
+    assert (second[gemv] > 0).all() and (first[gemv] * 0.2 + second[gemv] * 0.2 <= us[gemv] + 0.4).all()
+    # sixteen stages of 64 KB a task with every SM pulling: the copies take longer than the arithmetic
+    assert (third[gemv] <= second[gemv]).all() and (third[gemv] > 0).sum() > 74
+    assert (d[(kinds == '')] == 0).all()
