@@ -171,6 +171,17 @@ __device__ __forceinline__ bool kvm_gv_args_ok(const KvmCtx& c, const int32_t* a
   return ok;
 }
 
+// Reciprocal RMS of a row from the threads' sums of squares (one barrier).
+__device__ __forceinline__ float kvm_gv_rms(const KvmCtx& c, float q, int rg, int KP, int K, float eps) {
+  float* red = (float*)c.smem;
+  q = kvm_warp_sum(q);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = q;
+  kvm_sync();
+  q = 0.0f;
+  for (int i = 0; i < KP; ++i) q += red[rg * KP + i];
+  return 1.0f / sqrtf(q / K + eps);
+}
+
 template <int J, bool TR>      // TR: notes its times in `stamp` (KVM_ST_WAITED)
 __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, const KvmRing ring, unsigned cit, int R, int NC, int* stamp) {
   const int K = a[8], rows = a[7] - a[6], KP = kvm_gv_parts(K);
@@ -197,24 +208,43 @@ __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a,
     const float* up = nullptr;                             // the prologue's second operand: gamma or the up projection
     if (pro == 1) { up = (const float*)lb[2].p; f32 = f32 && kvm_vec_ok(lb[2]); }
     else if (pro == 2) { up = (const float*)lb[1].p; f32 = f32 && lb[1].dtype == KVM_F32 && kvm_vec_ok(lb[1]); }
-    if (J > 1 && ok && f32 && pro == 2) {
-      // piece after piece (the next one's loads in flight), the results through shared memory: with all 8 J evaluations of silu unrolled
-      // their code does not stay in the instruction cache between tasks (a token of the 8B shape: 5.63 ms unrolled, 5.56 as a loop)
+    if (J > 1 && ok && f32) {
+      // piece after piece (the next one's loads in flight), the results through shared memory: with a thread's 8 J evaluations of silu
+      // unrolled their code does not stay in the instruction cache between tasks (a token of the 8B shape: 5.63 ms unrolled, 5.56 as a
+      // loop), and all the loads of three pieces at once leave the kernel no registers
       uint4* mine = (uint4*)(c.smem + ((KVM_GV_RED + rows * KP * 4 + 15) & ~15));
       const float* xp = (const float*)x.p;
-      float4 a0, a1, b0, b1;
-      auto load = [&](int k) {
-        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      float rs = 1.0f;
+      float4 a0, a1, b0 = zero, b1 = zero;
+      auto load = [&](int k, bool both) {
         a0 = k < K ? *(const float4*)(xp + k) : zero; a1 = k < K ? *(const float4*)(xp + k + 4) : zero;
-        b0 = k < K ? *(const float4*)(up + k) : zero; b1 = k < K ? *(const float4*)(up + k + 4) : zero;
+        if (both) { b0 = k < K ? *(const float4*)(up + k) : zero; b1 = k < K ? *(const float4*)(up + k + 4) : zero; }
       };
-      load(k0);
+      if (pro == 1) {
+        float q = 0.0f;
+        load(k0, false);
+#pragma unroll 1
+        for (int k = k0; k < K; k += kstep) {
+          const float4 p0 = a0, p1 = a1;
+          load(k + kstep, false);
+          q += p0.x * p0.x; q += p0.y * p0.y; q += p0.z * p0.z; q += p0.w * p0.w; q += p1.x * p1.x; q += p1.y * p1.y; q += p1.z * p1.z; q += p1.w * p1.w;
+        }
+        rs = kvm_gv_rms(c, q, rg, KP, K, kvm_bits_f32(a[10]));
+      }
+      load(k0, pro != 0);
 #pragma unroll 1
       for (int k = k0; k < K; k += kstep) {
         const float4 p0 = a0, p1 = a1, q0 = b0, q1 = b1;
-        load(k + kstep);
-        const float t[8] = {kvm_silu(p0.x) * q0.x, kvm_silu(p0.y) * q0.y, kvm_silu(p0.z) * q0.z, kvm_silu(p0.w) * q0.w,
-                            kvm_silu(p1.x) * q1.x, kvm_silu(p1.y) * q1.y, kvm_silu(p1.z) * q1.z, kvm_silu(p1.w) * q1.w};
+        load(k + kstep, pro != 0);
+        const float p[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w}, q[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+        float t[8];
+        if (pro == 2)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) t[i] = kvm_silu(p[i]) * q[i];
+        else
+#pragma unroll
+          for (int i = 0; i < 8; ++i) t[i] = pro == 1 ? p[i] * rs * q[i] : p[i];
         mine[k / 8] = kvm_pack_bf16x8(t);
       }
 #pragma unroll
@@ -227,41 +257,26 @@ __device__ __forceinline__ void kvm_gemv_ring(const KvmCtx& c, const int32_t* a,
         put(j, t);
       }
     } else if (ok && f32) {
-      // float32 rows: all loads of a thread in flight together
-      float v[J][8], u[J][8];
+      // one piece per thread, float32: all loads in flight together
+      float v[8], u[8];
+      const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-      for (int j = 0; j < J; ++j) {
-        const int k = k0 + j * kstep;
-#pragma unroll
-        for (int i = 0; i < 8; i += 4) {
-          const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          const float4 t = k < K ? *(const float4*)((const float*)x.p + k + i) : zero, g = k < K && pro ? *(const float4*)(up + k + i) : zero;
-          v[j][i] = t.x; v[j][i + 1] = t.y; v[j][i + 2] = t.z; v[j][i + 3] = t.w;
-          u[j][i] = g.x; u[j][i + 1] = g.y; u[j][i + 2] = g.z; u[j][i + 3] = g.w;
-        }
+      for (int i = 0; i < 8; i += 4) {
+        const float4 t = k0 < K ? *(const float4*)((const float*)x.p + k0 + i) : zero, g = k0 < K && pro ? *(const float4*)(up + k0 + i) : zero;
+        v[i] = t.x; v[i + 1] = t.y; v[i + 2] = t.z; v[i + 3] = t.w;
+        u[i] = g.x; u[i + 1] = g.y; u[i + 2] = g.z; u[i + 3] = g.w;
       }
       float rs = 1.0f;
       if (pro == 1) {
         float q = 0.0f;
 #pragma unroll
-        for (int j = 0; j < J; ++j)
-#pragma unroll
-          for (int i = 0; i < 8; ++i) q += v[j][i] * v[j][i];
-        q = kvm_warp_sum(q);
-        float* red = (float*)c.smem;
-        if (lane == 0) red[warp] = q;
-        kvm_sync();
-        q = 0.0f;
-        for (int i = 0; i < KP; ++i) q += red[rg * KP + i];
-        rs = 1.0f / sqrtf(q / K + kvm_bits_f32(a[10]));
+        for (int i = 0; i < 8; ++i) q += v[i] * v[i];
+        rs = kvm_gv_rms(c, q, rg, KP, K, kvm_bits_f32(a[10]));
       }
+      float t[8];
 #pragma unroll
-      for (int j = 0; j < J; ++j) {
-        float t[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) t[i] = kvm_bf16_round(pro == 1 ? v[j][i] * rs * u[j][i] : pro == 2 ? kvm_silu(v[j][i]) * u[j][i] : v[j][i]);
-        put(j, t);
-      }
+      for (int i = 0; i < 8; ++i) t[i] = kvm_bf16_round(pro == 1 ? v[i] * rs * u[i] : pro == 2 ? kvm_silu(v[i]) * u[i] : v[i]);
+      put(0, t);
     } else {
       // anything else is staged through shared memory (behind the partial sums)
       __nv_bfloat16* vs = (__nv_bfloat16*)(c.smem + ((KVM_GV_RED + rows * KP * 4 + 15) & ~15));

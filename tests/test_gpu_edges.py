@@ -62,3 +62,23 @@ def test_argmax_of_masked_rows(kvm_lib, V):
     ex, vm, res = run_both(g.to_bundle())
     assert ex.read_buffer('t').ravel().tolist() == [0, 0, V - 1, 5000] == vm.buffer('t').a.ravel().tolist()
     ex.close()
+
+
+# rows of two, three and four pieces per thread, normalised and plain: the loop over a thread's pieces with its remainder
+@pytest.mark.parametrize('K', [4104, 8192, 12280, 12296])
+def test_streamed_gemv_of_several_pieces(kvm_lib, K):
+    from kvm_b200.workloads.graph import Graph
+    rng = np.random.default_rng(K)
+    g = Graph('pieces')
+    g.data('x', rng.standard_normal((1, K)).astype(np.float32)), g.data('u', rng.standard_normal((1, K)).astype(np.float32))
+    g.data('w', (rng.standard_normal((70, K)) * 0.02).astype(np.float32), 'bf16'), g.data('res', rng.standard_normal((1, 70)).astype(np.float32))
+    for pro in (0, 1, 2):
+        g.buffer(f'o{pro}', 1, 70)
+        for n0, n1 in ((0, 33), (33, 70)):
+            g.task('gemv_bf16', {'x': 'x', 'x2': 'u', 'gamma': 'u', 'w': 'w', 'out': f'o{pro}', 'res': 'res', 'n0': n0, 'n1': n1, 'K': K, 'pro': pro, 'eps': 1e-6},
+                   ['x'], [(f'o{pro}', (0, 1), (n0, n1))])
+    ex, vm, res = run_both(g.to_bundle())
+    assert ex.plan_info()[:2] == (True, True)
+    # an activation on a rounding tie of bf16 may fall on the other side: 2^-9 of one of K terms
+    compare(ex, vm, 2.0 ** -9 / K ** 0.5 * 4)
+    ex.close()
