@@ -670,6 +670,62 @@ KVM_OP_FN void kvm_attn_part_ring_traced(const KvmCtx& c, const int32_t* a, cons
   kvm_attn_part_ring<true>(c, a, lb, qkn, ring, cit, j0, j1, newrow, stamp);
 }
 
+// Splits that the warp form (kvm_ring_attn.cuh) does not take, from the same two stages: queries in float32 (flags 0 and 1), head dimension
+// 16.  One softmax over the split by all warps (kvm_attn_part_core); one, two or four query heads per key
+// head (eight need more scratch than the three stages leave).
+KVM_OP_FN void kvm_attn_part_ring_any(const KvmCtx& c, const int32_t* a, const KvmBuf* lb, bool qkn, const KvmRing ring, unsigned cit, int j0, int j1, int newrow, int* stamp) {
+  KvmBuf q, kc, vc, lens, part, kn, vn, gam{};
+  bool ok = kvm_buf_local(c, lb, a, 0, KVM_M_FLT, q) && kvm_buf_local(c, lb, a, 1, KVM_M_BF16, kc) && kvm_buf_local(c, lb, a, 2, KVM_M_BF16, vc) &&
+            kvm_buf_local(c, lb, a, 3, KVM_M_I32, lens) && kvm_buf_local(c, lb, a, 4, KVM_M_F32, part) && kvm_buf_local(c, lb, a, 5, KVM_M_FLT, kn, true) &&
+            kvm_buf_local(c, lb, a, 6, KVM_M_FLT, vn, true);
+  const int b = a[7], kvh = a[8], S = a[10], H = a[11], Hkv = a[12], hd = a[13], fl = a[17], G = H / Hkv, nk = max(j1 - j0, 0);
+  if (ok && qkn) ok = kvm_buf(c, a[18], KVM_M_F32, gam) && kvm_mat_ok(c, gam, 2, hd);
+  if (ok) ok = kvm_mat_ok(c, q, b + 1, H * hd) && kvm_mat_ok(c, part, (long long)(b + 1) * S * H, hd + 2) && kvm_mat_ok(c, kn, b + 1, Hkv * hd) && kvm_mat_ok(c, vn, b + 1, Hkv * hd);
+  if (ok && (fl & 1) && (!kn.p || !vn.p)) { c.fail(KVM_OPE_SHAPE, hd, fl); ok = false; }
+  auto wait = [&](unsigned it) {
+    const int t0 = stamp ? (int)kvm_globaltimer() : 0;
+    const bool landed = kvm_ring_wait_warp(ring, it, c.deadline, c.err);
+    if (stamp && threadIdx.x == 0) {
+      if (it == cit) stamp[0] = t0;
+      stamp[KVM_ST_WAITED] += (int)kvm_globaltimer() - t0;
+    }
+    return landed;
+  };
+  auto wk = [&]() { return wait(cit); };
+  auto wv = [&]() { return wait(cit + 1); };
+  kvm_sync();                                              // the previous task is done with the scratch
+  bool waited;
+  if (ok) {
+    unsigned char* sm = c.smem;
+    KvmPartPro P;
+    P.q = q; P.kc = kc; P.vc = vc; P.kn = kn; P.vn = vn; P.gam = gam;
+    P.b = b; P.kvh = kvh; P.G = G; P.hd = hd; P.fl = fl; P.p0 = ((const int*)lens.p)[b]; P.base = (size_t)(b * Hkv + kvh) * a[14]; P.theta = kvm_bits_f32(a[16]);
+    P.eps = qkn ? kvm_bits_f32(a[19]) : 0.0f; P.appends = newrow >= 0; P.rope_cache = c.rope_cache;
+    P.qs = (float*)(sm + KVM_AS_OFF_QS); P.inv = (float*)(sm + KVM_AS_OFF_INV); P.kns = (float*)(sm + KVM_AS_OFF_KNEW); P.vns = (float*)(sm + KVM_AS_OFF_VNEW);
+    P.rsq = (float*)(sm + KVM_AS_OFF_ML);
+    auto prologue = [&]() { kvm_part_prologue(P); };
+    auto emit = [&](int g, int cc, float M, float L, float A) {
+      float* row = (float*)part.p + ((size_t)(b * S + a[9]) * H + kvh * G + g) * part.ld;
+      row[cc] = L > 0.0f ? A : 0.0f;
+      if (cc == 0) { row[hd] = L > 0.0f ? M : KVM_ATTN_EMPTY_M_STREAM; row[hd + 1] = L; }
+    };
+    unsigned char* Ks = kvm_ring_stage(ring, cit);
+    unsigned char* Vs = kvm_ring_stage(ring, cit + 1);
+    const float sc = kvm_bits_f32(a[15]);
+    if (G <= 1) waited = kvm_attn_part_core<1>(sm, Ks, Vs, nk, newrow, G, hd, sc, prologue, wk, wv, emit);
+    else if (G <= 2) waited = kvm_attn_part_core<2>(sm, Ks, Vs, nk, newrow, G, hd, sc, prologue, wk, wv, emit);
+    else if (G <= 4) waited = kvm_attn_part_core<4>(sm, Ks, Vs, nk, newrow, G, hd, sc, prologue, wk, wv, emit);
+    else waited = kvm_attn_part_core<8>(sm, Ks, Vs, nk, newrow, G, hd, sc, prologue, wk, wv, emit);
+  } else {
+    waited = wk() && wv();
+  }
+  if (!waited && *(volatile int*)&c.err->code == 0) kvm_stream_timeout(c, 1135);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the appended row was written by threads; the next copies into these stages come after it
+  kvm_sync();
+  if (waited && (threadIdx.x & 31) == 0) { kvm_mbar_arrive(kvm_ring_empty(ring, cit)); kvm_mbar_arrive(kvm_ring_empty(ring, cit + 1)); }
+}
+__device__ __forceinline__ bool kvm_ra_takes(int hd, int flags) { return flags == 3 && hd != 16; }      // the warp form
+
 // ---- front warp: stream geometry of a fetched task (lane 0) ---------------------------------------------------------------------
 // Decides whether the task streams through the ring and with which chunking; every bound the copies rely on is checked here,
 // a task that fails one runs as a generic op (whose own checks then report the error).
@@ -694,16 +750,17 @@ static __device__ void kvm_static_geometry(const KvmDevState& S, KvmStSlot& sl, 
   } else if (op == 135 || op == 300) {
     const int kci = a[1], vci = a[2], li = a[3], b = a[7], kvh = a[8], s = a[9], Sp = a[10], H = a[11], Hkv = a[12], hd = a[13], Tmax = a[14], fl = a[17];
     if (kci < 0 || kci >= S.nbufs || vci < 0 || vci >= S.nbufs || li < 0 || li >= S.nbufs) return;
-    if (b < 0 || Hkv <= 0 || H <= 0 || H % Hkv || kvh < 0 || kvh >= Hkv || s < 0 || Sp <= 0 || s >= Sp || Tmax <= 0 || fl != 3) return;      // other flags: the op's own form
+    if (b < 0 || Hkv <= 0 || H <= 0 || H % Hkv || kvh < 0 || kvh >= Hkv || s < 0 || Sp <= 0 || s >= Sp || Tmax <= 0 || !(fl == 0 || fl == 1 || fl == 3)) return;
     const int G = H / Hkv;
-    if (G > 8 || !(hd == 32 || hd == 64 || hd == 128)) return;
+    const bool warp_form = kvm_ra_takes(hd, fl);
+    if (G > 8 || !(hd == 16 || hd == 32 || hd == 64 || hd == 128) || (!warp_form && (G & (G - 1)))) return;
     const KvmBuf kc = sl.lb[1], vc = sl.lb[2], lens = sl.lb[3];
     if (!kc.p || !vc.p || !lens.p || kc.dtype != KVM_BF16 || vc.dtype != KVM_BF16 || lens.dtype != KVM_I32 || kc.ld != hd || vc.ld != hd || ((uintptr_t)kc.p & 15) || ((uintptr_t)vc.p & 15)) return;
     if ((long long)(b + 1) * Hkv * Tmax > kc.rows || (long long)(b + 1) * Hkv * Tmax > vc.rows || hd > kc.cols || hd > vc.cols || lens.ld != lens.cols || b >= lens.rows * lens.cols) return;
     const int p0 = ((const int*)lens.p)[b], n = p0 + 1;
     if (p0 < 0 || n > Tmax) return;
     const int chunk = (n + Sp - 1) / Sp, j0 = s * chunk, j1 = min(n, s * chunk + chunk), nk = max(j1 - j0, 0);
-    if (nk * hd * 2 > KVM_ST_STAGE || KVM_RA_BYTES > scratch_bytes) return;
+    if (nk * hd * 2 > KVM_ST_STAGE || (warp_form ? KVM_RA_BYTES : kvm_attn_part_scratch(nk, G, hd)) > scratch_bytes) return;
     sl.kind = 2; sl.nchunks = 2; sl.j0 = j0; sl.j1 = j1;
     sl.newrow = ((fl & 1) && j0 <= n - 1 && n - 1 < j1) ? n - 1 - j0 : -1;
   }
@@ -950,7 +1007,8 @@ __global__ void __launch_bounds__(KVM_ST_THREADS, 1) kvm_static_kernel(KvmStatic
       }
       else if (kind == 3) kvm_gemv_mma_ring(c, sl.args, sl.lb, op == 301, ring, cit, sl.newrow, S.trace ? sctl + 3 : nullptr);
       else if (kind == 2) {
-        if (S.trace) kvm_attn_part_ring_traced(c, sl.args, sl.lb, op == 300, ring, cit, sl.j0, sl.j1, sl.newrow, sctl + 3);
+        if (!kvm_ra_takes(sl.args[13], sl.args[17])) kvm_attn_part_ring_any(c, sl.args, sl.lb, op == 300, ring, cit, sl.j0, sl.j1, sl.newrow, S.trace ? sctl + 3 : nullptr);
+        else if (S.trace) kvm_attn_part_ring_traced(c, sl.args, sl.lb, op == 300, ring, cit, sl.j0, sl.j1, sl.newrow, sctl + 3);
         else kvm_attn_part_ring<false>(c, sl.args, sl.lb, op == 300, ring, cit, sl.j0, sl.j1, sl.newrow, nullptr);
       }
       else if (op != 0 && go == 1 && !(op == 136 && kvm_hot_merge(c, sl.args))) kvm_dispatch(c, op, sl.args, sl.aux);
