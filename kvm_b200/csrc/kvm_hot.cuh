@@ -3,7 +3,7 @@
 // memory cannot hold: 2-4 us per task).  Each takes the common storage types and alignments and returns false for anything else,
 // argument errors included: the op's general body (kvm_ops_rows.cuh, kvm_ops_flat.cuh, kvm_ops_attn.cuh) then does the task or
 // reports the error.  Storage types are template arguments, so that the loads of a batch are issued back to back.
-// One SM's share of HBM is 44 KB/us at a loaded latency of 1.5 us: the loops below keep 48-64 KB per SM in flight.
+// One SM's share of HBM is 44 KB/us at a loaded latency of 1.5 us: 66 KB in flight keep it busy.  The streaming loops have 64 to 128.
 #pragma once
 #include "kvm_attn_tc.cuh"
 #include "kvm_decode_stream.cuh"
@@ -432,14 +432,16 @@ __device__ __forceinline__ bool kvm_hot_ce_fused(const KvmCtx& c, const int32_t*
 // NI inputs of a flat range come through shared memory: bulk copies of SE elements per input, four stages deep (96-128 KB in flight,
 // none of it in registers), every thread works on its part of the stage that has landed and stores its results from registers.
 // With the same bytes in flight in registers the loops spilled, and the spills' traffic cost more than the loads.
-// body(stage, i, n): stage = the inputs' parts of the stage (shared memory), elements [i, i + n) of the range.
+// body(stage, i, n): stage = the inputs' parts of the stage (shared memory), elements [i, i + n) of the range.  false, with nothing done, where
+// the stages do not fit the scratch.
 #define KVM_STREAM_DEPTH 4
 #define KVM_STREAM_BAR 8                               // barriers KVM_CTL_ABAR + 8 .. + 11 and their completed-phase counts
 template <int NI, int SE, class Body>
-__device__ __forceinline__ void kvm_stream(const KvmCtx& c, const char* const (&in)[NI], const int (&eb)[NI], int e0, int e1, Body body) {
+__device__ __forceinline__ bool kvm_stream(const KvmCtx& c, const char* const (&in)[NI], const int (&eb)[NI], int e0, int e1, Body body) {
   int off[NI], bytes = 0;
 #pragma unroll
   for (int n = 0; n < NI; ++n) { off[n] = bytes; bytes += SE * eb[n]; }
+  if (c.smem_bytes < 1024 + KVM_STREAM_DEPTH * bytes) return false;
   const int ns = (e1 - e0 + SE - 1) / SE;
   int* cnt = c.ctl + KVM_CTL_ACNT + KVM_STREAM_BAR;
   auto bar = [&](int s) { return kvm_bar_addr(c.ctl, KVM_CTL_ABAR + KVM_STREAM_BAR + (s & (KVM_STREAM_DEPTH - 1))); };
@@ -481,6 +483,7 @@ __device__ __forceinline__ void kvm_stream(const KvmCtx& c, const char* const (&
   }
   if (!ok) kvm_att_fail(c, 2000);
   if (threadIdx.x < KVM_STREAM_DEPTH) cnt[threadIdx.x] += (ns - (int)threadIdx.x + KVM_STREAM_DEPTH - 1) / KVM_STREAM_DEPTH;
+  return true;
 }
 __device__ __forceinline__ bool kvm_hot_range(int e0, int e1, int align) { return e0 >= 0 && e1 > e0 && ((e0 | e1) & (align - 1)) == 0; }
 
@@ -494,7 +497,7 @@ __device__ __forceinline__ bool kvm_hot_map2(const KvmCtx& c, int i0, int i1, in
   if (!kvm_hot_range(e0, e1, E) || !kvm_hot_buf(c, i0, dt, x) || !kvm_hot_buf(c, i1, dt, y) || !kvm_hot_buf(c, o, dt, z) || !kvm_hot_flat(x, e1) || !kvm_hot_flat(y, e1) || !kvm_hot_flat(z, e1)) return false;
   const char* const in[2] = {(const char*)x.p, (const char*)y.p};
   const int eb[2] = {EB, EB};
-  kvm_stream<2, KVM_NT * E>(c, in, eb, e0, e1, [&](const char* const (&part)[2], int i, int n) {
+  return kvm_stream<2, KVM_NT * E>(c, in, eb, e0, e1, [&](const char* const (&part)[2], int i, int n) {
     const int k = (int)threadIdx.x * E;
     if (k >= n) return;
     const uint4 u = *(const uint4*)(part[0] + k * EB), v = *(const uint4*)(part[1] + k * EB);
@@ -507,7 +510,6 @@ __device__ __forceinline__ bool kvm_hot_map2(const KvmCtx& c, int i0, int i1, in
     }
     *(uint4*)((char*)z.p + (size_t)(i + k) * EB) = w;
   });
-  return true;
 }
 // f32 -> bf16
 __device__ __forceinline__ bool kvm_hot_round_bf16(const KvmCtx& c, const int32_t* a) {
@@ -516,11 +518,10 @@ __device__ __forceinline__ bool kvm_hot_round_bf16(const KvmCtx& c, const int32_
   if (!kvm_hot_buf(c, a[0], KVM_F32, x) || !kvm_hot_buf(c, a[1], KVM_BF16, o) || !kvm_hot_range(e0, e1, 4) || !kvm_hot_flat(x, e1) || !kvm_hot_flat(o, e1)) return false;
   const char* const in[1] = {(const char*)x.p};
   const int eb[1] = {4};
-  kvm_stream<1, 4 * KVM_NT * 4>(c, in, eb, e0, e1, [&](const char* const (&part)[1], int i, int n) {
+  return kvm_stream<1, 4 * KVM_NT * 4>(c, in, eb, e0, e1, [&](const char* const (&part)[1], int i, int n) {
 #pragma unroll
     for (int u = 0; u < 4; ++u) { const int k = (u * KVM_NT + (int)threadIdx.x) * 4; if (k < n) *(uint2*)((__nv_bfloat16*)o.p + i + k) = kvm_to_bf16x4(*(const float4*)(part[0] + k * 4)); }
   });
-  return true;
 }
 // AdamW, float32 state
 __device__ __forceinline__ bool kvm_hot_adamw(const KvmCtx& c, const int32_t* a) {
@@ -536,7 +537,7 @@ __device__ __forceinline__ bool kvm_hot_adamw(const KvmCtx& c, const int32_t* a)
   const char* const in[4] = {(const char*)p.p, (const char*)g.p, (const char*)m.p, (const char*)v.p};
   const int eb[4] = {4, 4, 4, 4};
   float* pp = (float*)p.p; float* mp = (float*)m.p; float* vp = (float*)v.p;
-  kvm_stream<4, KVM_NT * 4>(c, in, eb, e0, e1, [&](const char* const (&part)[4], int i, int n) {
+  return kvm_stream<4, KVM_NT * 4>(c, in, eb, e0, e1, [&](const char* const (&part)[4], int i, int n) {
     const int q = (int)threadIdx.x * 4;
     if (q >= n) return;
     float4 P = *(const float4*)(part[0] + q * 4), M = *(const float4*)(part[2] + q * 4), W = *(const float4*)(part[3] + q * 4);
@@ -544,7 +545,6 @@ __device__ __forceinline__ bool kvm_hot_adamw(const KvmCtx& c, const int32_t* a)
     kvm_adamw_step(k, G.x, P.x, M.x, W.x); kvm_adamw_step(k, G.y, P.y, M.y, W.y); kvm_adamw_step(k, G.z, P.z, M.z, W.z); kvm_adamw_step(k, G.w, P.w, M.w, W.w);
     *(float4*)(pp + i + q) = P; *(float4*)(mp + i + q) = M; *(float4*)(vp + i + q) = W;
   });
-  return true;
 }
 __device__ __forceinline__ bool kvm_hot_gradnorm(const KvmCtx& c, const int32_t* a) {
   KvmBuf g, part;
@@ -553,7 +553,7 @@ __device__ __forceinline__ bool kvm_hot_gradnorm(const KvmCtx& c, const int32_t*
   double s = 0.0;
   const char* const in[1] = {(const char*)g.p};
   const int eb[1] = {4};
-  kvm_stream<1, 2 * KVM_NT * 8>(c, in, eb, e0, e1, [&](const char* const (&st)[1], int, int n) {
+  const bool taken = kvm_stream<1, 2 * KVM_NT * 8>(c, in, eb, e0, e1, [&](const char* const (&st)[1], int, int n) {
 #pragma unroll
     for (int u = 0; u < 2; ++u) {                      // eight squares in sequence, as the general body
       const int k = (u * KVM_NT + (int)threadIdx.x) * 8;
@@ -566,6 +566,7 @@ __device__ __forceinline__ bool kvm_hot_gradnorm(const KvmCtx& c, const int32_t*
       }
     }
   });
+  if (!taken) return false;
   s = kvm_block_sum(s, (double*)c.smem);
   if (threadIdx.x == 0) ((float*)part.p)[slot] = (float)s;
   return true;
