@@ -262,6 +262,7 @@ static std::string kvm_validate(const KvmTaskDesc* t, int nt, const int32_t* suc
   char m[256];
   if (nt <= 0) return "empty bundle";
   std::vector<int> in(nt, 0);
+  bool forward = true;      // every edge leads to a later task: no cycle to look for
   for (int i = 0; i < nt; ++i) {
     const KvmTaskDesc& d = t[i];
     const KvmOpInfo* op = kvm_find_op(d.op_id);
@@ -281,18 +282,21 @@ static std::string kvm_validate(const KvmTaskDesc* t, int nt, const int32_t* suc
     for (int k = 0; k < d.succ_cnt; ++k) {
       const int s = succ[d.succ_off + k];
       if (s < 0 || s >= nt || s == i) { snprintf(m, sizeof m, "task %d: successor %d out of range", i, s); return m; }
+      forward &= s > i;
       ++in[s];
     }
   }
   for (int i = 0; i < nt; ++i) if (in[i] != t[i].indegree) { snprintf(m, sizeof m, "task %d: indegree %d != in-edges %d", i, t[i].indegree, in[i]); return m; }
-  std::vector<int> q, rem = in;
-  q.reserve(nt);
-  for (int i = 0; i < nt; ++i) if (!rem[i]) q.push_back(i);
-  for (size_t x = 0; x < q.size(); ++x) {
-    const KvmTaskDesc& d = t[q[x]];
-    for (int k = 0; k < d.succ_cnt; ++k) if (--rem[succ[d.succ_off + k]] == 0) q.push_back(succ[d.succ_off + k]);
+  if (!forward) {
+    std::vector<int> q, rem = in;
+    q.reserve(nt);
+    for (int i = 0; i < nt; ++i) if (!rem[i]) q.push_back(i);
+    for (size_t x = 0; x < q.size(); ++x) {
+      const KvmTaskDesc& d = t[q[x]];
+      for (int k = 0; k < d.succ_cnt; ++k) if (--rem[succ[d.succ_off + k]] == 0) q.push_back(succ[d.succ_off + k]);
+    }
+    if ((int)q.size() != nt) return "dependency cycle";
   }
-  if ((int)q.size() != nt) return "dependency cycle";
   // version waits decidable inside the batch: publisher -> waiter edges must keep the graph acyclic
   std::vector<std::pair<int, int>> extra;
   for (int i = 0; i < nt; ++i) if (t[i].wait_var >= 0)
@@ -336,8 +340,10 @@ extern "C" int kvm_submit(KvmExec* h, const KvmTaskDesc* tasks, int32_t nt, cons
   const std::string problem = kvm_validate(tasks, nt, succ, ne, args, na, (int)h->bufs.size(), h->nvars);
   if (!problem.empty()) { h->error = problem; return KVM_E_BUNDLE; }
   const int tbase = (int)h->tasks.size(), sbase = (int)h->succ.size(), abase = (int)h->args.size();
-  for (int i = 0; i < nt; ++i) { KvmTaskDesc d = tasks[i]; d.succ_off += sbase; d.args_off += abase; h->tasks.push_back(d); }
-  for (int i = 0; i < ne; ++i) h->succ.push_back(succ[i] + tbase);
+  h->tasks.insert(h->tasks.end(), tasks, tasks + nt);
+  for (int i = 0; i < nt; ++i) { h->tasks[tbase + i].succ_off += sbase; h->tasks[tbase + i].args_off += abase; }
+  h->succ.insert(h->succ.end(), succ, succ + ne);
+  if (tbase) for (int i = 0; i < ne; ++i) h->succ[sbase + i] += tbase;
   h->args.insert(h->args.end(), args, args + na);
   h->aux.resize(h->tasks.size(), make_int4(0, 0, 0, 0));
   h->tasks_dirty = true; h->armed = false;
@@ -546,12 +552,13 @@ static int kvm_prepare(KvmExec* h, bool keep_error = false) {
       // device form of a successor entry: task index in the low 27 bits, above it the successor's priority class (2 bits) and
       // whether it waits on a version (1 bit), so that the releasing warp needs no look at the successor's descriptor
       if (nt >= (size_t)1 << KVM_SUCC_BITS) { h->error = "too many tasks for one launch"; return KVM_E_ARG; }
-      std::vector<int32_t> enc(h->succ.size());
-      for (size_t k = 0; k < enc.size(); ++k) {
-        const KvmTaskDesc& d = h->tasks[h->succ[k]];
+      std::vector<int32_t> enc(h->succ), entry(nt);
+      for (size_t i = 0; i < nt; ++i) {
+        const KvmTaskDesc& d = h->tasks[i];
         const int cls = d.priority < 0 ? 0 : (d.priority >> 3) >= KVM_NCLASS ? KVM_NCLASS - 1 : (d.priority >> 3);
-        enc[k] = h->succ[k] | (cls << KVM_SUCC_BITS) | ((d.wait_var >= 0 ? 1 : 0) << (KVM_SUCC_BITS + 2));
+        entry[i] = (int)i | (cls << KVM_SUCC_BITS) | ((d.wait_var >= 0 ? 1 : 0) << (KVM_SUCC_BITS + 2));
       }
+      for (int32_t& e : enc) e = entry[e];
       KVM_CUDA(cudaMemcpyAsync(h->d_succ, enc.data(), enc.size() * 4, cudaMemcpyHostToDevice, h->stream));
       KVM_CUDA(cudaStreamSynchronize(h->stream));      // `enc` is a local
     }
