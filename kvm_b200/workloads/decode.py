@@ -17,7 +17,7 @@ from dataclasses import dataclass, replace
 
 import numpy as np
 
-from .graph import Graph
+from .graph import SMS, Graph
 
 
 @dataclass(frozen=True)
@@ -39,7 +39,7 @@ class DecodeConfig:
     init_std: float = 0.02
     seed: int = 0
     rows_per_task: int = 64  # weight rows per gemv task; 0 = balance every phase over `workers` SMs
-    workers: int = 148
+    workers: int = SMS
     join_threshold: int = 24  # fan-ins wider than this go through a join no-op (fewer edges, one more hop)
     lockstep: bool = False    # several users: keep them in step phase by phase (see build_decode); measured slower, kept for experiments
     qk_norm: bool = False     # Qwen3: RMSNorm of every query head and of the new key over the head dimension before RoPE (extension op attn_decode_part_qkn)

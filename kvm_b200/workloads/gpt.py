@@ -18,7 +18,7 @@ from dataclasses import dataclass, replace
 
 import numpy as np
 
-from .graph import Graph
+from .graph import SMS, Graph
 
 
 @dataclass(frozen=True)
@@ -49,6 +49,7 @@ class GPTConfig:
     flat_chunk: int = 65536
     col_chunk: int = 64
     key_chunk: int = 256
+    workers: int = SMS        # SMs the executor runs on: phases are cut for as many tasks
     join_threshold: int = 24  # a read with more producers than this waits on one join no-op instead of on each of them
 
     @property
@@ -108,7 +109,7 @@ def param_shapes(c: GPTConfig):
 
 def opt_chunk(c: GPTConfig) -> int:
     """Elements per optimizer chunk: the parameters are updated side by side, about two chunks per SM."""
-    return Graph.spread(sum(rows * cols for _, rows, cols, _, _ in param_shapes(c)) // 2, c.flat_chunk)
+    return Graph.spread(sum(rows * cols for _, rows, cols, _, _ in param_shapes(c)) // 2, c.flat_chunk, c.workers)
 
 
 def dp_exchange_layout(c: GPTConfig, world: int):
@@ -182,7 +183,7 @@ class _Emit:
     def flat(self, op, bufs_r, bufs_w, n_elems, args, tag, chunk=None):
         """Elementwise op over equally shaped buffers, chunked on row boundaries."""
         g = self.g
-        for i, (e0, e1) in enumerate(g.flat_chunks(bufs_w[0], chunk or g.spread(n_elems, self.c.flat_chunk))):
+        for i, (e0, e1) in enumerate(g.flat_chunks(bufs_w[0], chunk or g.spread(n_elems, self.c.flat_chunk, self.c.workers))):
             rd = [(b, *g.region_of(b, e0, e1)) for b in bufs_r]
             wr = [(b, *g.region_of(b, e0, e1)) for b in bufs_w]
             g.task(op, {**args, 'e0': e0, 'e1': e1}, rd, wr, self.prio, f'{tag}.{i}')
@@ -193,7 +194,7 @@ class _Emit:
         if self.bf:
             op, tm, tn = 'matmul_mma_bf16', 128, 256
         else:
-            op, tm = 'matmul_tile', g.f32_tile((M, N))
+            op, tm = 'matmul_tile', g.f32_tile((M, N), workers=self.c.workers)
             tn = tm
         ta, tb, acc = flags & 1, flags & 2, flags & 4
         for m0 in range(0, M, tm):

@@ -40,7 +40,7 @@ class _Records:
             self.n = k
 
 
-SMS = 148        # workers of the executor on a B200: one CTA per SM
+SMS = 148        # workers of the executor on a B200: one CTA per SM (the configurations' `workers`)
 
 
 class Graph:
@@ -114,18 +114,18 @@ class Graph:
         return (e0 // c, -(-e1 // c)), ALL
 
     @staticmethod
-    def spread(n, chunk, least=4096):
-        """Chunk length for a phase of `n` elements: `chunk`, or less where that would leave SMs without a task.  Below 4096 elements a
+    def spread(n, chunk, workers=SMS, least=4096):
+        """Chunk length for a phase of `n` elements: `chunk`, or less where that would leave some of `workers` SMs without a task.  Below 4096 elements a
         task is all fixed cost (3-4 us)."""
-        return min(chunk, max(least, -(-n // SMS)))
+        return min(chunk, max(least, -(-n // workers)))
 
     @staticmethod
-    def f32_tile(*products):
+    def f32_tile(*products, workers=SMS):
         """Edge of the exact float32 matmul tiles of products (M, N) that run side by side: 64, or 32 where all of them together are one
         wave of 32x32 tiles.  A 32x32 tile takes about half as long (27 against 69 ns per k), so it shortens the chain where SMs are
         idle anyway; over full SMs it would cost 1.6 times the work.  Products of a single 64x64 tile stay whole (one task, as the
         reference compiler makes them)."""
-        return 32 if any(m > 64 or n > 64 for m, n in products) and sum(-(-m // 32) * -(-n // 32) for m, n in products) <= SMS else 64
+        return 32 if any(m > 64 or n > 64 for m, n in products) and sum(-(-m // 32) * -(-n // 32) for m, n in products) <= workers else 64
 
     def flat_chunks(self, buf, target):
         """Flat ranges [e0,e1) of about `target` elements covering `buf`, cut on row boundaries (or inside single rows when a row

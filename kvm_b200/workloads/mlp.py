@@ -15,7 +15,7 @@ from dataclasses import dataclass, replace
 
 import numpy as np
 
-from .graph import Graph
+from .graph import SMS, Graph
 
 
 @dataclass(frozen=True)
@@ -29,6 +29,7 @@ class MLPConfig:
     momentum: float = 0.9
     seed: int = 0
     flat_chunk: int = 1 << 16     # elements per elementwise / optimizer task
+    workers: int = SMS            # SMs the executor runs on: phases are cut for as many tasks
 
 
 PRESETS = {
@@ -59,7 +60,7 @@ def build_mlps(c: MLPConfig, steps: int) -> Graph:
 
     def mm(tag, a, b, out, M, N, K, flags=0, bias=None, pre=None, prio=10):
         # the models run side by side: the products of all of them, each with this one's shape in its own width
-        t = g.f32_tile(*((v if M == width else M, v if N == width else N) for v in c.widths))
+        t = g.f32_tile(*((v if M == width else M, v if N == width else N) for v in c.widths), workers=c.workers)
         for m0 in range(0, M, t):
             for n0 in range(0, N, t):
                 m1, n1 = min(m0 + t, M), min(n0 + t, N)
@@ -72,7 +73,7 @@ def build_mlps(c: MLPConfig, steps: int) -> Graph:
 
     def flat(op, tag, bufs, n, extra, reads, writes, prio=10):
         # the same phase of all the models side by side (most of their elements are width x width)
-        for i, (e0, e1) in enumerate(g.flat_chunks(writes[0], g.spread(n * sum(v * v for v in c.widths) // width ** 2, c.flat_chunk))):      # chunks on row boundaries: no false dependencies
+        for i, (e0, e1) in enumerate(g.flat_chunks(writes[0], g.spread(n * sum(v * v for v in c.widths) // width ** 2, c.flat_chunk, c.workers))):      # chunks on row boundaries: no false dependencies
             g.task(op, dict(bufs, e0=e0, e1=e1, **extra), [(b, *g.region_of(b, e0, e1)) for b in reads], [(b, *g.region_of(b, e0, e1)) for b in writes], prio, f'{tag}.{i}')
 
     for mi, w in enumerate(c.widths):

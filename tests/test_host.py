@@ -276,3 +276,14 @@ def test_command_line_runner_usage_and_registry_without_a_gpu(kvm_lib):
     # a bundle directory cannot run here: the tool says why on stderr and exits 1 without a result line
     r = subprocess.run([str(cli), '/nonexistent/bundle'], capture_output=True, text=True)
     assert r.returncode == 1 and r.stdout == '' and r.stderr
+
+
+def test_phases_are_cut_for_the_workers_of_the_configuration():
+    from kvm_b200.workloads.gpt import build_training, preset as gpt
+    from kvm_b200.workloads.graph import SMS, Graph
+    from kvm_b200.workloads.mlp import build_mlps, preset as mlp
+    assert [Graph.spread(1 << 20, 1 << 16, w) for w in (16, 64, SMS, 4096)] == [1 << 16, 1 << 14, -(-(1 << 20) // SMS), 4096]
+    assert [Graph.f32_tile((256, 256), workers=w) for w in (63, 64)] == [64, 32]
+    for build, cfg in ((build_training, gpt('gpt_tiny')), (build_mlps, mlp('mlp_small'))):
+        tasks = [len(build(cfg.__class__(**{**cfg.__dict__, 'workers': w}), 1).to_bundle(check=False).tasks) for w in (8, SMS)]
+        assert tasks[0] < tasks[1] == len(build(cfg, 1).to_bundle(check=False).tasks)
