@@ -11,8 +11,9 @@
 #include <unordered_map>
 
 // Estimated duration of a task in microseconds: bytes over one SM's share of HBM for the memory-bound ops, FLOPs over one SM's
-// tensor / FMA rate for the contractions, plus a fixed cost.  Only relative sizes matter (the plan balances the workers with it).
-static double kvm_static_cost(const KvmExec* h, const KvmTaskDesc& d, const int32_t* a) {
+// tensor / FMA rate for the contractions, plus a fixed cost, both as measured on this path (tasks of the small float32 and bf16 training
+// programs and of eight MLPs).  The plan balances the workers with it.
+static double kvm_static_cost(const KvmExec* h, const KvmTaskDesc& d, const int32_t* a, const int4& aux) {
   const double BPU = 40000.0;                 // bytes per microsecond per SM (HBM share)
   auto elems = [&](int e0, int e1) { return (double)(e1 > e0 ? e1 - e0 : 0); };
   switch (d.op_id) {
@@ -22,30 +23,35 @@ static double kvm_static_cost(const KvmExec* h, const KvmTaskDesc& d, const int3
     case 136: return 8.0;                     // a few dependent round trips, measured
     case 58: case 57: return 2.0 + elems(a[d.op_id == 58 ? 2 : 3], a[d.op_id == 58 ? 3 : 4]) * a[d.op_id == 58 ? 4 : 5] * 4.0 / BPU;
     case 122: { const double m = std::min(128, a[8] - a[6]), n = std::min(256, a[9] - a[7]); return 5.0 + 2.0 * m * n * a[10] / 8.0e6; }
-    case 34: case 114: { const int tm = (a[11] & 64) ? 256 : (a[11] & 32) ? 128 : 64, tn = (a[11] & 64) ? 128 : (a[11] & 32) ? 128 : 64;
-      const double m = std::min(tm, a[8] - a[6]), n = std::min(tn, a[9] - a[7]); return 2.0 + 2.0 * m * n * a[10] / 0.2e6; }
-    case 8: return 2.0 + 2.0 * (double)a[3] * a[4] * a[5] / 0.2e6;
-    case 45: return 4.0 + 4.0 * 128.0 * (a[7] + 64.0) * a[11] / 3.0e6;
-    case 47: return 4.0 + 5.0 * 128.0 * (a[9] + 64.0) * a[13] / 3.0e6;
-    case 48: return 4.0 + 5.0 * 128.0 * std::max(64.0, (double)a[11] - a[10] - 64.0) * a[13] / 3.0e6;
-    case 46: return 2.0 + elems(a[3], a[4]) * a[6] * a[7] * 4.0 / BPU;
+    case 34: case 114: {                      // one 32 x 32 tile, or 64 x 64 tiles one after the other
+      const int tm = (a[11] & 64) ? 256 : (a[11] & 32) ? 128 : 64, tn = (a[11] & 64) ? 128 : (a[11] & 32) ? 128 : 64;
+      const int m = std::min(tm, a[8] - a[6]), n = std::min(tn, a[9] - a[7]);
+      return m <= 32 && n <= 32 ? 10.0 + 0.031 * a[10] : 14.0 + 0.093 * a[10] * ((m + 63) / 64) * ((n + 63) / 64); }
+    case 8: return 14.0 + 0.093 * a[5] * ((a[3] + 63) / 64) * ((a[4] + 63) / 64);
+    case 45: case 47: case 48: {              // per (row of the other side) x (column of the head); tcgen05, or mma.sync on bf16 or on split float32 operands
+      const int r0 = a[d.op_id == 45 ? 7 : d.op_id == 47 ? 9 : 10], T = a[d.op_id == 45 ? 8 : d.op_id == 47 ? 10 : 11], hd = a[d.op_id == 45 ? 11 : 13];
+      const double n = (double)hd * (d.op_id == 48 ? T - r0 : std::min(r0 + 128, T));
+      const int k = d.op_id == 45 ? 0 : d.op_id == 47 ? 1 : 2;
+      if ((aux.x & 255) == 2) { const double per[3] = {0.45e-3, 0.43e-3, 0.7e-3}; return 3.0 + per[k] * n; }
+      const bool bf = a[0] >= 0 && a[0] < (int)h->bufs.size() && h->bufs[a[0]].dtype == KVM_BF16;
+      const double fix[2][3] = {{15.0, 12.0, 13.0}, {15.0, 20.0, 26.0}}, per[2][3] = {{3.2e-3, 6.5e-3, 7.6e-3}, {1.0e-3, 1.25e-3, 2.65e-3}};
+      return fix[bf][k] + per[bf][k] * n; }
+    case 46: return 6.0 + elems(a[3], a[4]) * a[6] * a[7] * 4.0 / BPU;
     case 35: case 36: case 37: case 38: { const int r0 = a[d.op_id == 36 ? 4 : 6], r1 = a[d.op_id == 36 ? 5 : 7], dd = a[d.op_id == 36 ? 6 : 8];
-      return 2.0 + elems(r0, r1) * dd * 10.0 / BPU; }
-    case 39: return 2.0 + (double)a[6] * elems(a[8], a[9]) * 8.0 / BPU;
+      return 5.0 + elems(r0, r1) * dd * 10.0 / BPU; }
+    case 39: return 10.0 + (double)a[6] * elems(a[8], a[9]) * 8.0 / BPU;
     case 61: return 2.0 + (double)a[2] * elems(a[3], a[4]) * 4.0 / BPU;
-    case 51: case 53: case 127: { const int r0 = a[d.op_id == 51 ? 4 : 5], r1 = a[d.op_id == 51 ? 5 : 6], V = a[d.op_id == 51 ? 6 : 7]; return 2.0 + elems(r0, r1) * V * 6.0 / BPU; }
-    case 54: case 115: return 2.0 + elems(a[6], a[7]) * 28.0 / BPU;
+    case 51: case 53: case 127: { const int r0 = a[d.op_id == 51 ? 4 : 5], r1 = a[d.op_id == 51 ? 5 : 6], V = a[d.op_id == 51 ? 6 : 7]; return 5.0 + elems(r0, r1) * V * 6.0 / BPU; }
+    case 54: case 115: return 8.0 + elems(a[6], a[7]) * 28.0 / BPU;
     case 55: return 1.5 + elems(a[3], a[4]) * 4.0 / BPU;
     case 32: return 2.0 + elems(a[4], a[5]) * a[7] * 8.0 / BPU;
     case 33: return 3.0 + (double)a[3] * 4.0 / BPU + elems(a[5], a[6]) * a[7] * 8.0 / BPU;
-    case 40: case 41: case 42: case 113: case 117: case 126: case 96: case 97: case 98: case 123: case 59: {
-      const int w = d.args_words;             // flat ops end with (..., e0, e1) or (e0, e1, acc / kind-dependent)
-      double n = 0;
-      for (int k = 0; k + 1 < w; ++k) if (a[k + 1] > a[k] && a[k] >= 0 && (double)a[k + 1] - a[k] > n && a[k + 1] < (1 << 30)) n = (double)a[k + 1] - a[k];
-      return 1.5 + n * 12.0 / BPU; }
+    case 59: return 2.5 + elems(a[1], a[2]) * 4.0 / BPU;
+    case 40: case 113: case 126: return 2.5 + elems(a[2], a[3]) * 8.0 / BPU;
+    case 41: case 42: case 96: case 98: case 117: case 123: return 2.5 + elems(a[3], a[4]) * 12.0 / BPU;
+    case 97: return 2.5 + elems(a[4], a[5]) * 12.0 / BPU;
     default: return 3.0;
   }
-  (void)h;
 }
 
 // Buffers some task of the batch may write.  Everything a task names counts as written unless the (op, argument) pair is known
@@ -110,7 +116,7 @@ static int kvm_plan_static(KvmExec* h, const std::vector<int>& base_versions, Kv
 
   std::vector<double> cost(nt), finish(nt, 0.0), avail(W, 0.0);
   std::vector<int> worker(nt, -1), pos(nt, 0), count(W, 0);
-  for (int i = 0; i < nt; ++i) cost[i] = kvm_static_cost(h, h->tasks[i], h->args.data() + h->tasks[i].args_off);
+  for (int i = 0; i < nt; ++i) cost[i] = kvm_static_cost(h, h->tasks[i], h->args.data() + h->tasks[i].args_off, h->aux[i]);
   typedef std::pair<int, int> Key;      // (-priority class, index): smallest first
   std::priority_queue<Key, std::vector<Key>, std::greater<Key>> ready;
   auto cls = [&](int i) { const int p = h->tasks[i].priority; return p < 0 ? 0 : (p >> 3) >= KVM_NCLASS ? KVM_NCLASS - 1 : (p >> 3); };

@@ -303,3 +303,19 @@ def test_splits_of_every_flag_stream(kvm_lib, hd, G, flags, streams):
             if trace:
                 split = b.tasks['op_id'] == 135
                 assert (ex.trace_detail()[split] > 0).all() == streams
+
+
+@pytest.mark.parametrize('program', ['mlps', 'training'])
+def test_planned_time_is_of_the_measured_size(kvm_lib, program):
+    """The planner's costs: the makespan it expects of a program of small tasks is within a factor of three of the time it takes (a
+    factor f32 of an elementwise op once counted as an element range: hours for a millisecond)."""
+    from kvm_b200.executor import CFG_STATIC, Executor
+    from kvm_b200.workloads.gpt import build_training, preset
+    from kvm_b200.workloads.mlp import MLPConfig, build_mlps
+    g = build_mlps(MLPConfig(widths=(72, 104, 200), in_dim=100, batch=96), 2) if program == 'mlps' else build_training(preset('gpt_tiny'), 1, stream_steps=8)
+    with Executor(flags=CFG_STATIC) as ex:
+        ex.load(g.to_bundle(check=False))
+        ex.run()
+        us = min(ex.run().ms for _ in range(5)) * 1e3
+        planned = ex.plan_info()[2]
+    assert planned / 3 <= us <= planned * 3, (planned, us)
