@@ -36,7 +36,8 @@ __device__ __forceinline__ void kvm_st4(const KvmBuf& b, size_t i, float4 v) {
 }
 
 // ---- layernorm forward, float32 rows -------------------------------------------------------------------------------------------
-// A warp per row, NV float4 per lane (pairs of them make up eight neighbouring columns: the general body's order of summation); gamma and beta wait in shared memory, the next row is in flight while this one is reduced.
+// A warp per row, NV float4 per lane (pairs of them make up eight neighbouring columns: the general body's order of summation, for rows of
+// a multiple of eight columns); gamma and beta wait in shared memory, the next row is in flight while this one is reduced.
 __device__ __forceinline__ int kvm_hot_ln_col(int t) { return (threadIdx.x & 31) * 8 + (t >> 1) * 256 + (t & 1) * 4; }      // first column of a lane's piece t
 template <int NV>
 __device__ __forceinline__ void kvm_hot_ln_fwd_t(const KvmBuf& x, const KvmBuf& out, float* mean, float* rstd, const float* gs, int r0, int r1, int d, float eps) {
@@ -81,7 +82,7 @@ __device__ __forceinline__ bool kvm_hot_ln_fwd(const KvmCtx& c, const int32_t* a
   const float eps = kvm_bits_f32(a[9]);
   if (!kvm_hot_buf(c, a[0], KVM_F32, x) || !kvm_hot_buf(c, a[1], KVM_F32, g) || !kvm_hot_buf(c, a[2], KVM_F32, be) || !kvm_hot_float(c, a[3], out) || !kvm_hot_buf(c, a[4], KVM_F32, mean) ||
       !kvm_hot_buf(c, a[5], KVM_F32, rstd)) return false;
-  if (r0 < 0 || r1 < r0 || d <= 0 || d > 1024 || (d & 3) || !kvm_hot_mat(x, r1, d) || !kvm_hot_mat(out, r1, d) || !kvm_hot_flat(g, d) || !kvm_hot_flat(be, d) || !kvm_hot_flat(mean, r1) ||
+  if (r0 < 0 || r1 < r0 || d <= 0 || d > 1024 || ((d | x.ld | out.ld) & 7) || !kvm_hot_mat(x, r1, d) || !kvm_hot_mat(out, r1, d) || !kvm_hot_flat(g, d) || !kvm_hot_flat(be, d) || !kvm_hot_flat(mean, r1) ||
       !kvm_hot_flat(rstd, r1)) return false;
   float* gs = (float*)c.smem;                     // gamma, beta
   kvm_sync();
@@ -149,7 +150,7 @@ __device__ __forceinline__ bool kvm_hot_ln_bwd(const KvmCtx& c, const int32_t* a
   const int r0 = a[6], r1 = a[7], d = a[8], acc = a[9];
   if (!kvm_hot_buf(c, a[0], KVM_F32, x) || !kvm_hot_float(c, a[1], dy) || !kvm_hot_buf(c, a[2], KVM_F32, g) || !kvm_hot_buf(c, a[3], KVM_F32, mean) || !kvm_hot_buf(c, a[4], KVM_F32, rstd) ||
       !kvm_hot_buf(c, a[5], KVM_F32, dx)) return false;
-  if (r0 < 0 || r1 < r0 || d <= 0 || d > 1024 || (d & 3) || !kvm_hot_mat(x, r1, d) || !kvm_hot_mat(dy, r1, d) || !kvm_hot_mat(dx, r1, d) || !kvm_hot_flat(g, d) || !kvm_hot_flat(mean, r1) ||
+  if (r0 < 0 || r1 < r0 || d <= 0 || d > 1024 || ((d | x.ld | dy.ld | dx.ld) & 7) || !kvm_hot_mat(x, r1, d) || !kvm_hot_mat(dy, r1, d) || !kvm_hot_mat(dx, r1, d) || !kvm_hot_flat(g, d) || !kvm_hot_flat(mean, r1) ||
       !kvm_hot_flat(rstd, r1)) return false;
   float* gs = (float*)c.smem;
   kvm_sync();

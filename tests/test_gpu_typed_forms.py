@@ -75,3 +75,80 @@ def test_elementwise(kvm_lib, e0, e1):
     x, o = g.data('x', normal(5, 1, n)), g.buffer('rounded', 1, n, 'bf16')
     g.task('round_bf16', {'x': x, 'out': o, 'e0': e0, 'e1': e1}, [x], [o])
     same_bits(g)
+
+
+# widths around the instances (256, 768, 1024 columns) and past them; rows that leave warps without one
+@pytest.mark.parametrize('d', [8, 248, 256, 260, 264, 768, 776, 1024, 1032])
+@pytest.mark.parametrize('rows', [1, 37])
+def test_layernorm(kvm_lib, d, rows):
+    g = Graph('layernorm')
+    g.data('x', normal(1, rows, d)), g.data('gamma', normal(2, 1, d)), g.data('beta', normal(3, 1, d))
+    for dt in ('f32', 'bf16'):
+        for n, r, c, t in (('out', rows, d, dt), ('mean', rows, 1, 'f32'), ('rstd', rows, 1, 'f32')):
+            g.buffer(f'{n}.{dt}', r, c, t)
+        g.task('layernorm_fwd', {'x': 'x', 'gamma': 'gamma', 'beta': 'beta', 'out': f'out.{dt}', 'mean': f'mean.{dt}', 'rstd': f'rstd.{dt}', 'r0': 0, 'r1': rows, 'd': d, 'eps': 1e-5},
+               ['x'], [f'out.{dt}', f'mean.{dt}', f'rstd.{dt}'])
+        g.data(f'dy.{dt}', normal(4, rows, d), dt)
+        for acc in (0, 1):
+            dx = g.data(f'dx.{dt}.{acc}', normal(5, rows, d))
+            g.task('layernorm_bwd_dx', {'x': 'x', 'dy': f'dy.{dt}', 'gamma': 'gamma', 'mean': f'mean.{dt}', 'rstd': f'rstd.{dt}', 'dx': dx, 'r0': 0, 'r1': rows, 'd': d, 'acc': acc},
+                   ['x', f'dy.{dt}', f'mean.{dt}', f'rstd.{dt}'], [dx])
+    same_bits(g)
+
+
+# the shortest typed row, two row buffers, one (more than half of the scratch), and a row too long for one
+@pytest.mark.parametrize('V', [1032, 8200, 50304, 65536, 120000])
+def test_cross_entropy(kvm_lib, V):
+    rows, rng = 5, np.random.default_rng(V)
+    g = Graph('ce')
+    g.data('logits', normal(1, rows, V), 'bf16'), g.data('tgt', rng.integers(0, V, (rows, 1), dtype=np.int32), 'i32')
+    g.buffer('rowloss', rows, 1), g.buffer('lse', rows, 1), g.buffer('dlogits', rows, V, 'bf16')
+    for r0, r1 in ((0, 2), (2, 5)):
+        g.task('softmax_ce_fused', {'logits': 'logits', 'tgt': 'tgt', 'rowloss': 'rowloss', 'lse': 'lse', 'dlogits': 'dlogits', 'r0': r0, 'r1': r1, 'V': V, 'ignore': -1, 'N': rows, 'scale': 1.0},
+               ['logits'], [(n, (r0, r1)) for n in ('rowloss', 'lse', 'dlogits')])
+    same_bits(g)
+
+
+@pytest.mark.parametrize('H,hd', [(1, 32), (3, 64), (5, 128), (12, 64)])
+def test_attention_delta(kvm_lib, H, hd):
+    T, B = 45, 3
+    g = Graph('delta')
+    for dt in ('f32', 'bf16'):
+        g.data(f'o.{dt}', normal(1, B * T, H * hd), dt), g.data(f'do.{dt}', normal(2, B * T, H * hd), dt), g.buffer(f'delta.{dt}', B * H * T, 1)
+        for r0, r1 in ((0, 17), (17, 90), (90, B * T)):
+            g.task('attn_bwd_delta', {'o': f'o.{dt}', 'do': f'do.{dt}', 'delta': f'delta.{dt}', 'r0': r0, 'r1': r1, 'T': T, 'H': H, 'hd': hd}, [f'o.{dt}'], [])
+    same_bits(g)
+
+
+@pytest.mark.parametrize('e0,e1', [(0, 4), (4, 2052), (0, 8192), (8, 20004), (2, 4099)])
+def test_adamw(kvm_lib, e0, e1):
+    n = -(-e1 // 8) * 8
+    g = Graph('adamw')
+    for i, name in enumerate('pgm'):
+        g.data(name, normal(i, 1, n))
+    g.data('v', np.abs(normal(9, 1, n))), g.data('clip', np.array([[0.7]], np.float32)), g.data('step', np.array([[3]], np.int32), 'i32')
+    g.task('adamw', {'p': 'p', 'g': 'g', 'm': 'm', 'v': 'v', 'gscale': 'clip', 'step': 'step', 'e0': e0, 'e1': e1, 'lr': 1e-3, 'b1': 0.9, 'b2': 0.999, 'eps': 1e-8, 'wd': 0.1},
+           ['g', 'clip', 'step'], ['p', 'm', 'v'])
+    same_bits(g)
+
+
+# twenty splits at once in the static kernel's form, more in the op's own; two forms of one sum: float32 roundings of up to 21 terms apart
+@pytest.mark.parametrize('S', [1, 20, 21, 30])
+def test_merge_of_splits(kvm_lib, S):
+    H, hd, rng = 3, 64, np.random.default_rng(S)
+    part = rng.standard_normal((S * H, hd + 2)).astype(np.float32)
+    part[:, hd + 1] = np.abs(part[:, hd + 1]) + 0.1
+    if S > 2:
+        part[H:2 * H, hd:] = [-3.4028234663852886e38, 0.0]      # an empty split
+    g = Graph('merge')
+    g.data('part', part), g.buffer('o', 1, H * hd)
+    g.task('attn_decode_merge', {'part': 'part', 'o': 'o', 'b': 0, 'h0': 0, 'h1': H, 'S': S, 'H': H, 'hd': hd}, ['part'], ['o'])
+    b = g.to_bundle()
+    p = part.reshape(S, H, hd + 2).astype(np.float64)
+    e = np.where(p[..., hd + 1] > 0, np.exp(p[..., hd] - p[..., hd].max(0)), 0)
+    ref = (np.einsum('sh,shc->hc', e, p[..., :hd]) / (e * p[..., hd + 1]).sum(0)[:, None]).ravel()
+    for flags in (CFG_DYNAMIC, CFG_STATIC):
+        with Executor(flags=flags) as ex:
+            ex.load(b)
+            ex.run()
+            assert np.abs(ex.read_buffer('o')[0] - ref).max() <= 2.0 ** -23 * (S + 4) * np.abs(ref).max()
