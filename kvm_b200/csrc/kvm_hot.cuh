@@ -166,10 +166,10 @@ __device__ __forceinline__ bool kvm_hot_ln_bwd(const KvmCtx& c, const int32_t* a
 }
 
 // ---- column sums (and the parameter gradients of a norm) -------------------------------------------------------------------------------
-// 64 columns at a time.  Rows come through shared memory, copied sixteen bytes at a time, 72 to 112 KB in flight (one column per thread straight from global memory left the loop at 10 KB/us); they are added from there by eight row
-// groups of a thread per column, in the general body's order.  Bound by HBM: 8192 rows of 64 columns take 43 us for a column sum of bf16
-// rows and 111 us for the parameter gradients of a norm in the 162M step (94 and 301 in the general body; 55 and 124 with 32 row groups
-// straight from global memory, which summed in another order).
+// 64 columns at a time.  Rows come through shared memory, copied sixteen bytes at a time, 72 to 112 KB in flight (one column per thread
+// straight from global memory left the loop at 10 KB/us); they are added from there by eight row groups of a thread per column, in the
+// general body's order.  Bound by HBM: 8192 rows of 64 columns take 43 us for a column sum of bf16 rows and 111 us for the parameter
+// gradients of a norm in the 162M step (94 and 301 in the general body).
 __device__ __forceinline__ void kvm_cp_async(uint32_t dst, const void* src, int bytes) {      // 16 or 4
   if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");

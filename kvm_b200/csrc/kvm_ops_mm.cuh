@@ -78,8 +78,8 @@ static __device__ bool kvm_mm_args(const KvmCtx& c, const int32_t* a, int kind /
 // 64x64 sub-tiles, K staged through shared memory 32 at a time.  The first eight warps multiply, a thread owns 4 rows x 4 columns:
 // per k two LDS.128 for 16 products.  The exact multiply-then-add (two roundings per step, no fused multiply-add) needs 64 issue
 // cycles per k and SM, the two loads 64 cycles of shared-memory bandwidth; the form before (one row x 8 columns per thread, all
-// sixteen warps) asked shared memory for 3 loads per 8 products.  The packed f32x2 instructions do not help: the compiler
-// contracts a packed multiply and add into a packed FMA.
+// sixteen warps) asked shared memory for 3 loads per 8 products.  Packed FMAs (the 32x32 form below) do not help here: 66-72 ns per k
+// against 69, shared memory and issue overlap no better with two multiplying warps per scheduler.
 // All sixteen warps stage: chunk i+2 is in flight from global memory (registers) while chunk i is multiplied, chunk i+1 is in the
 // other shared buffer: one barrier per chunk.  Both arrays are stored [k][.] with their 16-byte units XOR-swizzled by (k / 4) & 7, so
 // that the transposing stores (k contiguous in global memory) spread over the banks as well as the loads do.

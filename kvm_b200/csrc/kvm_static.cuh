@@ -95,9 +95,9 @@ __device__ __forceinline__ bool kvm_ring_wait_warp(const KvmRing& ring, unsigned
 // ---- streamed GEMV, consumer side --------------------------------------------------------------------------------------------
 // Stage use `cit + ci` holds rows n0 + ci*R .. of the weight matrix in full (R*K*2 bytes).  All sixteen warps consume: warp = (row group,
 // part of K), KP parts of 256 columns or more, 16 / KP row groups of up to eight rows a stage.  A thread owns J pieces of eight columns
-// of the activation row v = bf16(prologue(x)): it computes them itself and keeps them as float32 over the task, so the activations cost
-// no shared memory and the prologue has one barrier at most (the sum of squares).  The eight rows' sums leave a warp through one
-// transposing reduction (nine shuffles for eight rows).
+// of the activation row v = bf16(prologue(x)): it computes them itself and keeps them over the task (as float32, or as bf16 from four
+// pieces on), so the prologue has one barrier at most (the sum of squares).  The eight rows' sums leave a warp through one transposing
+// reduction (nine shuffles for eight rows).
 // What bounds it: a 64 KB stage is 1.5 us of an SM's share of HBM and about 700 issue cycles here; every value of the loop has to stay
 // in registers, since a spilled one costs an L2 round trip per stage (the stages leave 28 KB of L1 for 512 threads' local memory).
 // Partial sums are added in pairs.  Semantics as kvm_op_gemv_bf16 (runtime/ref_extra.py:398-415).  Always consumes its nchunks
@@ -766,7 +766,7 @@ static __device__ void kvm_static_geometry(const KvmDevState& S, KvmStSlot& sl, 
   }
 }
 
-// Issue the copies of chunk `ci` of the task in `sl` as stage use `it` (front warp, lane 0; the stage is known to be free).
+// Issue the copies of chunk `ci` of the task in `sl` as stage use `it` (stream warp, lane 0; the stage is known to be free).
 static __device__ void kvm_static_issue(const KvmDevState& S, const KvmStSlot& sl, const KvmRing& ring, unsigned it, int ci) {
   const uint32_t full = kvm_ring_full(ring, it), dst = ring.base_addr + kvm_ring_slot(ring, it) * KVM_ST_STAGE;
   const int32_t* a = sl.args;

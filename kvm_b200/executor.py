@@ -342,7 +342,7 @@ class Executor:
         return s, e, sm
 
     def trace_detail(self, n=None):
-        """Per task the packed prologue / stage-wait times of a streamed GEMV on the static path (see kvm_trace_detail)."""
+        """Per task the packed prologue / stage-wait times of a streamed GEMV or attention split on the static path (see kvm_trace_detail)."""
         n = n if n is not None else len(self.bundle.tasks)
         d = np.empty(n, np.int32)
         self._check(self.L.kvm_trace_detail(self._h, d.ctypes.data, n))

@@ -1,4 +1,4 @@
-"""GPU parity of causal attention forward / backward (SIMT form and the tcgen05 form for bf16 hd=64) against the CPU oracle."""
+"""GPU parity of causal attention forward / backward (mma.sync form, and the tcgen05 form for bf16 hd=64) against the CPU oracle."""
 import numpy as np
 import pytest
 
