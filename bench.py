@@ -115,8 +115,8 @@ def workload_name(model, cfg):
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one kvm_exec_kernel launch of the step, from the one-pass ncu captures summarised
 # in profiles/bench_gpt162m_launch_list.md (full size) and profiles/kvm_exec_kernel_gpt162m_2l_ncu_full.md (two-layer cut)
-DECODE_TRAFFIC_RATIO = (2901808000 + 218917888) / 2855e6      # kvm_static_kernel on qwen3_8b_4l: profiles/kvm_static_kernel_decode_4l_ncu.md
-DRAM_TRAFFIC = {'gpt_162m': 24079402496 + 11409903104, 'gpt_162m_2l': 6419808000 + 3092519000}
+DECODE_TRAFFIC_RATIO = (2859055000 + 98225920) / 2855e6      # kvm_static_kernel on qwen3_8b_4l: profiles/kvm_static_kernel_decode_4l_ncu.md
+DRAM_TRAFFIC = {'gpt_162m': 24255992576 + 10744735744, 'gpt_162m_2l': 6230917000 + 2979900000}
 
 
 def get_bundle(model, rank, world, stream_steps, over):
@@ -656,7 +656,7 @@ def run_decode(args, device):
            'value': tok_s, 'unit': 'tok/s', 'ms_per_token': res.ms / ntok, 'tokens': ntok, 'e2e': {'value': e2e, 'unit': 'tok/s', 'h2d_bytes_per_step': 0, 'd2h_bytes_per_step': 4, 'tokens': n_e2e},
            'roofline': {'bound': 'hbm', 'achieved': gbs, 'peak': pk.get('hbm_gbs', PEAK_FALLBACK['hbm_gbs']), 'unit': 'GB/s', 'frac': gbs / pk.get('hbm_gbs', PEAK_FALLBACK['hbm_gbs']),
                         'bytes_per_token': bytes_tok, 'peak_source': f'{kind} hbm_gbs', 'traffic': bytes_tok * DECODE_TRAFFIC_RATIO,
-                        'traffic_note': 'DRAM bytes of the 4-layer cut under ncu (3.12 GB for 2.86 GB algorithmic), scaled by the algorithmic bytes'}, 'last_token': int(tok[0]),
+                        'traffic_note': 'DRAM bytes of the 4-layer cut under ncu (2.96 GB for 2.86 GB algorithmic), scaled by the algorithmic bytes'}, 'last_token': int(tok[0]),
            'path': {'static_schedule': path[0], 'stream_ring': path[1], 'planned_us_per_token': path[2]}}
     ex.close()
     pkh = pk.get('hbm_gbs', PEAK_FALLBACK['hbm_gbs'])
