@@ -107,9 +107,15 @@ def param_shapes(c: GPTConfig):
     return out
 
 
+# Elements of a task at least: a chunk is an edge to every tile that reads its tensor, and below this many the edges cost more than the
+# shorter task gives (small f32 GPT, four steps: 9.93 ms and 1.19 M edges with 4096, 9.75 and 0.79 M with 16384; 3 x 200 tokens bf16 2.16
+# and 2.11 ms; tiny model 1.27 either way).  The MLP programs, chains of a few tasks a phase, keep 4096 (small ones 1.07 ms against 1.13).
+LEAST = 16384
+
+
 def opt_chunk(c: GPTConfig) -> int:
     """Elements per optimizer chunk: the parameters are updated side by side, about two chunks per SM."""
-    return Graph.spread(sum(rows * cols for _, rows, cols, _, _ in param_shapes(c)) // 2, c.flat_chunk, c.workers)
+    return Graph.spread(sum(rows * cols for _, rows, cols, _, _ in param_shapes(c)) // 2, c.flat_chunk, c.workers, LEAST)
 
 
 def dp_exchange_layout(c: GPTConfig, world: int):
@@ -183,7 +189,7 @@ class _Emit:
     def flat(self, op, bufs_r, bufs_w, n_elems, args, tag, chunk=None):
         """Elementwise op over equally shaped buffers, chunked on row boundaries."""
         g = self.g
-        for i, (e0, e1) in enumerate(g.flat_chunks(bufs_w[0], chunk or g.spread(n_elems, self.c.flat_chunk, self.c.workers))):
+        for i, (e0, e1) in enumerate(g.flat_chunks(bufs_w[0], chunk or g.spread(n_elems, self.c.flat_chunk, self.c.workers, LEAST))):
             rd = [(b, *g.region_of(b, e0, e1)) for b in bufs_r]
             wr = [(b, *g.region_of(b, e0, e1)) for b in bufs_w]
             g.task(op, {**args, 'e0': e0, 'e1': e1}, rd, wr, self.prio, f'{tag}.{i}')

@@ -115,8 +115,8 @@ class Graph:
 
     @staticmethod
     def spread(n, chunk, workers=SMS, least=4096):
-        """Chunk length for a phase of `n` elements: `chunk`, or less where that would leave some of `workers` SMs without a task.  Below 4096 elements a
-        task is all fixed cost (3-4 us)."""
+        """Chunk length for a phase of `n` elements: `chunk`, or less where that would leave some of `workers` SMs without a task, but
+        `least` at least.  Below 4096 elements a task is all fixed cost (3-4 us)."""
         return min(chunk, max(least, -(-n // workers)))
 
     @staticmethod

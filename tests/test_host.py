@@ -287,3 +287,17 @@ def test_phases_are_cut_for_the_workers_of_the_configuration():
     for build, cfg in ((build_training, gpt('gpt_tiny')), (build_mlps, mlp('mlp_small'))):
         tasks = [len(build(cfg.__class__(**{**cfg.__dict__, 'workers': w}), 1).to_bundle(check=False).tasks) for w in (8, SMS)]
         assert tasks[0] < tasks[1] == len(build(cfg, 1).to_bundle(check=False).tasks)
+
+
+def test_training_phases_are_not_cut_below_their_edges():
+    """Elementwise and optimizer tasks of the small float32 GPT: no more of them than 16384 elements each leave, and the edges that go
+    with them."""
+    from kvm_b200 import abi
+    from kvm_b200.workloads.gpt import GPTConfig, build_training
+    c = GPTConfig(layers=3, d_model=192, heads=3, d_ff=768, vocab=1001, seq=120, batch=5, tied=False)
+    b = build_training(c, 1).to_bundle(check=False)
+    op = {v.id: k for k, v in abi.load_ops().items()}
+    flat = [b.args[t['args_off']:t['args_off'] + t['args_words']] for t in b.tasks if op[int(t['op_id'])] in ('adamw', 'gelu_bwd')]
+    sizes = [int(a[7] - a[6]) if len(a) == 13 else int(a[4] - a[3]) for a in flat]
+    full = [n for n in sizes if n > 8192]
+    assert sum(full) / len(full) >= 0.75 * 16384        # cut on row boundaries
